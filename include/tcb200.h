@@ -216,8 +216,10 @@ typedef struct tcb_mono {
                                 most whose rows fit (2, else 1); 1 or 2 pins it */
     int32_t fused_step;      /* 1: each step is one launch, the ionic update fused into the CG kernel that
                                 keeps rows in shared memory (where that kernel applies: int16 column
-                                offsets, rows that fit); 0: the ionic and CG kernels as two launches.
-                                The values are the same either way */
+                                offsets, rows that fit); 2: the ionic and CG kernels as two launches;
+                                0: many steps in one persistent launch for meshes it suits (given `work`),
+                                else two launches.  The values are the same either way up to the order of
+                                the float64 sums */
     /* device bookkeeping (caller-allocated, zero-initialised) */
     int32_t* step_iters;     /* [nt+1] CG iterations of each step */
     int32_t* counter;        /* [4]: next step, error code, 2 spare */
@@ -227,9 +229,20 @@ typedef struct tcb_mono {
     const double* params;
     /* per-node model parameters (tcb_model_node_params), n_pad floats per row, or NULL */
     const float* node_params;
+    /* optional: tcb_mono_work_bytes() bytes, zeroed once, 16-byte aligned; with it tcb_mono_run and
+     * tcb_mono_cg_run run stretches of steps as persistent launches where that is the faster form
+     * (fused_step = 0); NULL: every step is launched by itself */
+    void* work;
+    int32_t work_entries;    /* as tcb_mono_work_bytes() gave it */
 } tcb_mono;
 
 int64_t tcb_mono_scratch_doubles(void);
+/* Bytes of tcb_mono.work for this simulation on the current device, and in *entries the
+ * value of tcb_mono.work_entries (the most sliced-ELL entries one block of rows has; read from
+ * slice_ptr, so the stream is synchronised).  0 where steps are launched one by one in any
+ * case: meshes whose matrix does not fit in the GPU's shared memory, fused_step != 0.
+ * Negative = error status. */
+int64_t tcb_mono_work_bytes(const tcb_mono* m, int32_t* entries, void* stream);
 /* Run steps [step_begin, step_end) (1-based, step_begin must equal the device
  * counter).  Non-convergence is not an error (n_iter == max_iter), as in the
  * reference. */
@@ -247,8 +260,9 @@ int tcb_mono_cg_run(const tcb_mono* m, int64_t step_begin, int64_t step_end, voi
  * A fused step's single kernel counts as CG time (ms_ionic gets nothing). */
 int tcb_mono_profile(const tcb_mono* m, int64_t step_begin, int64_t step_end, void* stream, double* ms_ionic,
                      double* ms_cg);
-/* Which CG kernel tcb_mono_run launches for this simulation on the current
- * device: 2 = the fused step (ionic update inside the CG kernel that keeps rows
+/* Which CG kernel a single step of this simulation launches on the current
+ * device (tcb_mono_profile; tcb_mono_run too where it does not run stretches of steps
+ * as one launch, see tcb_mono.work): 2 = the fused step (ionic update inside the CG kernel that keeps rows
  * in shared memory), 1 = that CG kernel after a separate ionic launch, 0 = the
  * streaming kernel; negative = error status.  No counterpart in the reference
  * (used to label measurements). */

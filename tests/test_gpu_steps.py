@@ -1,0 +1,97 @@
+"""Many steps in one persistent launch (``csrc/steps.cu``) against the step-by-step launches.
+
+Both run the same equations from the same state; they differ in the order of
+the float64 sums over rows, in the stopping test (formed from the sums of the
+pass instead of a second reduction) and in r' taken from float32 pairs, each a
+relative 1e-12 or less of what is rounded to float32 once.  So after a stretch
+of steps the solutions agree to a few float32 ulp of their range per step:
+steps * 2^-23 is the bound used, and the iteration counts are equal.
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+from torchcor_b200 import meshgen
+
+pytestmark = pytest.mark.gpu
+
+
+def _sim(mesh, size, model, device, theta=0.5, dt=0.02, steps=160):
+    from torchcor_b200.ionic import CourtemancheRamirezNattel, ModifiedMS2v, TenTusscherPanfilov
+    from torchcor_b200.simulator import Monodomain
+    if model == "ttp":
+        im = TenTusscherPanfilov("ENDO", dt, device=device)
+    elif model == "crn":
+        im = CourtemancheRamirezNattel(dt, device=device)
+    else:
+        im = ModifiedMS2v(dt, device=device)
+    sim = Monodomain(im, T=(steps + 0.5) * dt, dt=dt, device=device)
+    sim.theta = theta
+    if mesh == "cube":
+        nodes, elems = meshgen.cube(size, 0.25)
+        fib = meshgen.fibres_constant(len(elems))
+    else:
+        nodes, elems = meshgen.icosphere_fast(size, 25.0)
+        fib = meshgen.fibres_random_tangent(nodes, elems, 3)
+    sim.load_arrays(nodes / 1000.0, elems, np.ones(len(elems), dtype=np.int64), fib)
+    sim.add_conductivity([1], il=0.5, it=0.2)
+    sim.add_stimulus(None, 0.0, 1.0, 100, region=np.arange(max(1, len(nodes) // 9)))
+    return sim
+
+
+def _run(sim, tol, max_iter, guess, fused_step, chunks, frames=False):
+    from torchcor_b200._lib import check, load, stream_ptr
+    sim._sim = None
+    sim.prepare(tol, tol, max_iter, linear_guess=guess, snapshot_interval=1 if frames else sim.T)
+    sim.set_launch(fused_step=fused_step)
+    for k in chunks:
+        sim.run_steps(k)
+    check(load().tcb_mono_check(C.byref(sim._sim["struct"]), stream_ptr()))
+    assert (sim._sim["work"] is not None) == (fused_step == 0)
+    d = sim._sim
+    n = sim.n_nodes
+    out = dict(x=d["x"][:, :n].clone(), state=sim.ionic_model.state[:, :n].clone(), at=d["at"].clone(), rt=d["rt"].clone(),
+               iters=d["step_iters"].clone())
+    if frames:
+        out["frames"] = d["snaps"][: sim._frames_written() + 1].clone()
+    return out
+
+
+@pytest.mark.parametrize("mesh,size,model,tol,max_iter,guess,theta", [
+    ("cube", 2, "ms", 1e-5, 100, True, 0.5),        # 27 nodes: one ragged slice, one block
+    ("cube", 7, "ttp", 1e-5, 100, True, 0.5),       # 512 nodes: whole slices
+    ("cube", 9, "crn", 1e-8, 100, False, 0.5),      # many passes a step
+    ("cube", 11, "ms", 1e-8, 2, True, 0.5),         # stopped by max_iter
+    ("cube", 11, "ms", 1e-5, 0, True, 0.5),         # no pass at all
+    ("cube", 13, "ttp", 1e-6, 100, True, 0.25),     # A is not M Cm + K'
+    ("ico", 3, "crn", 1e-6, 100, True, 0.5),        # rows of 6 and 7 entries
+    ("ico", 6, "ms", 1e-6, 100, True, 0.5),         # 32-bit columns
+    ("cube", 46, "ttp", 1e-6, 100, True, 0.5),      # two rows a thread, state held
+])
+def test_persistent_steps_match_single_launches(lib, cuda, mesh, size, model, tol, max_iter, guess, theta):
+    steps = 120
+    sim = _sim(mesh, size, model, cuda, theta, steps=steps)
+    a = _run(sim, tol, max_iter, guess, 0, [steps])
+    if mesh == "ico" and size == 6:
+        assert sim.system.sell_dcol is None
+    assert bool(sim.system.a_split) == (theta == 0.5)
+    b = _run(sim, tol, max_iter, guess, 2, [steps])
+    assert torch.equal(a["iters"], b["iters"])
+    for k in ("x", "state"):
+        # Mitchell-Schaeffer's gate switches branch at a voltage: a node on it may go either way for a step
+        bound = 1e-2 if (k, model) == ("state", "ms") else steps * 2.0 ** -23
+        err = (a[k] - b[k]).abs().max().item() / b[k].abs().max().item()
+        assert err <= bound, (k, err)
+    assert (a["at"] - b["at"]).abs().max().item() <= 0.0201 and (a["rt"] - b["rt"]).abs().max().item() <= 0.0201
+
+
+def test_stretches_of_any_length_are_the_same(lib, cuda):
+    """Where a launch begins and ends changes nothing, bit for bit: 145 steps at once
+    (more than one launch's limit), and in stretches with and without the state held on chip."""
+    sim = _sim("cube", 10, "ttp", cuda)
+    ref = _run(sim, 1e-6, 100, True, 0, [145], frames=True)
+    got = _run(sim, 1e-6, 100, True, 0, [1, 1, 2, 3, 4, 5, 129], frames=True)
+    for k in ref:
+        assert torch.equal(ref[k], got[k]), k

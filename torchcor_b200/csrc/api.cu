@@ -108,6 +108,7 @@ int validate(const tcb_mono* m) {
         return fail(TCB_EINVAL, "tcb_mono: tables not 16-byte aligned");
     if (m->max_iter < 0 || m->per_frame < 0 || m->snap_ring < 0)
         return fail(TCB_EINVAL, "tcb_mono: negative max_iter/per_frame/snap_ring");
+    if ((uintptr_t)m->work & 15u) return fail(TCB_EINVAL, "tcb_mono: work not 16-byte aligned");
     if (m->ionic_variant < 0 || m->cg_per_sm < 0 || m->cg_per_sm > 2)
         return fail(TCB_EINVAL, "tcb_mono: ionic_variant < 0 or cg_per_sm outside 0..2");
     return TCB_OK;
@@ -150,6 +151,10 @@ extern "C" int tcb_mono_run(const tcb_mono* m, int64_t step_begin, int64_t step_
         return fail(TCB_EINVAL, "tcb_mono_run: step range outside [1, nt]");
     cudaStream_t s = as_stream(stream);
     MonoDev d = make_dev(m);
+    if (step_begin < step_end) {
+        st = launch_steps(m, d, step_end - step_begin, true, s);
+        if (st != 0) return st < 0 ? st : TCB_OK;
+    }
     const bool fused = step_begin < step_end && uses_fused_step(m, d);
     for (int64_t n = step_begin; n < step_end; ++n) {
         if (fused) {
@@ -172,6 +177,10 @@ extern "C" int tcb_mono_cg_run(const tcb_mono* m, int64_t step_begin, int64_t st
         return fail(TCB_EINVAL, "tcb_mono_cg_run: step range outside [1, nt]");
     cudaStream_t s = as_stream(stream);
     MonoDev d = make_dev(m);
+    if (step_begin < step_end) {
+        st = launch_steps(m, d, step_end - step_begin, false, s);
+        if (st != 0) return st < 0 ? st : TCB_OK;
+    }
     for (int64_t n = step_begin; n < step_end; ++n) {
         st = launch_cg(d, s);
         if (st) return st;

@@ -55,10 +55,12 @@ int launch_cg_resident(const MonoDev& d, cudaStream_t s);
 int resident_blocks(const MonoDev& d);
 int launch_mono_step(const tcb_mono* m, const MonoDev& d, cudaStream_t s);   // 1 launched, 0 not applicable
 int mono_step_fusable(const tcb_mono* m, const MonoDev& d);
+// many steps per launch (steps.cu): 1 launched, 0 not applicable, < 0 error; without the ionic update b' is the caller's
+int launch_steps(const tcb_mono* m, const MonoDev& d, int64_t n_steps, bool ionic, cudaStream_t s);
 bool cg_forced_fallback();
 // 1 if tcb_mono_run runs this simulation's steps as the fused kernel
 inline int uses_fused_step(const tcb_mono* m, const MonoDev& d) {
-    return m->fused_step && !cg_forced_fallback() && mono_step_fusable(m, d);
+    return m->fused_step == 1 && !cg_forced_fallback() && mono_step_fusable(m, d);
 }
 int cg_uses_resident(const MonoDev& d);
 

@@ -1,0 +1,681 @@
+// Many time steps of one simulation in one persistent cooperative launch.
+//
+// Small and middle-sized meshes are bound by latency: launches, grid barriers
+// and the chain column -> neighbour -> sum.  Here one launch runs a whole
+// stretch of steps (ionic update, right-hand side, Jacobi-PCG of
+// torchcor/core/solver.py:40-76) and keeps what the steps share on chip: a block
+// owns a contiguous range of rows; the solution, the CG vectors, the rows'
+// columns and matrix values and (where it fits) the ionic state stay in its shared
+// memory from step to step.  Blocks exchange
+// one 16-byte record per row through L2: {b', u, x0} for the right-hand side and
+// {r, p, A p, 1/diag} between CG passes; records of the block's own rows are
+// read from shared memory.
+//
+// Grid barriers: a step needs one after the ionic update, one after the
+// right-hand side (z of the neighbours) and one per CG pass.
+//  * Arrivals are counted in a word that only grows, so a barrier is a fence, an
+//    add without a result and a poll.  (Every block polling a flag word of every
+//    other one, with the partial sums in the words, has a round trip less but
+//    measured 4.7 us at 148 blocks: they all read the same lines.)
+//  * One barrier per CG pass: the sums a pass takes over r, p and A p give alpha
+//    and, by the identities
+//      |z'|^2 = |z|^2 - 2 alpha (D r, D A p) + alpha^2 |D A p|^2,
+//      (r', z') = (r, z) - 2 alpha (z, A p) + alpha^2 (A p, D A p),
+//    the stopping test and beta of the same pass (float64 throughout; every pass
+//    sums r and z anew, so nothing accumulates).  The next pass forms r', z' and p'
+//    of its own and its neighbours' rows from the records with the same roundings.
+//
+// What bounds it: the chain of latencies of a step (three grid barriers of about
+// 1.7 us, one of them with the sums 2.3 us; the ionic update's table reads 1-3 us;
+// column, gather and sum of a row 1-2 us a pass), not bytes.  Measured on B200, us a
+// step with x CG iterations, the two launches of a step replayed as a CUDA graph ->
+// here: TTP cube 1,000 nodes (0) 26.0 -> 10.8; MS cube 9,261 (0.4) 34.9 -> 12.1; TTP
+// cube 50,653 (1) 43.1 -> 17.7, 117,649 (0.8) 48.6 -> 26.0; CRN shell 40,962 (1) 36.6
+// -> 15.8, 163,842 (1) 51.7 -> 31.8.  The line to the two-launch form lies where the
+// matrix no longer fits (about 170,000 nodes of a tetrahedral mesh): reading it from
+// L2 instead, 262,144 nodes took 59.9 us here and 49.1 in two launches.
+//
+// Sums inside a row run in the order of the other CG kernels (M b' and K u in
+// float32, A x0 and A p in float64); sums over rows are float64 in an order that
+// depends on the launch shape only.
+#include <cuda_runtime.h>
+#include <math.h>
+
+#include <algorithm>
+#include <vector>
+
+#include "cg_common.cuh"
+#include "ionic_crn.cuh"
+#include "ionic_ms.cuh"
+#include "ionic_node.cuh"
+#include "ionic_ttp.cuh"
+#include "mono.cuh"
+#include "tcb_internal.h"
+
+namespace tcb {
+int validate_mono(const tcb_mono* m);
+namespace {
+
+using namespace cgk;
+
+constexpr int kThreads = 512;
+constexpr int kWarps = kThreads / 32;
+constexpr int kSums = 8;                  // sums of a CG pass (see pass_sums)
+constexpr int kSlots = 160;               // most blocks of a launch
+constexpr size_t kHeadBytes = 256;        // arrivals of all launches so far; their number when the launch began
+constexpr size_t kPartBytes = 2 * (size_t)kSums * kSlots * sizeof(double);
+
+// no ionic update: b' comes from the caller (tcb_mono_cg_run)
+struct GivenRhs {
+    static constexpr bool kIonic = false;
+};
+template <class M, class Q>
+struct Ionic {
+    static constexpr bool kIonic = true;
+    static constexpr int kStates = M::kStates;
+    using Model = M;
+    using Policy = Q;
+    typename M::C c;
+    typename M::Tables T;
+};
+
+struct StepsPlan {
+    int32_t n_steps, cap_rows, cap_entries;        // rows and matrix entries a block has at most
+    int32_t smem_bytes, held_at, state_at;         // byte offsets of the matrix and the state (0: not held)
+    uint32_t *arrivals, *base;                     // barrier word; its value between launches
+    double* parts;                                 // [2 parities][kSums][kSlots] block sums
+    float4* rec[2];                                // per-row records, n_pad each
+};
+
+// ---------------------------------------------------------------- grid barrier
+struct Shared {
+    double part[kWarps][kSums];
+    double total[kSums];
+};
+
+// One thread announces its block and waits until all have: an add without a
+// result and a poll of the same word, which only ever grows (`target` = its value
+// once everybody has arrived, modulo 2^32).  Bounded: false after the time limit or
+// when another block has recorded an error.
+__device__ __forceinline__ bool arrive_and_wait(uint32_t* word, uint32_t target, int32_t* err, const WaitLimit& lim) {
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");   // the block's writes before its arrival
+    asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(word) : "memory");
+    target += lim.extra_arrivals;
+    uint64_t t0 = 0;
+    for (int spin = 1;; ++spin) {
+        uint32_t v;
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
+        if ((int32_t)(v - target) >= 0) break;
+        if ((spin & 31) == 0) {
+            if (*(volatile int32_t*)err != 0) return false;
+            const uint64_t now = globaltimer();
+            if (t0 == 0) t0 = now;
+            if (now - t0 > lim.timeout_ns) {
+                atomicCAS(err, 0, TCB_ETIMEOUT);
+                return false;
+            }
+        }
+    }
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    return true;
+}
+
+// Grid barrier: every block's earlier writes are visible to every block after it.
+__device__ __forceinline__ bool barrier(const StepsPlan& pl, uint32_t& target, int32_t* err, const WaitLimit& lim) {
+    __syncthreads();
+    target += gridDim.x;
+    int bad = 0;
+    if (threadIdx.x == 0) bad = !arrive_and_wait(pl.arrivals, target, err, lim);
+    return !__syncthreads_or(bad);
+}
+
+// Grid barrier that also returns the totals of kSums float64 values per thread.
+// A warp's values are added by halving exchanges (16 lanes' worth of four values,
+// then eight lanes' worth of two, ...), the warps' by warp 0; after the barrier warp j
+// adds the blocks' value j.
+__device__ __forceinline__ bool barrier_sums(double (&v)[kSums], Shared& sh, const StepsPlan& pl, uint32_t& target,
+                                             int parity, int32_t* err, const WaitLimit& lim) {
+    static_assert(kSums == 8 && kWarps == 16, "exchange pattern");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double a[4], b[2], c;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const bool up = lane & 16;
+        const double give = up ? v[i] : v[i + 4], mine = up ? v[i + 4] : v[i];
+        a[i] = mine + __shfl_xor_sync(0xffffffffu, give, 16);
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const bool up = lane & 8;
+        const double give = up ? a[i] : a[i + 2], mine = up ? a[i + 2] : a[i];
+        b[i] = mine + __shfl_xor_sync(0xffffffffu, give, 8);
+    }
+    {
+        const bool up = lane & 4;
+        const double give = up ? b[0] : b[1], mine = up ? b[1] : b[0];
+        c = mine + __shfl_xor_sync(0xffffffffu, give, 4);
+    }
+    c += __shfl_xor_sync(0xffffffffu, c, 2);
+    c += __shfl_xor_sync(0xffffffffu, c, 1);
+    if ((lane & 3) == 0) sh.part[warp][((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1)] = c;
+    __syncthreads();
+    double* parts = pl.parts + (size_t)parity * kSums * kSlots;
+    target += gridDim.x;
+    int bad = 0;
+    if (warp == 0) {
+        const int q = lane & 7, g = lane >> 3;
+        double t = (sh.part[4 * g][q] + sh.part[4 * g + 1][q]) + (sh.part[4 * g + 2][q] + sh.part[4 * g + 3][q]);
+        t += __shfl_xor_sync(0xffffffffu, t, 8);
+        t += __shfl_xor_sync(0xffffffffu, t, 16);
+        if (lane < kSums) parts[q * kSlots + blockIdx.x] = t;
+        __syncwarp();
+        if (lane == 0) bad = !arrive_and_wait(pl.arrivals, target, err, lim);
+    }
+    if (__syncthreads_or(bad)) return false;
+    if (warp < kSums) {
+        double t[kSlots / 32];
+#pragma unroll
+        for (int k = 0; k < kSlots / 32; ++k) {
+            const int i = lane + 32 * k;
+            t[k] = i < (int)gridDim.x ? __ldcg(parts + warp * kSlots + i) : 0.0;
+        }
+        double sum = 0.0;
+#pragma unroll
+        for (int k = 0; k < kSlots / 32; ++k) sum += t[k];
+        sum = warp_sum(sum);
+        if (lane == 0) sh.total[warp] = sum;
+    }
+    __syncthreads();
+    return true;
+}
+
+// alpha as a pair of float32 (high and low part) for advance()
+struct Alpha {
+    float hi, lo;
+};
+__device__ __forceinline__ Alpha split(double alpha) {
+    Alpha a;
+    a.hi = (float)alpha;
+    a.lo = (float)(alpha - (double)a.hi);
+    return a;
+}
+
+// r' = r - alpha A p, z' = D r', p' = z' + beta p of a row from its record
+// {r, p, A p, 1/diag}.  Every row that needs p' of a neighbour forms it, so the
+// conversions to float64 that r' would take (8.5 cycles of a scheduler each, three for
+// r' alone) weigh more than the sum: r' is taken from the exact product and sum in
+// float32 pairs instead (Dekker 1971, Knuth's two-sum), right to about 2^-45 before its one
+// rounding.  z' is one rounding of an exact product in either form.
+__device__ __forceinline__ void advance(const float4& f, const Alpha& alpha, float beta, float& r, float& z, float& p) {
+    const float h = __fmul_rn(alpha.hi, f.z);
+    const float l = __fmaf_rn(alpha.lo, f.z, __fmaf_rn(alpha.hi, f.z, -h));
+    const float s = __fsub_rn(f.x, h);
+    const float t = __fsub_rn(s, f.x);
+    const float e = __fsub_rn(__fsub_rn(f.x, __fsub_rn(s, t)), __fadd_rn(h, t));
+    r = __fadd_rn(s, __fsub_rn(e, l));
+    z = __fmul_rn(f.w, r);
+    p = __fmaf_rn(beta, f.y, z);
+}
+
+// the sums of one CG pass for a row
+__device__ __forceinline__ void pass_sums(double (&s)[kSums], float r, float z, float p, float ap, float di) {
+    const double d_ap = (double)ap, dap = (double)di * d_ap, dr = (double)di * (double)r;
+    s[0] += (double)p * d_ap;
+    s[1] += dr * d_ap;
+    s[2] += dap * d_ap;
+    s[3] += dr * dap;
+    s[4] += dap * dap;
+    s[5] += (double)r * (double)z;
+    s[6] += (double)z * (double)z;
+}
+
+// copy `bytes` (a multiple of 64; both sides 16-byte aligned) into shared memory, whole block
+__device__ __forceinline__ void hold(void* dst, const void* src, size_t bytes) {
+    for (size_t i = threadIdx.x; i < bytes / 16; i += kThreads)
+        static_cast<uint4*>(dst)[i] = static_cast<const uint4*>(src)[i];
+}
+
+// The block's part of the matrix in shared memory and where its neighbours' values are.
+template <typename IDX>
+struct Rows {
+    const IDX* col;       // int16: column - row; int32: column
+    const float *m, *k, *a;
+    int row0, rows;
+    float cm;
+    __device__ __forceinline__ int column(int e, int i) const {
+        return sizeof(IDX) == 2 ? row0 + i + (int)col[e] : (int)col[e];
+    }
+    // a neighbour's value: the block's own rows from shared memory, others through L1
+    template <class T>
+    __device__ __forceinline__ T value(const T* own, const T* all, int c) const {
+        const int l = c - row0;
+        const T* p = (unsigned)l < (unsigned)rows ? own + l : all + c;
+        return *p;
+    }
+};
+
+// Entries 0 .. w-1 of a row, C at a time, without branches: entries past the end
+// repeat the last one with a coefficient of zero.  All C gathers are in flight
+// before the first is used.
+template <int C, bool ASPLIT, typename IDX>
+__device__ __forceinline__ void row_rhs(const Rows<IDX>& R, const float4* own, const float4* all, int base, int w, int i,
+                                        float& mb, float& ku, double& ax) {
+    for (int k0 = 0; k0 < w; k0 += C) {
+        float4 q[C];
+#pragma unroll
+        for (int j = 0; j < C; ++j) q[j] = R.value(own, all, R.column(base + min(k0 + j, w - 1) * TCB_SLICE, i));
+#pragma unroll
+        for (int j = 0; j < C; ++j) {
+            const bool ok = k0 + j < w;
+            const int e = base + min(k0 + j, w - 1) * TCB_SLICE;
+            const float m = ok ? R.m[e] : 0.0f, k = ok ? R.k[e] : 0.0f;
+            float a;
+            if constexpr (ASPLIT) a = __fadd_rn(__fmul_rn(m, R.cm), k);
+            else a = ok ? R.a[e] : 0.0f;
+            mb = __fmaf_rn(m, q[j].x, mb);
+            ku = __fmaf_rn(k, q[j].y, ku);
+            ax += (double)a * (double)q[j].z;
+        }
+    }
+}
+
+template <bool ASPLIT, typename IDX>
+__device__ __forceinline__ float coefficient(const Rows<IDX>& R, int e) {
+    if constexpr (ASPLIT) return __fadd_rn(__fmul_rn(R.m[e], R.cm), R.k[e]);
+    else return R.a[e];
+}
+
+template <int C, bool ASPLIT, typename IDX>
+__device__ __forceinline__ double row_first(const Rows<IDX>& R, const float* own, const float* all, int base, int w, int i) {
+    double acc = 0.0;
+    for (int k0 = 0; k0 < w; k0 += C) {
+        float z[C];
+#pragma unroll
+        for (int j = 0; j < C; ++j) z[j] = R.value(own, all, R.column(base + min(k0 + j, w - 1) * TCB_SLICE, i));
+#pragma unroll
+        for (int j = 0; j < C; ++j) {
+            const float a = coefficient<ASPLIT>(R, base + min(k0 + j, w - 1) * TCB_SLICE);
+            acc += (double)(k0 + j < w ? a : 0.0f) * (double)z[j];
+        }
+    }
+    return acc;
+}
+
+template <int C, bool ASPLIT, typename IDX>
+__device__ __forceinline__ double row_next(const Rows<IDX>& R, const float4* own, const float4* all, int base, int w, int i,
+                                           const Alpha& alpha, float beta) {
+    double acc = 0.0;
+    for (int k0 = 0; k0 < w; k0 += C) {
+        float4 f[C];
+#pragma unroll
+        for (int j = 0; j < C; ++j) f[j] = R.value(own, all, R.column(base + min(k0 + j, w - 1) * TCB_SLICE, i));
+#pragma unroll
+        for (int j = 0; j < C; ++j) {
+            const float a = coefficient<ASPLIT>(R, base + min(k0 + j, w - 1) * TCB_SLICE);
+            float r, z, p;
+            advance(f[j], alpha, beta, r, z, p);
+            acc += (double)(k0 + j < w ? a : 0.0f) * (double)p;
+        }
+    }
+    return acc;
+}
+
+template <typename IDX, bool ASPLIT, class ION>
+__global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, const IDX* __restrict__ col, StepsPlan pl,
+                                                                 ION ion) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ Shared sh;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t s_begin = (int64_t)blockIdx.x * d.n_slices / gridDim.x;
+    const int64_t s_end = (int64_t)(blockIdx.x + 1) * d.n_slices / gridDim.x;
+    const int slices = (int)(s_end - s_begin);
+    const int row0 = (int)s_begin * TCB_SLICE;
+    const int rows = (int)((d.n < s_end * TCB_SLICE ? d.n : s_end * TCB_SLICE) - row0);
+    int32_t* err = d.counter + 1;
+    const int first_step = d.counter[0];
+    uint32_t arrived = *pl.base;
+    int parity = 0;
+    if (*(volatile int32_t*)err != 0) return;
+
+    // ---- shared memory (steps_layout): records, solutions, z, slice offsets, matrix, ionic state
+    const int cap = pl.cap_rows;
+    float4* rec0 = reinterpret_cast<float4*>(smem);
+    float4* rec1 = rec0 + cap;
+    float* sx = reinterpret_cast<float*>(rec1 + cap);
+    float* sxp = sx + cap;
+    float* sz = sxp + cap;
+    int* off = reinterpret_cast<int*>(sz + cap);
+    unsigned char* held = smem + pl.held_at;
+    const size_t vals = (size_t)pl.cap_entries * 4;
+    float* sm = reinterpret_cast<float*>(held);
+    float* sk = reinterpret_cast<float*>(held + vals);
+    float* sa = ASPLIT ? sk : reinterpret_cast<float*>(held + 2 * vals);
+    IDX* sc = reinterpret_cast<IDX*>(held + (ASPLIT ? 2 : 3) * vals);
+    float* ss = reinterpret_cast<float*>(smem + pl.state_at);
+    const int64_t e0 = d.slice_ptr[s_begin];
+    const size_t ent = (size_t)(d.slice_ptr[s_end] - e0);   // multiple of 32, at most cap_entries
+    hold(sc, col + e0, ent * sizeof(IDX));
+    hold(sm, d.mv + e0, ent * 4);
+    hold(sk, d.kv + e0, ent * 4);
+    if (!ASPLIT) hold(sa, d.av + e0, ent * 4);
+    const bool state_held = pl.state_at != 0;
+    if constexpr (ION::kIonic) {
+        if (state_held)
+            for (int k = 0; k < ION::kStates; ++k)
+                for (int i = threadIdx.x; i < rows; i += kThreads) ss[k * cap + i] = d.state[k * d.n_pad + row0 + i];
+    }
+    for (int i = threadIdx.x; i <= slices; i += kThreads) off[i] = (int)(d.slice_ptr[s_begin + i] - e0);
+    for (int i = threadIdx.x; i < rows; i += kThreads) {
+        sx[i] = d.x[ring_cur(first_step) * d.n_pad + row0 + i];
+        sxp[i] = d.x[ring_prev(first_step) * d.n_pad + row0 + i];
+        rec0[i].w = d.dinv[row0 + i];
+    }
+    __syncthreads();
+
+    const Rows<IDX> R{sc, sm, sk, sa, row0, rows, d.cm};
+    const bool lg = d.linear_guess != 0;
+    float* zg = d.r;
+    float4* q4 = pl.rec[1];        // {b', u, x0, -}; read before the first pass that writes rec[1]
+    const int last_step = first_step + pl.n_steps;
+    for (int n = first_step; n < last_step; ++n) {
+        // ---- ionic update of the block's rows, b', guess (monodomain.py:117-128, solver.py:35-38)
+        {
+            StepView sv;
+            if constexpr (ION::kIonic) sv = step_view(d, n);
+            for (int i = threadIdx.x; i < rows; i += kThreads) {
+                const float u = sx[i];
+                float bp;
+                if constexpr (ION::kIonic) {
+                    using M = typename ION::Model;
+                    using Q = typename ION::Policy;
+                    const int row = row0 + i;
+                    if (sv.do_atrt) at_rt_update(u, sv.t_prev, d.at, d.rt, row);
+                    if (sv.snap) sv.snap[row] = u;
+                    float s[M::kStates];
+                    if (state_held) {
+#pragma unroll
+                        for (int k = 0; k < M::kStates; ++k) s[k] = ss[k * cap + i];
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < M::kStates; ++k) s[k] = d.state[k * d.n_pad + row];
+                    }
+                    const float dV = M::template step<Q>(u, s, ion.c, ion.T, M::node_g(ion.c, d.node_params, d.n_pad, row));
+                    if (state_held) {
+#pragma unroll
+                        for (int k = 0; k < M::kStates; ++k) ss[k * cap + i] = s[k];
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < M::kStates; ++k) d.state[k * d.n_pad + row] = s[k];
+                    }
+                    bp = u * d.cm + d.dt * Q::div(dV, 100.0f);
+                    if (sv.smask) {
+                        const uint32_t bits = d.stim_bits[row] & sv.smask;
+                        if (bits) bp = bp + d.dt * Q::div(stim_sum(d, sv.smask, bits), 100.0f);
+                    }
+                } else {
+                    bp = d.bp[row0 + i];
+                }
+                const float4 q = make_float4(bp, u, lg ? 2.0f * u - sxp[i] : u, 0.0f);
+                rec1[i] = q;
+                q4[row0 + i] = q;
+            }
+        }
+        if (!barrier(pl, arrived, err, d.wait)) return;
+
+        // ---- right-hand side, r0, z0 (monodomain.py:130-131, solver.py:46-55)
+        double sums[kSums];
+#pragma unroll
+        for (int j = 0; j < kSums; ++j) sums[j] = 0.0;
+        for (int s = warp; s < slices; s += kWarps) {
+            const int i = s * TCB_SLICE + lane;
+            if (i >= rows) continue;
+            const int base = off[s] + lane, w = (off[s + 1] - off[s]) / TCB_SLICE;
+            float mb = 0.0f, ku = 0.0f;
+            double ax = 0.0;
+            if (w <= 8) row_rhs<8, ASPLIT>(R, rec1, q4, base, w, i, mb, ku, ax);
+            else row_rhs<16, ASPLIT>(R, rec1, q4, base, w, i, mb, ku, ax);
+            const float4 own = rec1[i];
+            sxp[i] = own.y;
+            sx[i] = own.z;
+            const float rhs = mb - ku;
+            const float di = rec0[i].w;
+            const float r = (float)((double)rhs - ax);
+            const float z = __fmul_rn(di, r);
+            rec0[i].x = r;
+            sz[i] = z;
+            zg[row0 + i] = z;
+            const double db = (double)di * (double)rhs;
+            sums[7] += db * db;
+        }
+        if (!barrier(pl, arrived, err, d.wait)) return;
+
+        int it = 0;
+        Alpha alpha = {0.0f, 0.0f};
+        double b_norm = 0.0;
+        float beta = 0.0f;
+        while (it < d.max_iter) {
+            // ---- p, A p; the sums that give alpha, beta and the stopping test
+            float4* rout = (it & 1) ? rec1 : rec0;
+            const float4* rin = (it & 1) ? rec0 : rec1;
+            float4* gout = pl.rec[it & 1];
+            const float4* gin = pl.rec[(it & 1) ^ 1];
+            for (int s = warp; s < slices; s += kWarps) {
+                const int i = s * TCB_SLICE + lane;
+                if (i >= rows) continue;
+                const int base = off[s] + lane, w = (off[s + 1] - off[s]) / TCB_SLICE;
+                float r, z, p, ap, di;
+                if (it == 0) {
+                    r = rec0[i].x;
+                    di = rec0[i].w;
+                    p = z = sz[i];
+                    ap = (float)(w <= 8 ? row_first<8, ASPLIT>(R, sz, zg, base, w, i)
+                                        : row_first<16, ASPLIT>(R, sz, zg, base, w, i));
+                } else {
+                    const float4 f = rin[i];
+                    di = f.w;
+                    advance(f, alpha, beta, r, z, p);
+                    ap = (float)row_next<8, ASPLIT>(R, rin, gin, base, w, i, alpha, beta);
+                }
+                pass_sums(sums, r, z, p, ap, di);
+                const float4 out = make_float4(r, p, ap, di);
+                rout[i] = out;
+                gout[row0 + i] = out;
+            }
+            if (!barrier_sums(sums, sh, pl, arrived, parity ^= 1, err, d.wait)) return;
+            const double rz = sh.total[5];
+            if (it == 0) b_norm = sqrt(sh.total[7]);
+            const double al = rz / sh.total[0];
+            alpha = split(al);
+            const double zz = sh.total[6] - al * (2.0 * sh.total[3] - al * sh.total[4]);
+            const double rz1 = rz - al * (2.0 * sh.total[1] - al * sh.total[2]);
+            for (int s = warp; s < slices; s += kWarps) {
+                const int i = s * TCB_SLICE + lane;
+                if (i < rows) sx[i] = (float)((double)sx[i] + al * (double)rout[i].y);
+            }
+            const double zn = sqrt(zz < 0.0 ? 0.0 : zz);
+            if (zn < d.a_tol || (zn / b_norm) < d.r_tol) break;   // solver.py:66-69
+            beta = (float)(rz1 / rz);
+            ++it;
+#pragma unroll
+            for (int j = 0; j < kSums; ++j) sums[j] = 0.0;
+        }
+        // the last three solutions of the stretch go to the ring (the next launch
+        // needs two of them; a shorter stretch leaves the older slots as they are)
+        if (n >= last_step - 3) {
+            float* xout = d.x + ring_next(n) * d.n_pad + row0;
+            for (int s = warp; s < slices; s += kWarps) {
+                const int i = s * TCB_SLICE + lane;
+                if (i < rows) xout[i] = sx[i];
+            }
+        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) d.step_iters[n] = it;
+    }
+    if constexpr (ION::kIonic) {
+        if (state_held)
+            for (int k = 0; k < ION::kStates; ++k)
+                for (int i = threadIdx.x; i < rows; i += kThreads) d.state[k * d.n_pad + row0 + i] = ss[k * cap + i];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        d.counter[0] = last_step;
+        *pl.base = arrived;
+    }
+}
+
+// ---------------------------------------------------------------- launch
+struct StepsInfo {
+    int sms = 0, max_smem = 0;
+};
+const StepsInfo& steps_info() {
+    static StepsInfo infos[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    StepsInfo& si = infos[dev & 63];
+    if (si.sms == 0) {
+        cudaDeviceGetAttribute(&si.max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+        si.max_smem -= (int)sizeof(Shared) + 1024;
+        int sms = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        si.sms = sms;
+    }
+    return si;
+}
+
+constexpr int kMinSlices = 8;              // slices a block has at least
+constexpr int kHoldStateFrom = 4;          // shorter launches update the ionic state where it is
+constexpr int64_t kStepsPerLaunch = 128;   // about a millisecond or a few: other streams get their turn
+
+bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
+
+unsigned steps_blocks(const MonoDev& d) {
+    const int64_t nb = std::min<int64_t>(ceil_div(d.n_slices, kMinSlices), std::min(steps_info().sms, kSlots));
+    return (unsigned)std::max<int64_t>(nb, 1);
+}
+
+// Shared memory of a block with at most `entries` matrix entries; false where it
+// does not fit (the matrix has to; the ionic state stays in global memory if need be).
+bool steps_layout(const MonoDev& d, int64_t entries, int states, StepsPlan* pl) {
+    const size_t max = (size_t)steps_info().max_smem;
+    auto up = [](size_t b) { return (b + 127) / 128 * 128; };
+    const int64_t cap = ceil_div(d.n_slices, steps_blocks(d)) * TCB_SLICE;
+    const size_t fixed = (size_t)cap * 44 + up((size_t)(cap / TCB_SLICE + 1) * 4);
+    const size_t per_entry = (d.a_split ? 8 : 12) + (d.dcol ? 2 : 4);
+    const size_t matrix = up((size_t)entries * per_entry), state = (size_t)cap * 4 * states;
+    if (cap > 16384 || entries > (1 << 20) || fixed + matrix > max) return false;
+    pl->cap_rows = (int)cap;
+    pl->cap_entries = (int)entries;
+    pl->held_at = (int)fixed;
+    pl->state_at = states > 0 && fixed + matrix + state <= max ? (int)(fixed + matrix) : 0;
+    pl->smem_bytes = (int)(fixed + matrix + (pl->state_at ? state : 0));
+    return true;
+}
+
+// false where the step-by-step launches run instead
+bool steps_plan(const tcb_mono* m, const MonoDev& d, int states, StepsPlan* pl) {
+    if (!m->work || m->work_entries <= 0 || m->fused_step != 0 || cg_forced_fallback()) return false;
+    if (!steps_layout(d, m->work_entries, states, pl)) return false;
+    unsigned char* w = static_cast<unsigned char*>(m->work);
+    pl->arrivals = reinterpret_cast<uint32_t*>(w);
+    pl->base = reinterpret_cast<uint32_t*>(w + kHeadBytes / 2);
+    pl->parts = reinterpret_cast<double*>(w + kHeadBytes);
+    pl->rec[0] = reinterpret_cast<float4*>(w + kHeadBytes + kPartBytes);
+    pl->rec[1] = pl->rec[0] + d.n_pad;
+    return true;
+}
+
+template <typename IDX, bool ASPLIT, class ION>
+int launch(const MonoDev& d, const IDX* col, const StepsPlan& pl, const ION& ion, cudaStream_t s) {
+    static bool configured[64] = {};
+    int dev = 0;
+    TCB_CHECK_CUDA(cudaGetDevice(&dev));
+    const void* fn = (const void*)mono_steps_kernel<IDX, ASPLIT, ION>;
+    if (!configured[dev & 63]) {
+        TCB_CHECK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, steps_info().max_smem));
+        configured[dev & 63] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(steps_blocks(d));
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = (size_t)pl.smem_bytes;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    void* args[] = {const_cast<MonoDev*>(&d), &col, const_cast<StepsPlan*>(&pl), const_cast<ION*>(&ion)};
+    cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
+    if (e != cudaSuccess) return cuda_fail(e, "steps kernel launch");
+    return 1;
+}
+
+template <class ION>
+int launch_any(const MonoDev& d, const StepsPlan& pl, const ION& ion, cudaStream_t s) {
+    if (d.dcol)
+        return d.a_split ? launch<int16_t, true, ION>(d, d.dcol, pl, ion, s) : launch<int16_t, false, ION>(d, d.dcol, pl, ion, s);
+    return d.a_split ? launch<int32_t, true, ION>(d, d.col, pl, ion, s) : launch<int32_t, false, ION>(d, d.col, pl, ion, s);
+}
+
+template <class M, class Q>
+int launch_model(const tcb_mono* m, const MonoDev& d, const StepsPlan& pl, cudaStream_t s) {
+    Ionic<M, Q> ion;
+    ion.c = M::derive(m->params);
+    ion.T = M::tables(m->tables, m->params);
+    return launch_any(d, pl, ion, s);
+}
+
+}  // namespace
+
+// Steps [counter, counter + n_steps) as persistent launches of up to kStepsPerLaunch steps:
+// 1 = launched, 0 = not applicable (the caller launches step by step), < 0 = error
+int launch_steps(const tcb_mono* m, const MonoDev& d, int64_t n_steps, bool ionic, cudaStream_t s) {
+    StepsPlan pl;
+    constexpr int kStates[4] = {0, MS::kStates, TTP::kStates, CRN::kStates};
+    if (ionic && (m->model < TCB_MODEL_MS || m->model > TCB_MODEL_CRN)) return 0;
+    if (!steps_plan(m, d, ionic ? kStates[m->model] : 0, &pl)) return 0;
+    int32_t count, v, b, fast = 0, staged;
+    if (ionic) {
+        // the chosen instance's division policy
+        const int st = tcb_ionic_variant(m->model, m->ionic_variant, &count, &v, &b, &fast, &staged);
+        if (st) return st;
+    }
+    for (int64_t done = 0; done < n_steps; done += kStepsPerLaunch) {
+        pl.n_steps = (int)std::min(kStepsPerLaunch, n_steps - done);
+        if (pl.n_steps < kHoldStateFrom && pl.state_at) {
+            pl.smem_bytes = pl.state_at;
+            pl.state_at = 0;
+        }
+        int st;
+        if (!ionic) st = launch_any(d, pl, GivenRhs{}, s);
+        else if (m->model == TCB_MODEL_MS) st = launch_model<MS, QExact>(m, d, pl, s);
+        else if (m->model == TCB_MODEL_TTP) st = fast ? launch_model<TTP, QFast>(m, d, pl, s) : launch_model<TTP, QExact>(m, d, pl, s);
+        else st = fast ? launch_model<CRN, QFast>(m, d, pl, s) : launch_model<CRN, QExact>(m, d, pl, s);
+        if (st != 1) return st;
+    }
+    return 1;
+}
+
+}  // namespace tcb
+
+extern "C" int64_t tcb_mono_work_bytes(const tcb_mono* m, int32_t* entries, void* stream) {
+    using namespace tcb;
+    const int st = validate_mono(m);
+    if (st) return st;
+    if (!entries) return fail(TCB_EINVAL, "tcb_mono_work_bytes: null output");
+    *entries = 0;
+    const MonoDev d = make_dev(m);
+    StepsPlan pl;
+    // (16-byte copies of the matrix; nothing to ask the device for where even an empty matrix would not fit)
+    if (m->fused_step != 0 || cg_forced_fallback() || !aligned16(d.dcol ? (const void*)d.dcol : (const void*)d.col) ||
+        !aligned16(d.mv) || !aligned16(d.kv) || !aligned16(d.av) || !steps_layout(d, TCB_SLICE * ceil_div(d.n_slices, steps_blocks(d)), 0, &pl))
+        return 0;
+    std::vector<int64_t> sp((size_t)d.n_slices + 1);
+    cudaStream_t s = as_stream(stream);
+    TCB_CHECK_CUDA(cudaMemcpyAsync(sp.data(), d.slice_ptr, sp.size() * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    TCB_CHECK_CUDA(cudaStreamSynchronize(s));
+    const int64_t nb = steps_blocks(d);
+    int64_t most = 0;
+    for (int64_t b = 0; b < nb; ++b) most = std::max(most, sp[(b + 1) * d.n_slices / nb] - sp[b * d.n_slices / nb]);
+    if (!steps_layout(d, most, 0, &pl)) return 0;
+    *entries = (int32_t)most;
+    return (int64_t)(kHeadBytes + kPartBytes + 2 * (size_t)m->n_pad * sizeof(float4));
+}

@@ -40,6 +40,20 @@ def rcm_order(elems, n_nodes):
     return np.asarray(reverse_cuthill_mckee(g, symmetric_mode=True), dtype=np.int64)
 
 
+def _work_buffer(m, device):
+    """Zeroed ``tcb_mono.work`` of the struct ``m`` (set in it), or None where steps are
+    launched one by one in any case."""
+    entries = C.c_int32()
+    nbytes = int(_lib.load().tcb_mono_work_bytes(C.byref(m), C.byref(entries), stream_ptr()))
+    if nbytes < 0:
+        check(nbytes)
+    if nbytes == 0:
+        return None
+    work = torch.zeros(nbytes, device=device, dtype=torch.uint8)
+    m.work, m.work_entries = ptr(work), entries.value
+    return work
+
+
 class Monodomain:
     def __init__(self, ionic_model, T, dt, device=None, dtype=None, reorder=False):
         self.device = torch.device(device) if device is not None else get_device()
@@ -241,9 +255,18 @@ class Monodomain:
         if (m.node_params or None) != want:
             m.node_params = want
 
+    def _sync_launch(self):
+        """What a launch reads besides the buffers of ``_setup``: the per-node parameters,
+        and the exchange buffer of the many-steps-per-launch kernel where it applies
+        (allocated when the simulation is first stepped by itself; batches do without)."""
+        self._sync_node_params()
+        sim = self._sim
+        if "work" not in sim:
+            sim["work"] = _work_buffer(sim["struct"], self.device)
+
     def run_steps(self, n_steps, stream=None):
         """Advance the prepared simulation by ``n_steps`` steps (asynchronous)."""
-        self._sync_node_params()
+        self._sync_launch()
         sim = self._sim
         a = sim["next_step"]
         b = min(a + n_steps, self.nt + 1)
@@ -271,7 +294,7 @@ class Monodomain:
     def capture_steps(self, n_steps):
         """Record ``n_steps`` steps of the prepared simulation in a CUDA graph;
         returns a callable replaying them (with the step bookkeeping)."""
-        self._sync_node_params()
+        self._sync_launch()
         sim = self._sim
         lib = _lib.load()
         # the first launch on a device configures kernel attributes: keep it outside capture
@@ -475,6 +498,7 @@ class Monodomain:
         m.step_iters, m.counter = ptr(buf["step_iters"]), ptr(buf["counter"])
         m.scratch, m.barrier = ptr(buf["scratch"]), ptr(buf["barrier"])
         m.params = buf["params"].ctypes.data
+        buf["work"] = _work_buffer(m, dev)
         lib = _lib.load()
         out = torch.empty((F, n), **f32)
         for k in range(F):

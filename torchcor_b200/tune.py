@@ -240,9 +240,13 @@ def tune_single(sim, steps=5, cache=None, force=False):
     key = single_key(sim.device, int(m.n_nodes), int(sim.system.nnz), model.name)
     hit = None if force else cache.get(key)
     shapes = _lib.ionic_variants(model.model_id)
+    lib = _lib.load()
+    # where a stretch of steps is one persistent launch (tcb_mono.work), the fused step is no candidate
+    m.fused_step = 0
+    stretches = int(lib.tcb_mono_work_bytes(C.byref(m), C.byref(C.c_int32()), _lib.stream_ptr())) > 0
     if hit is not None and 0 <= int(hit.get("ionic_variant", 0)) <= len(shapes):
         m.ionic_variant, m.cg_per_sm = int(hit["ionic_variant"]), int(hit.get("cg_per_sm", 0))
-        m.fused_step = int(hit.get("fused_step", 0))
+        m.fused_step = 0 if stretches else int(hit.get("fused_step", 0))
         return dict(hit, cached=True)
     first = d["next_step"]
     if sim.nt + 1 - first < steps + 1:
@@ -257,9 +261,8 @@ def tune_single(sim, steps=5, cache=None, force=False):
     best_ion = min(t_ion, key=t_ion.get)
     # the step as two launches (ionic + CG) or as one (fused), for each CG blocks per SM
     t_step = {}
-    lib = _lib.load()
     for c in (2, 1):
-        for fused in (0, 1):
+        for fused in (0,) if stretches else (0, 1):
             st = scratch.struct
             st.ionic_variant, st.cg_per_sm, st.fused_step = best_ion, c, fused
             if lib.tcb_mono_cg_kernel(C.byref(st)) != (2 if fused else 1):   # not resident / not fusable
