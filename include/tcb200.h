@@ -64,6 +64,11 @@ int tcb_pattern_build(const int32_t* elems, int64_t n_elems, int32_t k, int64_t 
 /* Sliced-ELL layout of a CSR pattern: slice_ptr[n_slices+1] entry offsets
  * (each slice holds 32 * its widest row entries).  Host code. */
 int tcb_sell_layout(const int32_t* rowptr, int64_t n_rows, int64_t* slice_ptr, int64_t* n_entries);
+/* The same layout from a rowptr on the device; `scratch` holds tcb_sell_layout_scratch(n_rows)
+ * int64 values.  Synchronises the stream (*n_entries is on the host). */
+int64_t tcb_sell_layout_scratch(int64_t n_rows);
+int tcb_sell_layout_device(const int32_t* rowptr, int64_t n_rows, int64_t* slice_ptr, int64_t* scratch,
+                           int64_t* n_entries, void* stream);
 
 /* ---------------------------------------------------------------- device ingest
  * Mesh ingest on the device (replaces MeshReader's np.loadtxt, mesh.py:26-63, and

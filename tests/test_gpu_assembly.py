@@ -1,0 +1,94 @@
+"""Assembly kernels at their edges: the device pattern's register sorts (32, 64,
+128 and 256 contributions a row, columns too far away for the 32-bit key, rows
+left to the shared-memory sort), the multi-block scans, the device layout of the
+sliced ELL and its packing, each against the host builder."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+NAMES = ("rowptr", "col", "slot_ptr", "slot_src", "diag")
+
+
+def _fans(k, degrees, rng):
+    """Elements of k nodes whose i-th hub node has degrees[i] of them; every node is in one."""
+    out, n = [], len(degrees)
+    for hub, deg in enumerate(degrees):
+        rim = np.arange(n, n + max(deg, k))
+        n += len(rim)
+        for i in range(deg):
+            el = [hub] + [int(rim[(i + j) % len(rim)]) for j in range(k - 1)]
+            out.append(rng.permutation(el))
+        out.append(rim[:k])                                # short fans: every rim node has an element
+        out.extend(rim[j: j + k] if j + k <= len(rim) else rim[-k:] for j in range(k, len(rim), k))
+    return rng.permutation(np.array(out, dtype=np.int32)), n
+
+
+def _equal(el, n, cuda):
+    from torchcor_b200.core.assemble import build_pattern, build_pattern_device
+    h = build_pattern(el, n)
+    g = build_pattern_device(torch.from_numpy(el).to(cuda), n)
+    assert g.nnz == h.nnz
+    for name in NAMES:
+        assert np.array_equal(g.host(name), h.host(name)), name
+    return h
+
+
+@pytest.mark.parametrize("k,degrees", [
+    (4, [1, 7, 8, 9, 15, 16, 17, 31, 32, 33, 63, 64, 65, 200, 255]),
+    (3, [1, 9, 10, 11, 20, 21, 22, 31, 32, 33, 63, 64, 65, 100, 340]),
+])
+def test_rows_of_every_sort(lib, cuda, k, degrees):
+    el, n = _fans(k, degrees, np.random.default_rng(k))
+    _equal(el, n, cuda)
+
+
+def test_far_columns_and_multi_block_scans(lib, cuda):
+    """A strip of triangles over 4.3 million nodes, some joined to nodes millions of
+    rows away: beyond the 22- and 23-bit column offsets of the register sorts."""
+    n = 4_300_001
+    i = np.arange(0, n - 2, 2, dtype=np.int64)
+    strip = np.stack([i, i + 1, i + 2], 1)
+    far = np.array([(0, n - 1, 5), (7, n // 2, n - 3), (n - 2, 1, n // 3)], dtype=np.int64)
+    fan = np.array([(9, 20 + 2 * j, 4_200_000 + j) for j in range(45)], dtype=np.int64)
+    _equal(np.concatenate([strip, far, fan]).astype(np.int32), n, cuda)
+
+
+@pytest.mark.parametrize("n,widest", [(1, 1), (31, 5), (32, 7), (33, 40), (5000, 90), (300_000, 6)])
+def test_sliced_ell_on_the_device(lib, cuda, n, widest):
+    """Layout and packing against the host layout and a plain loop; rows of up to 90
+    entries make slices beyond what a warp stages."""
+    from torchcor_b200._lib import TCB_SLICE
+    from torchcor_b200.core.assemble import Pattern, _sliced_ell
+    rng = np.random.default_rng(n)
+    length = rng.integers(1, widest + 1, size=n)
+    rowptr = np.concatenate([[0], np.cumsum(length)]).astype(np.int32)
+    nnz = int(rowptr[-1])
+    col = rng.integers(0, n, size=nnz).astype(np.int32)
+    vals = [rng.normal(size=nnz).astype(np.float32) for _ in range(3)]
+    dev = [torch.from_numpy(a).to(cuda) for a in (rowptr, col, *vals)]
+    pat = Pattern(n, 4, dev[0], dev[1], None, None, None, n_nonzero=nnz)
+    ns, sp, scol, dcol, sell, flag = _sliced_ell(pat, dev[0], dev[1], dev[2:], cuda, torch.ones(1, device=cuda, dtype=torch.int32))
+    assert flag
+    want = np.empty(ns + 1, dtype=np.int64)
+    ne = C.c_int64()
+    assert lib.tcb_sell_layout(rowptr.ctypes.data, n, want.ctypes.data, C.byref(ne)) == 0
+    assert np.array_equal(sp.cpu().numpy(), want)
+    pc, pv = np.empty(ne.value, dtype=np.int32), [np.zeros(ne.value, dtype=np.float32) for _ in range(3)]
+    for s in range(ns):
+        w = int(want[s + 1] - want[s]) // TCB_SLICE
+        for lane in range(TCB_SLICE):
+            row = s * TCB_SLICE + lane
+            at = want[s] + lane + TCB_SLICE * np.arange(w)
+            pc[at] = row if row < n else 0
+            if row < n:
+                b, m = rowptr[row], length[row]
+                pc[at[:m]] = col[b:b + m]
+                for p, v in zip(pv, vals):
+                    p[at[:m]] = v[b:b + m]
+    assert np.array_equal(scol.cpu().numpy(), pc)
+    for t, p in zip(sell, pv):
+        assert np.array_equal(t.cpu().numpy(), p)

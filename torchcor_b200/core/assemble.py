@@ -145,6 +145,34 @@ class System:
         return torch.sparse_csr_tensor(self.rowptr, self.col, values, size=(self.n, self.n))
 
 
+def _sliced_ell(pat, rowptr, col, values, dev, flag=None):
+    """Sliced-ELL copy of CSR values on the device: (n_slices, slice_ptr, columns, int16
+    column offsets or None, [values...], flag as a bool).  ``flag``: an int32 device scalar read in
+    the same synchronisation as the width of the columns."""
+    lib = _lib.load()
+    s = stream_ptr()
+    n = pat.n_nodes
+    n_slices = (n + _lib.TCB_SLICE - 1) // _lib.TCB_SLICE
+    slice_ptr = torch.empty(n_slices + 1, device=dev, dtype=torch.int64)
+    scratch = torch.empty(int(lib.tcb_sell_layout_scratch(n)), device=dev, dtype=torch.int64)
+    n_entries = C.c_int64()
+    check(lib.tcb_sell_layout_device(ptr(rowptr), n, ptr(slice_ptr), ptr(scratch), C.byref(n_entries), s))
+    ne = n_entries.value
+    sell_col = torch.empty(ne, device=dev, dtype=torch.int32)
+    sell = [torch.empty(ne, device=dev, dtype=torch.float32) for _ in values]
+    vin = (C.c_void_p * len(values))(*[ptr(t) for t in values])
+    vout = (C.c_void_p * len(values))(*[ptr(t) for t in sell])
+    check(lib.tcb_sell_pack(n, ptr(rowptr), ptr(col), ptr(slice_ptr), n_slices, len(values), vin, ptr(sell_col), vout, s))
+    # int16 column offsets when the mesh ordering keeps every |col - row| < 32768
+    dcol = torch.empty(ne, device=dev, dtype=torch.int16)
+    flags = torch.zeros(2, device=dev, dtype=torch.int32)
+    check(lib.tcb_sell_delta(n, ptr(slice_ptr), n_slices, ptr(sell_col), ptr(dcol), ptr(flags), s))
+    if flag is not None:
+        flags[1:] = flag
+    width, flag = flags.tolist()
+    return n_slices, slice_ptr, sell_col, dcol if width < 32768 else None, sell, bool(flag)
+
+
 def assemble_system(nodes, elems_np, sl, st, fibres, dt, chi=140, cm=0.01, theta=0.5, pattern=None) -> System:
     """Assemble M, K/chi, A and the Jacobi preconditioner (monodomain.py:83-106)."""
     lib = _lib.load()
@@ -170,30 +198,11 @@ def assemble_system(nodes, elems_np, sl, st, fibres, dt, chi=140, cm=0.01, theta
     a_split = torch.ones(1, device=dev, dtype=torch.int32)
     check(lib.tcb_assemble_system(nnz, n, n_pad, ptr(diag), ptr(k_val), ptr(m_val), float(chi), float(cm), float(dt),
                                   float(theta), ptr(a_val), ptr(krhs), ptr(d_inv), ptr(a_split), s))
-    # sliced ELL
-    n_slices = (n + _lib.TCB_SLICE - 1) // _lib.TCB_SLICE
-    sp = np.empty(n_slices + 1, dtype=np.int64)
-    n_entries = C.c_int64()
-    rowptr_host = pat.host("rowptr")           # keep the host copy alive across the call
-    check(lib.tcb_sell_layout(ptr(rowptr_host), n, ptr(sp), C.byref(n_entries)))
-    rowptr = pat.on("rowptr", dev)
-    col = pat.on("col", dev)
-    slice_ptr = torch.from_numpy(sp).to(dev)
-    ne = n_entries.value
-    sell_col = torch.empty(ne, device=dev, dtype=torch.int32)
-    sell = [torch.empty(ne, device=dev, dtype=torch.float32) for _ in range(3)]
-    vin = (C.c_void_p * 3)(ptr(m_val), ptr(krhs), ptr(a_val))
-    vout = (C.c_void_p * 3)(*[ptr(t) for t in sell])
-    check(lib.tcb_sell_pack(n, ptr(rowptr), ptr(col), ptr(slice_ptr), n_slices, 3, vin, ptr(sell_col), vout, s))
-    # int16 column offsets when the mesh ordering keeps every |col - row| < 32768
-    dcol = torch.empty(ne, device=dev, dtype=torch.int16)
-    mx = torch.zeros(1, device=dev, dtype=torch.int32)
-    check(lib.tcb_sell_delta(n, ptr(slice_ptr), n_slices, ptr(sell_col), ptr(dcol), ptr(mx), s))
-    if int(mx.item()) >= 32768:
-        dcol = None
+    rowptr, col = pat.on("rowptr", dev), pat.on("col", dev)
+    n_slices, slice_ptr, sell_col, dcol, sell, split = _sliced_ell(pat, rowptr, col, [m_val, krhs, a_val], dev, a_split)
     return System(n=n, n_pad=n_pad, nnz=nnz, rowptr=rowptr, col=col, m_val=m_val, k_val=k_val, a_val=a_val,
                   krhs_val=krhs, d_inv=d_inv, n_slices=n_slices, slice_ptr=slice_ptr, sell_col=sell_col,
-                  sell_m=sell[0], sell_k=sell[1], sell_a=sell[2], sell_dcol=dcol, a_split=bool(a_split.item()))
+                  sell_m=sell[0], sell_k=sell[1], sell_a=sell[2], sell_dcol=dcol, a_split=split)
 
 
 def assemble_phie(nodes, elems_np, sl_i, st_i, sl_e, st_e, fibres) -> System:
@@ -228,25 +237,8 @@ def assemble_phie(nodes, elems_np, sl_i, st_i, sl_e, st_e, fibres) -> System:
     d_inv = torch.empty(n_pad, device=dev, dtype=torch.float32)
     check(lib.tcb_assemble_system(nnz, n, n_pad, ptr(diag), ptr(kie), ptr(mass), 1.0, 0.0, 1.0, 1.0,
                                   ptr(a_val), ptr(zero), ptr(d_inv), None, s))
-    n_slices = (n + _lib.TCB_SLICE - 1) // _lib.TCB_SLICE
-    sp = np.empty(n_slices + 1, dtype=np.int64)
-    n_entries = C.c_int64()
-    rowptr_host = pat.host("rowptr")           # keep the host copy alive across the call
-    check(lib.tcb_sell_layout(ptr(rowptr_host), n, ptr(sp), C.byref(n_entries)))
-    rowptr = pat.on("rowptr", dev)
-    col = pat.on("col", dev)
-    slice_ptr = torch.from_numpy(sp).to(dev)
-    ne = n_entries.value
-    sell_col = torch.empty(ne, device=dev, dtype=torch.int32)
-    sell = [torch.empty(ne, device=dev, dtype=torch.float32) for _ in range(3)]
-    vin = (C.c_void_p * 3)(ptr(ki), ptr(zero), ptr(a_val))
-    vout = (C.c_void_p * 3)(*[ptr(t) for t in sell])
-    check(lib.tcb_sell_pack(n, ptr(rowptr), ptr(col), ptr(slice_ptr), n_slices, 3, vin, ptr(sell_col), vout, s))
-    dcol = torch.empty(ne, device=dev, dtype=torch.int16)
-    mx = torch.zeros(1, device=dev, dtype=torch.int32)
-    check(lib.tcb_sell_delta(n, ptr(slice_ptr), n_slices, ptr(sell_col), ptr(dcol), ptr(mx), s))
-    if int(mx.item()) >= 32768:
-        dcol = None
+    rowptr, col = pat.on("rowptr", dev), pat.on("col", dev)
+    n_slices, slice_ptr, sell_col, dcol, sell, _ = _sliced_ell(pat, rowptr, col, [ki, zero, a_val], dev)
     return System(n=n, n_pad=n_pad, nnz=nnz, rowptr=rowptr, col=col, m_val=ki, k_val=kie, a_val=a_val,
                   krhs_val=zero, d_inv=d_inv, n_slices=n_slices, slice_ptr=slice_ptr, sell_col=sell_col,
                   sell_m=sell[0], sell_k=sell[1], sell_a=sell[2], sell_dcol=dcol, a_split=False)

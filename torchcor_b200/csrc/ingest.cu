@@ -14,14 +14,15 @@
 // exponents, malformed fields) are counted in `bad`; the caller then parses the
 // file on the host instead.
 //
-// Pattern: every element contribution (a, b, e) becomes the key
-// (col << 32 | order), order = (a*k + b)*E + e its position in the reference's
-// COO list, bucketed by row, sorted per row (bitonic, one warp per row in
-// shared memory) and compacted: the unique columns are the CSR columns and, for
-// each slot, its contributions in COO order -- the host builder's output, bit
-// for bit.
+// Pattern: every element corner is put into its node's segment; one warp per row
+// expands them into the row's contributions (column, position in the reference's
+// COO list (a*k + b)*E + e), sorts and compacts them: the unique columns are the CSR
+// columns and, for each slot, its contributions in COO order -- the host builder's
+// output, bit for bit.
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "tcb_internal.h"
 
@@ -54,29 +55,111 @@ __global__ void nl_count_kernel(const char* __restrict__ t, int64_t n, int64_t* 
     if (threadIdx.x == 0) block_cnt[blockIdx.x] = sh[0];
 }
 
-// exclusive scan of n values in place (one block, sequential over chunks)
-__global__ void scan_kernel(int64_t* __restrict__ v, int64_t n, int64_t* __restrict__ total) {
-    __shared__ int64_t sh[kScanThreads];
-    __shared__ int64_t carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (int64_t base = 0; base < n; base += kScanThreads) {
-        const int64_t i = base + threadIdx.x;
-        const int64_t x = i < n ? v[i] : 0;
-        sh[threadIdx.x] = x;
-        __syncthreads();
-        for (int o = 1; o < kScanThreads; o <<= 1) {
-            const int64_t y = threadIdx.x >= o ? sh[threadIdx.x - o] : 0;
-            __syncthreads();
-            sh[threadIdx.x] += y;
-            __syncthreads();
-        }
-        if (i < n) v[i] = carry + sh[threadIdx.x] - x;
-        __syncthreads();
-        if (threadIdx.x == kScanThreads - 1) carry += sh[kScanThreads - 1];
-        __syncthreads();
+// ---------------------------------------------------------------- exclusive scans
+// Counts (times mul) -> int64 offsets with the total behind the last one; in place
+// where input and output are the same int64 array.  A block takes kScanTile values,
+// kScanItems consecutive ones a thread.  Up to kScanOneBlock values one block walks the
+// tiles with a running carry; more take three launches (tile sums, their scan, the
+// tiles again), so that 531,441 counts take 11 us instead of the 820 us one block
+// took value by value with a barrier per doubling.
+constexpr int kScanItems = 8;
+constexpr int kScanTile = kScanThreads * kScanItems;
+constexpr int64_t kScanOneBlock = 4 * kScanTile;
+
+// exclusive prefix of v over the block; `total` = the block's sum.  sh: 33 values.
+__device__ __forceinline__ int64_t block_prefix(int64_t v, int64_t* sh, int64_t& total) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int64_t inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int64_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
     }
+    if (lane == 31) sh[warp] = inc;
+    __syncthreads();
+    if (warp == 0) {
+        const int64_t w = sh[lane];
+        int64_t x = w;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        sh[lane] = x - w;
+        if (lane == 31) sh[32] = x;
+    }
+    __syncthreads();
+    const int64_t r = sh[warp] + inc - v;
+    total = sh[32];
+    __syncthreads();
+    return r;
+}
+
+// offsets of the tile at `base`, on top of `carry`; returns the tile's sum
+template <typename T>
+__device__ __forceinline__ int64_t scan_tile(const T* v, int64_t* out, int64_t n, int64_t mul, int64_t base, int64_t carry,
+                                             int64_t* sh) {
+    int64_t x[kScanItems], sum = 0;
+#pragma unroll
+    for (int j = 0; j < kScanItems; ++j) {
+        const int64_t i = base + threadIdx.x * kScanItems + j;
+        x[j] = i < n ? (int64_t)v[i] * mul : 0;
+        sum += x[j];
+    }
+    int64_t total;
+    int64_t at = carry + block_prefix(sum, sh, total);
+#pragma unroll
+    for (int j = 0; j < kScanItems; ++j) {
+        const int64_t i = base + threadIdx.x * kScanItems + j;
+        if (i < n) out[i] = at;
+        at += x[j];
+    }
+    return total;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kScanThreads) scan_block_kernel(const T* v, int64_t* out, int64_t n, int64_t mul, int64_t* total) {
+    __shared__ int64_t sh[33];
+    int64_t carry = 0;
+    for (int64_t base = 0; base < n; base += kScanTile) carry += scan_tile(v, out, n, mul, base, carry, sh);
     if (threadIdx.x == 0 && total) *total = carry;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kScanThreads) scan_sums_kernel(const T* v, int64_t n, int64_t mul, int64_t* sums) {
+    __shared__ int64_t sh[33];
+    const int64_t base = (int64_t)blockIdx.x * kScanTile;
+    int64_t sum = 0;
+    for (int j = 0; j < kScanItems; ++j) {
+        const int64_t i = base + j * kScanThreads + threadIdx.x;
+        if (i < n) sum += (int64_t)v[i] * mul;
+    }
+    int64_t total;
+    block_prefix(sum, sh, total);
+    if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kScanThreads) scan_tiles_kernel(const T* v, int64_t* out, int64_t n, int64_t mul, const int64_t* sums) {
+    __shared__ int64_t sh[33];
+    scan_tile(v, out, n, mul, (int64_t)blockIdx.x * kScanTile, sums[blockIdx.x], sh);
+}
+
+inline int64_t scan_tiles(int64_t n) { return (n + kScanTile - 1) / kScanTile; }
+
+// out[0..n): offsets, *total: the sum (both on the device); tmp: scan_tiles(n) values of its own
+template <typename T>
+int scan(const T* v, int64_t* out, int64_t n, int64_t mul, int64_t* total, int64_t* tmp, cudaStream_t s) {
+    if (n <= kScanOneBlock || !tmp) {
+        scan_block_kernel<T><<<1, kScanThreads, 0, s>>>(v, out, n, mul, total);
+    } else {
+        const unsigned nb = (unsigned)scan_tiles(n);
+        scan_sums_kernel<T><<<nb, kScanThreads, 0, s>>>(v, n, mul, tmp);
+        scan_block_kernel<int64_t><<<1, kScanThreads, 0, s>>>(tmp, tmp, nb, 1, total);
+        scan_tiles_kernel<T><<<nb, kScanThreads, 0, s>>>(v, out, n, mul, tmp);
+    }
+    TCB_CHECK_LAUNCH("scan kernel");
+    return TCB_OK;
 }
 
 __global__ void nl_write_kernel(const char* __restrict__ t, int64_t n, const int64_t* __restrict__ block_off,
@@ -275,112 +358,252 @@ __global__ void pattern_count_kernel(const int32_t* __restrict__ el, int64_t E, 
             atomicExch(err, 1);
             return;
         }
-        atomicAdd(row_cnt + v, k);
+        atomicAdd(row_cnt + v, 1);
     }
 }
 
-__global__ void pattern_fill_kernel(const int32_t* __restrict__ el, int64_t E, int k, const int64_t* __restrict__ row_off,
+// e*k + a of every element corner, in its node's segment (any order; the segment
+// has room for k entries a corner, the first ones are used)
+__global__ void pattern_fill_kernel(const int32_t* __restrict__ el, int64_t E, int k, int64_t N, const int64_t* __restrict__ row_off,
                                     int32_t* __restrict__ fill, uint64_t* __restrict__ keys) {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= E) return;
     for (int a = 0; a < k; ++a) {
         const int32_t row = el[e * k + a];
-        const int64_t base = row_off[row] + atomicAdd(fill + row, k);
-        for (int b = 0; b < k; ++b) {
-            const uint64_t order = (uint64_t)(a * k + b) * (uint64_t)E + (uint64_t)e;
-            keys[base + b] = ((uint64_t)(uint32_t)el[e * k + b] << 32) | order;
-        }
+        if (row < 0 || row >= N) return;   // recorded by the count
+        keys[row_off[row] + atomicAdd(fill + row, 1)] = (uint64_t)(e * k + a);
     }
 }
 
-// one warp per row: bitonic sort of the row's keys in shared memory, then the
-// number of distinct columns
-__global__ void pattern_sort_kernel(const int64_t* __restrict__ row_off, int64_t N, uint64_t* __restrict__ keys,
-                                    int32_t* __restrict__ uniq, int32_t* __restrict__ err) {
-    __shared__ uint64_t sh[kSortWarps][kRowCap];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t row = (int64_t)blockIdx.x * kSortWarps + warp;
-    if (row >= N) return;
-    const int64_t b = row_off[row];
-    const int cnt = (int)(row_off[row + 1] - b);
-    if (cnt > kRowCap) {
-        if (lane == 0) atomicExch(err, 2);
-        return;
-    }
-    int p2 = 1;
-    while (p2 < cnt) p2 <<= 1;
-    uint64_t* s = sh[warp];
-    for (int i = lane; i < p2; i += 32) s[i] = i < cnt ? keys[b + i] : ~0ull;
-    __syncwarp();
-    for (int size = 2; size <= p2; size <<= 1)
+// A row's contributions as the emit kernel reads them: column in the high half, the
+// flat element-matrix index e*k*k + a*k + b in the low half, its top bit set at
+// the first contribution of a column.
+constexpr uint64_t kFirstOfColumn = 0x80000000ull;
+
+// ascending bitonic sort of 32*R keys in registers, key r of a lane at lane*R + r
+template <int R>
+__device__ __forceinline__ void warp_sort(uint32_t (&key)[R]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int size = 2; size <= 32 * R; size <<= 1) {
+#pragma unroll
         for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int i = lane; i < p2; i += 32) {
-                const int j = i ^ stride;
-                if (j > i) {
-                    const bool up = (i & size) == 0;
-                    const uint64_t x = s[i], y = s[j];
-                    if ((x > y) == up) {
-                        s[i] = y;
-                        s[j] = x;
-                    }
+            if (stride >= R) {
+                const bool lower = (lane & (stride / R)) == 0;
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const bool up = ((lane * R + r) & size) == 0;
+                    const uint32_t o = __shfl_xor_sync(0xffffffffu, key[r], stride / R);
+                    key[r] = lower == up ? min(key[r], o) : max(key[r], o);
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    if (r & stride) continue;
+                    const bool up = ((lane * R + r) & size) == 0;
+                    const uint32_t x = key[r], y = key[r | stride];
+                    key[r] = up ? min(x, y) : max(x, y);
+                    key[r | stride] = up ? max(x, y) : min(x, y);
                 }
             }
-            __syncwarp();
         }
-    int u = 0;
-    for (int i = lane; i < cnt; i += 32) {
-        keys[b + i] = s[i];
-        u += (i == 0 || (s[i] >> 32) != (s[i - 1] >> 32));
     }
-    for (int o = 16; o > 0; o >>= 1) u += __shfl_xor_sync(0xffffffffu, u, o);
-    if (lane == 0) uniq[row] = u;
 }
 
-// one warp per row: CSR columns, slot boundaries, contributions (flat element-
-// matrix index e*k*k + a*k + b) and the diagonal slot
-__global__ void pattern_emit_kernel(const int64_t* __restrict__ row_off, const int64_t* __restrict__ rowptr64,
-                                    int64_t N, int64_t E, int k, const uint64_t* __restrict__ keys,
-                                    int32_t* __restrict__ rowptr, int32_t* __restrict__ col,
-                                    int32_t* __restrict__ slot_ptr, int32_t* __restrict__ slot_src,
-                                    int32_t* __restrict__ diag) {
+// One warp sorts a row's contributions in registers: its element corners first (so
+// that a corner's rank orders elements as the reference's COO list does), then
+// one 32-bit key per contribution, (column - row, a*k + b, corner rank), R a lane.
+// A = corners a lane.  false (nothing written) if a column is too far from the row for
+// the key's 23 (A = 1) or 22 bits.
+template <int R, int A, int K>
+__device__ __forceinline__ bool sort_row(const int32_t* __restrict__ el, int64_t row, int deg, uint64_t* __restrict__ seg,
+                                         int32_t* uniq) {
+    constexpr uint32_t k = K;
+    constexpr int kRankBits = A == 1 ? 5 : 6, kLow = 4 + kRankBits;
+    constexpr int kHalf = 1 << (31 - kLow);   // |column - row| below this
+    const int lane = threadIdx.x & 31;
+    const int cnt = deg * K;
+    uint32_t corner[A];
+#pragma unroll
+    for (int r = 0; r < A; ++r) corner[r] = lane * A + r < deg ? (uint32_t)seg[lane * A + r] : 0xffffffffu;
+    warp_sort<A>(corner);
+    uint32_t key[R];
+    bool ok = true;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int i = r * 32 + lane, j = i / K, b = i - j * K;
+        uint32_t c = __shfl_sync(0xffffffffu, corner[0], A == 1 ? j & 31 : (j / A) & 31);
+        if constexpr (A == 2) {
+            const uint32_t c1 = __shfl_sync(0xffffffffu, corner[1], (j / A) & 31);
+            if (j & 1) c = c1;
+        }
+        key[r] = 0xffffffffu;
+        if (i < cnt) {
+            const uint32_t e = c / k, a = c - e * k;
+            const int64_t d = (int64_t)el[e * k + b] - row;
+            ok = ok && d > -kHalf && d < kHalf - 1;   // (kHalf - 1 with all low bits set would be the padding)
+            key[r] = ((uint32_t)(int32_t)(d + kHalf) << kLow) | ((a * k + b) << kRankBits) | (uint32_t)j;
+        }
+    }
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    warp_sort<R>(key);
+    uint32_t before = __shfl_up_sync(0xffffffffu, key[R - 1], 1);
+    int u = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int p = lane * R + r;
+        const int j = key[r] & ((1 << kRankBits) - 1), ab = (key[r] >> kRankBits) & 15;
+        uint32_t c = __shfl_sync(0xffffffffu, corner[0], A == 1 ? j : j / A);
+        if constexpr (A == 2) {
+            const uint32_t c1 = __shfl_sync(0xffffffffu, corner[1], j / A);
+            if (j & 1) c = c1;
+        }
+        if (p < cnt) {
+            const bool first = p == 0 || (key[r] >> kLow) != (before >> kLow);
+            u += first;
+            const uint32_t col = (uint32_t)(row + (int64_t)(key[r] >> kLow) - kHalf);
+            seg[p] = ((uint64_t)col << 32) | (first ? kFirstOfColumn : 0ull) | (uint64_t)((c / k) * (k * k) + ab);
+        }
+        before = key[r];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) u += __shfl_xor_sync(0xffffffffu, u, o);
+    if (lane == 0) *uniq = u;
+    return true;
+}
+
+// Rows of up to 64 corners whose columns are near enough (all rows of meshes below two
+// million nodes), one warp each; the others go to `rest` (rest[0] counts).  Bound by
+// integer issue: 28 exchange steps of 128 keys in registers (one 32-bit shuffle and one
+// minimum a key) where the 64-bit keys took as many round trips through shared memory.
+template <int K>
+__global__ void __launch_bounds__(256) pattern_sort_kernel(const int32_t* __restrict__ el, const int64_t* __restrict__ row_off, int64_t N,
+                                                           uint64_t* __restrict__ keys, int32_t* __restrict__ uniq,
+                                                           int64_t* __restrict__ rest) {
+    const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (row >= N) return;
+    const int64_t b = row_off[row];
+    const int cnt = (int)(row_off[row + 1] - b), deg = cnt / K;
+    bool done = false;
+    if (cnt <= 32) done = sort_row<1, 1, K>(el, row, deg, keys + b, uniq + row);
+    else if (cnt <= 64) done = sort_row<2, 1, K>(el, row, deg, keys + b, uniq + row);
+    else if (deg <= 32) done = sort_row<4, 1, K>(el, row, deg, keys + b, uniq + row);
+    else if (deg <= 64) done = sort_row<8, 2, K>(el, row, deg, keys + b, uniq + row);
+    if (!done && (threadIdx.x & 31) == 0)
+        rest[1 + atomicAdd(reinterpret_cast<unsigned long long*>(rest), 1ull)] = row;
+}
+
+// The remaining rows: 64-bit keys (column, COO order) sorted in shared memory, one warp a row
+__global__ void pattern_rest_kernel(const int32_t* __restrict__ el, int64_t E, int k, const int64_t* __restrict__ row_off,
+                                    uint64_t* __restrict__ keys, int32_t* __restrict__ uniq, const int64_t* __restrict__ rest,
+                                    int32_t* __restrict__ err) {
+    __shared__ uint64_t sh[kSortWarps][kRowCap];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t row = (int64_t)blockIdx.x * kSortWarps + warp;
+    const int64_t n = rest[0];
+    for (int64_t q = (int64_t)blockIdx.x * kSortWarps + warp; q < n; q += (int64_t)gridDim.x * kSortWarps) {
+        const int64_t row = rest[1 + q], b = row_off[row];
+        const int64_t cnt64 = row_off[row + 1] - b;
+        if (cnt64 > kRowCap) {
+            if (lane == 0) {
+                atomicExch(err, 2);
+                uniq[row] = 0;
+            }
+            continue;
+        }
+        const int cnt = (int)cnt64;
+        int p2 = 1;
+        while (p2 < cnt) p2 <<= 1;
+        uint64_t* s = sh[warp];
+        for (int i = lane; i < p2; i += 32) {
+            uint64_t v = ~0ull;
+            if (i < cnt) {
+                const int64_t corner = (int64_t)keys[b + i / k], e = corner / k, a = corner - e * k, c = i % k;
+                v = ((uint64_t)(uint32_t)el[e * k + c] << 32) | ((uint64_t)(a * k + c) * (uint64_t)E + (uint64_t)e);
+            }
+            s[i] = v;
+        }
+        __syncwarp();
+        for (int size = 2; size <= p2; size <<= 1)
+            for (int stride = size >> 1; stride > 0; stride >>= 1) {
+                for (int i = lane; i < p2; i += 32) {
+                    const int j = i ^ stride;
+                    if (j > i) {
+                        const bool up = (i & size) == 0;
+                        const uint64_t x = s[i], y = s[j];
+                        if ((x > y) == up) {
+                            s[i] = y;
+                            s[j] = x;
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+        int u = 0;
+        for (int i = lane; i < cnt; i += 32) {
+            const bool first = i == 0 || (s[i] >> 32) != (s[i - 1] >> 32);
+            const uint64_t order = s[i] & 0xffffffffull, ab = order / (uint64_t)E, e = order - ab * (uint64_t)E;
+            keys[b + i] = (s[i] & 0xffffffff00000000ull) | (first ? kFirstOfColumn : 0ull) | (e * k * k + ab);
+            u += first;
+        }
+        for (int o = 16; o > 0; o >>= 1) u += __shfl_xor_sync(0xffffffffu, u, o);
+        if (lane == 0) uniq[row] = u;
+        __syncwarp();
+    }
+}
+
+// one warp per row: CSR columns, slot boundaries, contributions and the diagonal slot
+__global__ void __launch_bounds__(256) pattern_emit_kernel(const int64_t* __restrict__ row_off, const int64_t* __restrict__ rowptr64,
+                                                           int64_t N, const uint64_t* __restrict__ keys,
+                                                           int32_t* __restrict__ rowptr, int32_t* __restrict__ col,
+                                                           int32_t* __restrict__ slot_ptr, int32_t* __restrict__ slot_src,
+                                                           int32_t* __restrict__ diag) {
+    const int lane = threadIdx.x & 31;
+    const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= N) return;
     const int64_t b = row_off[row];
     const int cnt = (int)(row_off[row + 1] - b);
     int64_t w = rowptr64[row];
     if (lane == 0) rowptr[row] = (int32_t)w;
-    for (int i0 = 0; i0 < cnt; i0 += 32) {
-        const int i = i0 + lane;
-        bool first = false;
-        uint64_t key = 0;
-        if (i < cnt) {
-            key = keys[b + i];
-            const uint64_t order = key & 0xffffffffull;
-            const int64_t ab = (int64_t)(order / (uint64_t)E), e = (int64_t)(order % (uint64_t)E);
-            slot_src[b + i] = (int32_t)(e * k * k + ab);
-            first = i == 0 || (keys[b + i - 1] >> 32) != (key >> 32);
+    constexpr int U = 4;   // rounds in flight (a cube's interior rows have three)
+    for (int i0 = 0; i0 < cnt; i0 += 32 * U) {
+        uint64_t key[U];
+#pragma unroll
+        for (int r = 0; r < U; ++r) {
+            const int i = i0 + 32 * r + lane;
+            key[r] = i < cnt ? keys[b + i] : 0ull;
         }
-        const unsigned m = __ballot_sync(0xffffffffu, first);
-        if (first) {
-            const int64_t j = w + __popc(m & ((1u << lane) - 1));
-            const int32_t c = (int32_t)(key >> 32);
-            col[j] = c;
-            slot_ptr[j] = (int32_t)(b + i);
-            if (c == row) diag[row] = (int32_t)j;
+#pragma unroll
+        for (int r = 0; r < U; ++r) {
+            const int i = i0 + 32 * r + lane;
+            const bool first = (key[r] & kFirstOfColumn) != 0;
+            const unsigned m = __ballot_sync(0xffffffffu, first);
+            if (i < cnt) slot_src[b + i] = (int32_t)(key[r] & 0x7fffffffull);
+            if (first) {
+                const int64_t j = w + __popc(m & ((1u << lane) - 1));
+                const int32_t c = (int32_t)(key[r] >> 32);
+                col[j] = c;
+                slot_ptr[j] = (int32_t)(b + i);
+                if (c == row) diag[row] = (int32_t)j;
+            }
+            w += __popc(m);
         }
-        w += __popc(m);
     }
-}
-
-__global__ void widen_kernel(const int32_t* __restrict__ c, int64_t* __restrict__ o, int64_t n) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) o[i] = c[i];
 }
 
 __global__ void pattern_tail_kernel(const int64_t* rp64, const int64_t* ro, int64_t n, int32_t* rp, int32_t* sp) {
     rp[n] = (int32_t)rp64[n];
     sp[rp64[n]] = (int32_t)ro[n];
+}
+
+// one warp per slice: its widest row
+__global__ void __launch_bounds__(256) slice_width_kernel(const int32_t* __restrict__ rowptr, int64_t n_rows, int64_t n_slices, int64_t* __restrict__ width) {
+    const int64_t s = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (s >= n_slices) return;
+    const int64_t r = s * TCB_SLICE + (threadIdx.x & 31);
+    int w = r < n_rows ? rowptr[r + 1] - rowptr[r] : 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) w = max(w, __shfl_xor_sync(0xffffffffu, w, o));
+    if ((threadIdx.x & 31) == 0) width[s] = w;
 }
 
 inline unsigned blocks(int64_t n, int per) { return (unsigned)((n + per - 1) / per); }
@@ -403,8 +626,8 @@ extern "C" int tcb_text_newlines(const char* text, int64_t n_bytes, int64_t* scr
     const unsigned nb = blocks(n_bytes, kThreads * kBytesPerThread);
     nl_count_kernel<<<nb, kThreads, 0, s>>>(text, n_bytes, scratch);
     TCB_CHECK_LAUNCH("newline count kernel");
-    scan_kernel<<<1, kScanThreads, 0, s>>>(scratch, nb, scratch + nb);
-    TCB_CHECK_LAUNCH("scan kernel");
+    int st = scan(scratch, scratch, nb, 1, scratch + nb, (int64_t*)nullptr, s);
+    if (st) return st;
     int64_t total = 0;
     TCB_CHECK_CUDA(cudaMemcpyAsync(&total, scratch + nb, sizeof total, cudaMemcpyDeviceToHost, s));
     TCB_CHECK_CUDA(cudaStreamSynchronize(s));
@@ -445,20 +668,24 @@ extern "C" int tcb_pattern_device(const int32_t* elems, int64_t E, int32_t k, in
     TCB_CHECK_CUDA(cudaMemsetAsync(iwork, 0, sizeof(int32_t) * (2 * N + 1), s));
     pattern_count_kernel<<<blocks(E, kThreads), kThreads, 0, s>>>(elems, E, k, N, cnt, err);
     TCB_CHECK_LAUNCH("pattern count kernel");
-    // row_off = exclusive scan of the counts (widened to int64 on the way)
-    widen_kernel<<<blocks(N, kThreads), kThreads, 0, s>>>(cnt, row_off, N);
-    TCB_CHECK_LAUNCH("widen kernel");
-    scan_kernel<<<1, kScanThreads, 0, s>>>(row_off, N, row_off + N);
-    TCB_CHECK_LAUNCH("scan kernel");
+    // rowptr64 is written last: until then it holds the tile sums and the rows left over by the sort
+    // (their number, then the rows: at most N + 1 values)
+    int st = scan(cnt, row_off, N, k, row_off + N, rowptr64, s);
+    if (st) return st;
     TCB_CHECK_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * N, s));
-    pattern_fill_kernel<<<blocks(E, kThreads), kThreads, 0, s>>>(elems, E, k, row_off, cnt, keys);
+    TCB_CHECK_CUDA(cudaMemsetAsync(rowptr64, 0, sizeof(int64_t), s));
+    pattern_fill_kernel<<<blocks(E, kThreads), kThreads, 0, s>>>(elems, E, k, N, row_off, cnt, keys);
     TCB_CHECK_LAUNCH("pattern fill kernel");
-    pattern_sort_kernel<<<blocks(N, kSortWarps), kSortWarps * 32, 0, s>>>(row_off, N, keys, uniq, err);
+    if (k == 4) pattern_sort_kernel<4><<<blocks(N, 8), 256, 0, s>>>(elems, row_off, N, keys, uniq, rowptr64);
+    else pattern_sort_kernel<3><<<blocks(N, 8), 256, 0, s>>>(elems, row_off, N, keys, uniq, rowptr64);
     TCB_CHECK_LAUNCH("pattern sort kernel");
-    widen_kernel<<<blocks(N, kThreads), kThreads, 0, s>>>(uniq, rowptr64, N);
-    TCB_CHECK_LAUNCH("widen kernel");
-    scan_kernel<<<1, kScanThreads, 0, s>>>(rowptr64, N, rowptr64 + N);
-    TCB_CHECK_LAUNCH("scan kernel");
+    pattern_rest_kernel<<<(unsigned)std::min<int64_t>(blocks(N, kSortWarps), 592), kSortWarps * 32, 0, s>>>(
+        elems, E, k, row_off, keys, uniq, rowptr64, err);
+    TCB_CHECK_LAUNCH("pattern rest kernel");
+    // (the tile sums of this scan go where the corner counts were: 8-byte aligned, read no more)
+    int64_t* tmp = reinterpret_cast<int64_t*>(((uintptr_t)cnt + 7) & ~(uintptr_t)7);
+    st = scan(uniq, rowptr64, N, 1, rowptr64 + N, tmp, s);
+    if (st) return st;
     int32_t h_err = 0;
     TCB_CHECK_CUDA(cudaMemcpyAsync(&h_err, err, sizeof h_err, cudaMemcpyDeviceToHost, s));
     TCB_CHECK_CUDA(cudaMemcpyAsync(nnz, rowptr64 + N, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
@@ -478,10 +705,30 @@ extern "C" int tcb_pattern_device_emit(const int64_t* work, const uint64_t* keys
     cudaStream_t s = as_stream(stream);
     const int64_t* row_off = work;
     const int64_t* rowptr64 = work + N + 1;
-    pattern_emit_kernel<<<blocks(N, kSortWarps), kSortWarps * 32, 0, s>>>(row_off, rowptr64, N, E, k, keys, rowptr,
-                                                                          col, slot_ptr, slot_src, diag);
+    pattern_emit_kernel<<<blocks(N, 8), 256, 0, s>>>(row_off, rowptr64, N, keys, rowptr, col, slot_ptr, slot_src, diag);
     TCB_CHECK_LAUNCH("pattern emit kernel");
     pattern_tail_kernel<<<1, 1, 0, s>>>(rowptr64, row_off, N, rowptr, slot_ptr);
     TCB_CHECK_LAUNCH("pattern tail kernel");
+    return TCB_OK;
+}
+
+extern "C" int64_t tcb_sell_layout_scratch(int64_t n_rows) {
+    if (n_rows < 0) return -1;
+    const int64_t ns = ceil_div(n_rows, TCB_SLICE);
+    return scan_tiles(ns) + 1;
+}
+
+extern "C" int tcb_sell_layout_device(const int32_t* rowptr, int64_t n_rows, int64_t* slice_ptr, int64_t* scratch,
+                                      int64_t* n_entries, void* stream) {
+    if (!rowptr || !slice_ptr || !scratch || !n_entries || n_rows <= 0)
+        return fail(TCB_EINVAL, "tcb_sell_layout_device: bad arguments");
+    cudaStream_t s = as_stream(stream);
+    const int64_t ns = ceil_div(n_rows, TCB_SLICE);
+    slice_width_kernel<<<blocks(ns, 8), 256, 0, s>>>(rowptr, n_rows, ns, slice_ptr);
+    TCB_CHECK_LAUNCH("slice width kernel");
+    const int st = scan(slice_ptr, slice_ptr, ns, TCB_SLICE, slice_ptr + ns, scratch, s);
+    if (st) return st;
+    TCB_CHECK_CUDA(cudaMemcpyAsync(n_entries, slice_ptr + ns, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    TCB_CHECK_CUDA(cudaStreamSynchronize(s));
     return TCB_OK;
 }
