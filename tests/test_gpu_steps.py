@@ -95,3 +95,24 @@ def test_stretches_of_any_length_are_the_same(lib, cuda):
     got = _run(sim, 1e-6, 100, True, 0, [1, 1, 2, 3, 4, 5, 129], frames=True)
     for k in ref:
         assert torch.equal(ref[k], got[k]), k
+
+
+def test_step_graph_recorded_while_garbage_holds_device_memory(lib, cuda):
+    """A collection in the middle of a recording would free what unreachable cycles hold
+    (other step graphs, tensors) on the recording thread and break it: with the collector
+    at its most eager the recording still succeeds."""
+    import gc
+    sim = _sim("cube", 5, "ms", cuda)
+    sim.prepare(1e-5, 1e-5, 100, snapshot_interval=sim.T)
+    old = gc.get_threshold()
+    try:
+        for _ in range(20):
+            cycle = [torch.empty(3 << 20, device=cuda), sim.capture_steps(3)]
+            cycle.append(cycle)
+            del cycle
+            gc.set_threshold(1, 1, 1)
+            sim.capture_steps(5)()
+            gc.set_threshold(*old)
+    finally:
+        gc.set_threshold(*old)
+    torch.cuda.synchronize(cuda)

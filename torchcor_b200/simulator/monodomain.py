@@ -11,6 +11,8 @@ synchronisation until it finishes.
 from __future__ import annotations
 
 import ctypes as C
+import gc
+import threading
 import time
 from pathlib import Path
 
@@ -25,6 +27,9 @@ from torchcor_b200.core.mesh import MeshReader
 from torchcor_b200.core.stimulation import Stimuli
 from torchcor_b200.device import get_device
 from torchcor_b200.simulator.resultio import FrameWriter
+
+
+_recording = threading.Lock()      # one step graph at a time is recorded (the collector is off meanwhile)
 
 
 def rcm_order(elems, n_nodes):
@@ -301,15 +306,25 @@ class Monodomain:
         graph = torch.cuda.CUDAGraph()
         # recorded on a stream of its own without the garbage collection, device
         # synchronisation and release of cached memory that torch.cuda.graph() begins
-        # with (2 to 60 ms): nothing is allocated while the launches are recorded
+        # with (2 to 60 ms): nothing is allocated while the launches are recorded, and
+        # the collector, which could free another graph or tensor in the middle of it
+        # on this thread, waits until it is over
         side = torch.cuda.Stream(self.device)
-        with torch.cuda.stream(side):
-            # thread-local capture: a thread writing result files may use CUDA meanwhile
-            graph.capture_begin(capture_error_mode="thread_local")
+        struct, stream = C.byref(sim["struct"]), side.cuda_stream
+        with _recording, torch.cuda.stream(side):
+            collecting = gc.isenabled()
+            gc.disable()
             try:
-                check(lib.tcb_mono_run(C.byref(sim["struct"]), 1, 1 + n_steps, stream_ptr()))
+                # thread-local capture: a thread writing result files may use CUDA meanwhile
+                graph.capture_begin(capture_error_mode="thread_local")
+                try:
+                    status = lib.tcb_mono_run(struct, 1, 1 + n_steps, stream)
+                finally:
+                    graph.capture_end()
             finally:
-                graph.capture_end()
+                if collecting:
+                    gc.enable()
+        check(status)
 
         def replay():
             if sim["next_step"] + n_steps > self.nt + 1:
