@@ -54,7 +54,7 @@ Layout layout(int n) {
     L.dev = take(sizeof(MonoDev) * n);
     L.cg = take(sizeof(CgView) * n);
     L.slices = take(sizeof(int32_t) * n);
-    L.parts = take(sizeof(double) * 3 * (size_t)n * kBatchMaxBlocks);   // any grid of the plan
+    L.parts = take(sizeof(double) * 6 * (size_t)n * kBatchMaxBlocks);   // any grid of the plan
     L.bar = take(sizeof(uint32_t) * 4);
     L.err = take(sizeof(int32_t) * 4);
     for (int g = 0; g < kBatchGroups; ++g) {

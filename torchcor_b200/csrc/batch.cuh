@@ -15,7 +15,7 @@ namespace tcb {
 
 constexpr int kBatchMaxSims = 1024;        // simulations per batch
 constexpr int kBatchMaxPerBlock = 64;      // simulations staged at once by one CG block
-constexpr int kBatchMaxBlocks = 1024;      // CG blocks of a batch
+constexpr int kBatchMaxBlocks = 512;      // CG blocks of a batch
 constexpr int kBatchTile = 128;            // nodes per ionic tile (n_pad is a multiple of it)
 constexpr int kBatchGroups = 3;            // one per ionic model
 
@@ -48,7 +48,7 @@ struct BatchWS {
     const MonoDev* dev;        // [n]
     const CgView* cg;          // [n]
     const int32_t* slices;     // [n] 32-row slices of each simulation
-    double* parts;             // [3 values][n][nb] per-simulation block partials
+    double* parts;             // two sets of [3 values][n][nb] per-simulation block partials
     uint32_t* bar;             // [4] grid barrier words
     int32_t* err;              // [1] error word
     cgk::WaitLimit wait;       // bounded-wait limits (grid barrier, bulk-copy mbarriers)

@@ -17,6 +17,12 @@
 // double-buffered p, float64 row sums and inner products, int16 column offsets
 // and A rebuilt from M and K' where the simulation allows.
 //
+// Stopping test.  A pass's sums tell which simulations it stops (as in the
+// single-simulation kernel); those update x alone, and where none goes on the
+// launch ends without another barrier.  24 cubes of 2.0 M nodes (one or two passes)
+// take 213 us a launch on B200, 245 before this, the unpredicated chunks of 5 and
+// the shorter barrier; 12 cubes and shells of 340,000 nodes 85, 99 before.
+//
 // Reductions are per simulation and deterministic: each lane accumulates its
 // rows of one simulation in slice order, a warp reduces its lanes with a fixed
 // shuffle tree when its simulation changes, the block adds its warps' values
@@ -52,10 +58,15 @@ __device__ __forceinline__ float p_update(float z, float p_old, float beta, bool
 // matrix streams (columns, M, K, A) of a batch are far larger than L2 and read
 // once a pass: they are loaded as first to leave L2, ahead of the row vectors the
 // neighbour gathers reuse.
-template <bool DC>
+// J: entry e + J of the row (an immediate offset of the load).
+template <bool DC, int J>
 __device__ __forceinline__ int col_at(const CgView& d, int64_t e, int row) {
-    if constexpr (DC) return row + ld_hint_sched(d.dcol + e, l2_once_sched());
-    else return ld_hint_sched(d.col + e, l2_once_sched());
+    if constexpr (DC) return row + ld_hint_sched_at<J * TCB_SLICE * 2>(d.dcol + e, l2_once_sched());
+    else return ld_hint_sched_at<J * TCB_SLICE * 4>(d.col + e, l2_once_sched());
+}
+template <int J>
+__device__ __forceinline__ float val_at(const float* v) {
+    return ld_hint_sched_at<J * TCB_SLICE * 4>(v, l2_once_sched());
 }
 
 // Call f with std::integral_constant<int, flags> for the simulation's combination
@@ -90,12 +101,16 @@ __device__ __forceinline__ void with_dcol(const CgView& d, F&& f) {
     }
 }
 
+// entries of a row in flight at once (as in the single-simulation kernel: whole
+// chunks are loaded without predicates)
+constexpr int kRhsChunk = 5;
+
 // Right-hand side, guess, r0 = b - A x0, z0 = D r0 for the 32 rows of slice ls
-// (solver.py:46-55, monodomain.py:130-131); adds ||D b||^2 and r0.z0 into acc.
+// (solver.py:46-55, monodomain.py:130-131); adds ||D b||^2, r0.z0 and z0.z0 into acc.
 // DC: int16 column offsets; AS: A rebuilt as fp32(fp32(M*Cm) + K'); LG: linear
 // extrapolation guess.  Vectors other than x's next slot are read-only here.
 template <bool DC, bool AS, bool LG>
-__device__ __forceinline__ void rhs_slice(const CgView& d, int step, int64_t ls, int lane, double (&acc)[2]) {
+__device__ __forceinline__ void rhs_slice(const CgView& d, int step, int64_t ls, int lane, double (&acc)[3]) {
     const int64_t row = ls * TCB_SLICE + lane;
     if (row >= d.n) return;
     const float* __restrict__ u = d.x + ring_cur(step) * d.n_pad;
@@ -109,32 +124,30 @@ __device__ __forceinline__ void rhs_slice(const CgView& d, int step, int64_t ls,
     // A x0 in float64 (the reference's CG is float64; b - A x0 cancels)
     float mb = 0.0f, ku = 0.0f;
     double ax = 0.0;
-    // the columns of the next 4-entry chunk are loaded while this chunk's
-    // gathers and coefficients are in flight (a column load heads each chain)
-    int c[4];
+    for (int k0 = 0; k0 < w; k0 += kRhsChunk) {
+        const int64_t e = base + (int64_t)k0 * TCB_SLICE;
+        int c[kRhsChunk];
+        float mv[kRhsChunk], kv[kRhsChunk], av[kRhsChunk], bc[kRhsChunk], uc[kRhsChunk], xc[kRhsChunk];
+        auto load = [&](auto full) {
+            unrolled<0, kRhsChunk>([&](auto J) {
+                constexpr int j = J.value;
+                const bool ok = decltype(full)::value || k0 + j < w;
+                c[j] = ok ? col_at<DC, j>(d, e, r) : r;
+                mv[j] = ok ? val_at<j>(d.mv + e) : 0.0f;
+                kv[j] = ok ? val_at<j>(d.kv + e) : 0.0f;
+                if constexpr (!AS) av[j] = ok ? val_at<j>(d.av + e) : 0.0f;
+            });
+        };
+        if (k0 + kRhsChunk <= w) load(std::true_type{});
+        else load(std::false_type{});
 #pragma unroll
-    for (int j = 0; j < 4; ++j) c[j] = j < w ? col_at<DC>(d, base + (int64_t)j * TCB_SLICE, r) : r;
-    for (int k0 = 0; k0 < w; k0 += 4) {
-        float mv[4], kv[4], av[4], bc[4], uc[4], xc[4];
-        int cn[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const bool ok = k0 + j < w;
-            const int64_t e = base + (int64_t)(k0 + j) * TCB_SLICE;
-            mv[j] = ok ? ld_hint_sched(d.mv + e, l2_once_sched()) : 0.0f;
-            kv[j] = ok ? ld_hint_sched(d.kv + e, l2_once_sched()) : 0.0f;
-            if constexpr (!AS) av[j] = ok ? ld_hint_sched(d.av + e, l2_once_sched()) : 0.0f;
+        for (int j = 0; j < kRhsChunk; ++j) {
             bc[j] = __ldg(bp + c[j]);
             uc[j] = __ldg(u + c[j]);
             if constexpr (LG) xc[j] = __ldg(xp + c[j]);
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const bool ok = k0 + 4 + j < w;
-            cn[j] = ok ? col_at<DC>(d, base + (int64_t)(k0 + 4 + j) * TCB_SLICE, r) : r;
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < kRhsChunk; ++j) {
             if constexpr (AS) av[j] = __fadd_rn(__fmul_rn(mv[j], d.cm), kv[j]);
             float xg;
             if constexpr (LG) xg = 2.0f * uc[j] - xc[j];
@@ -142,7 +155,6 @@ __device__ __forceinline__ void rhs_slice(const CgView& d, int step, int64_t ls,
             mb = __fmaf_rn(mv[j], bc[j], mb);
             ku = __fmaf_rn(kv[j], uc[j], ku);
             ax += (double)av[j] * (double)xg;
-            c[j] = cn[j];
         }
     }
     const float rhs = mb - ku;
@@ -153,12 +165,25 @@ __device__ __forceinline__ void rhs_slice(const CgView& d, int step, int64_t ls,
     __stwb(d.x + ring_next(step) * d.n_pad + row, xg0);
     const float r32 = (float)((double)rhs - ax);
     const float di = __ldg(d.dinv + row);
-    const float z32 = (float)((double)di * (double)r32);
+    const float z32 = __fmul_rn(di, r32);
     __stwb(d.r + row, r32);
     __stwb(d.z + row, z32);
-    const double db = (double)di * (double)rhs;
+    const double db = (double)di * (double)rhs, z = (double)z32;
     acc[0] += db * db;
-    acc[1] += (double)r32 * (double)z32;
+    acc[1] += (double)r32 * z;
+    acc[2] += z * z;
+}
+
+// The end of a row of A p: p and A p to memory; p.Ap and, with w = D A p, z.w and w.w
+// into acc.
+__device__ __forceinline__ void ap_sums(const CgView& d, int64_t row, float z, float p, float ap, float* pout,
+                                        double (&acc)[3]) {
+    __stwb(pout + row, p);
+    __stwb(d.ap + row, ap);
+    const double w = (double)__fmul_rn(__ldg(d.dinv + row), ap);
+    acc[0] += (double)p * (double)ap;
+    acc[1] += (double)z * w;
+    acc[2] += w * w;
 }
 
 // p_new = z + beta p_old formed on the fly for every column, Ap for the rows of
@@ -167,7 +192,7 @@ __device__ __forceinline__ void rhs_slice(const CgView& d, int step, int64_t ls,
 // global loads, ordered after their writers by the grid barrier.
 template <bool DC, bool FIRST>
 __device__ __forceinline__ void ap_slice(const CgView& d, const float* pin, float* pout, float beta, int64_t ls,
-                                         int lane, double (&acc)[1]) {
+                                         int lane, double (&acc)[3]) {
     const int64_t row = ls * TCB_SLICE + lane;
     if (row >= d.n) return;
     const int64_t s0 = __ldg(d.slice_ptr + ls);
@@ -177,15 +202,19 @@ __device__ __forceinline__ void ap_slice(const CgView& d, const float* pin, floa
     const float* z = d.z;
     double a = 0.0;
     for (int k0 = 0; k0 < w; k0 += 8) {
+        const int64_t e = base + (int64_t)k0 * TCB_SLICE;
         int c[8];
         float av[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const bool ok = k0 + j < w;
-            const int64_t e = base + (int64_t)(k0 + j) * TCB_SLICE;
-            c[j] = ok ? col_at<DC>(d, e, r) : r;
-            av[j] = ok ? ld_hint_sched(d.av + e, l2_once_sched()) : 0.0f;
-        }
+        auto load = [&](auto full) {
+            unrolled<0, 8>([&](auto J) {
+                constexpr int j = J.value;
+                const bool ok = decltype(full)::value || k0 + j < w;
+                c[j] = ok ? col_at<DC, j>(d, e, r) : r;
+                av[j] = ok ? val_at<j>(d.av + e) : 0.0f;
+            });
+        };
+        if (k0 + 8 <= w) load(std::true_type{});
+        else load(std::false_type{});
         float zc[8], pc[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -195,11 +224,7 @@ __device__ __forceinline__ void ap_slice(const CgView& d, const float* pin, floa
 #pragma unroll
         for (int j = 0; j < 8; ++j) a += (double)av[j] * (double)p_update(zc[j], pc[j], beta, FIRST);
     }
-    const float pn = p_update(__ldca(z + row), FIRST ? 0.0f : __ldca(pin + row), beta, FIRST);
-    __stwb(pout + row, pn);
-    const float a32 = (float)a;
-    __stwb(d.ap + row, a32);
-    acc[0] += (double)pn * (double)a32;
+    ap_sums(d, row, __ldca(z + row), p_update(__ldca(z + row), FIRST ? 0.0f : __ldca(pin + row), beta, FIRST), (float)a, pout, acc);
 }
 
 // ---------------------------------------------------------------------------
@@ -284,23 +309,24 @@ struct ApStreams {
 };
 
 struct BatchShared {
-    double *rz, *bn, *al, *be;   // [n] per simulation
-    double* wp;                  // [warps][kBatchMaxPerBlock][2] warp partials of the staged simulations
+    double *rz, *zz, *bn, *al, *be;   // [n] per simulation
+    double* wp;                  // [warps][kBatchMaxPerBlock][3] warp partials of the staged simulations
     int64_t* pre;                // [n+1] prefix of the active simulations' slice counts
     int64_t* bb;                 // [nb+1] first virtual slice of each block
     CgView* cg;                  // [kBatchMaxPerBlock] staged views
-    int *it, *act, *step, *ns;   // [n]
+    int *it, *act, *step, *ns;   // [n]; act: 0 done, 1 iterating, 2 in its last pass
     int *w0, *w1;                // [n] first and last block holding each active simulation's slices
 };
 
 __device__ __forceinline__ BatchShared carve(double* smd, int n, int nb) {
     BatchShared s;
     s.rz = smd;
-    s.bn = s.rz + n;
+    s.zz = s.rz + n;
+    s.bn = s.zz + n;
     s.al = s.bn + n;
     s.be = s.al + n;
     s.wp = s.be + n;
-    s.pre = reinterpret_cast<int64_t*>(s.wp + kCgWarps * kBatchMaxPerBlock * 2);
+    s.pre = reinterpret_cast<int64_t*>(s.wp + kCgWarps * kBatchMaxPerBlock * 3);
     s.bb = s.pre + n + 1;
     s.cg = reinterpret_cast<CgView*>(s.bb + nb + 1);
     s.it = reinterpret_cast<int*>(s.cg + kBatchMaxPerBlock);
@@ -382,7 +408,7 @@ __device__ __forceinline__ void flush(BatchShared& S, int warp, int lane, int j,
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
         const double t = warp_sum(acc[v]);
-        if (lane == 0) S.wp[(warp * kBatchMaxPerBlock + j) * 2 + v] += t;
+        if (lane == 0) S.wp[(warp * kBatchMaxPerBlock + j) * 3 + v] += t;
         acc[v] = 0.0;
     }
 }
@@ -405,7 +431,7 @@ __device__ __forceinline__ void sweep(const BatchWS* W, BatchShared& S, double* 
             uint32_t* dst = reinterpret_cast<uint32_t*>(S.cg);
             const int words = (j1 - j0) * (int)(sizeof(CgView) / 4);
             for (int t = threadIdx.x; t < words; t += blockDim.x) dst[t] = src[t];
-            for (int t = threadIdx.x; t < kCgWarps * kBatchMaxPerBlock * 2; t += blockDim.x) S.wp[t] = 0.0;
+            for (int t = threadIdx.x; t < kCgWarps * kBatchMaxPerBlock * 3; t += blockDim.x) S.wp[t] = 0.0;
         }
         __syncthreads();
         const int64_t sb = max(vb, S.pre[j0]), se = min(ve, S.pre[j1]);
@@ -429,7 +455,7 @@ __device__ __forceinline__ void sweep(const BatchWS* W, BatchShared& S, double* 
 #pragma unroll
             for (int v = 0; v < NV; ++v) {
                 double t = 0.0;
-                for (int w = 0; w < kCgWarps; ++w) t += S.wp[(w * kBatchMaxPerBlock + j) * 2 + v];
+                for (int w = 0; w < kCgWarps; ++w) t += S.wp[(w * kBatchMaxPerBlock + j) * 3 + v];
                 parts[((size_t)v * n + i2) * nb + b] = t;
             }
         }
@@ -482,7 +508,7 @@ __device__ __forceinline__ void issue(Pipe& P, int s, const CgView& d, const Wal
 // sweep() with the ELL streams staged: unit(i, view, ls, nk, stage buffer, row)
 // accumulates one unit into the row's partial sums, end(i, view, ls, row, acc)
 // finishes a row after its slice's last unit.  Returns false after a timed-out
-// wait (the error word is set; the caller's next grid barrier ends the kernel).
+// wait (the error word is set; the block returns).
 template <int NV, class Streams, class Unit, class End>
 __device__ __forceinline__ bool sweep_staged(const BatchWS* W, BatchShared& S, double* parts, Pipe& P,
                                              int32_t* err, Unit&& unit, End&& end) {
@@ -500,7 +526,7 @@ __device__ __forceinline__ bool sweep_staged(const BatchWS* W, BatchShared& S, d
             uint32_t* dst = reinterpret_cast<uint32_t*>(S.cg);
             const int words = (j1 - j0) * (int)(sizeof(CgView) / 4);
             for (int t = threadIdx.x; t < words; t += blockDim.x) dst[t] = src[t];
-            for (int t = threadIdx.x; t < kCgWarps * kBatchMaxPerBlock * 2; t += blockDim.x) S.wp[t] = 0.0;
+            for (int t = threadIdx.x; t < kCgWarps * kBatchMaxPerBlock * 3; t += blockDim.x) S.wp[t] = 0.0;
         }
         __syncthreads();
         Walk<Streams> cons;
@@ -551,7 +577,7 @@ __device__ __forceinline__ bool sweep_staged(const BatchWS* W, BatchShared& S, d
 #pragma unroll
             for (int v = 0; v < NV; ++v) {
                 double t = 0.0;
-                for (int w = 0; w < kCgWarps; ++w) t += S.wp[(w * kBatchMaxPerBlock + j) * 2 + v];
+                for (int w = 0; w < kCgWarps; ++w) t += S.wp[(w * kBatchMaxPerBlock + j) * 3 + v];
                 parts[((size_t)v * n + i2) * nb + b] = t;
             }
         }
@@ -616,7 +642,7 @@ __device__ __forceinline__ void rhs_unit(const CgView& d, int step, int64_t ls, 
 }
 
 // the end of a right-hand-side row (as the tail of rhs_slice)
-__device__ __forceinline__ void rhs_end(const CgView& d, int step, int64_t ls, const Row& rw, double (&acc)[2],
+__device__ __forceinline__ void rhs_end(const CgView& d, int step, int64_t ls, const Row& rw, double (&acc)[3],
                                         int lane) {
     const int64_t row = ls * TCB_SLICE + lane;
     if (row >= d.n) return;
@@ -627,12 +653,13 @@ __device__ __forceinline__ void rhs_end(const CgView& d, int step, int64_t ls, c
     __stwb(d.x + ring_next(step) * d.n_pad + row, xg0);
     const float r32 = (float)((double)rhs - rw.v[2]);
     const float di = __ldg(d.dinv + row);
-    const float z32 = (float)((double)di * (double)r32);
+    const float z32 = __fmul_rn(di, r32);
     __stwb(d.r + row, r32);
     __stwb(d.z + row, z32);
-    const double db = (double)di * (double)rhs;
+    const double db = (double)di * (double)rhs, z = (double)z32;
     acc[0] += db * db;
-    acc[1] += (double)r32 * (double)z32;
+    acc[1] += (double)r32 * z;
+    acc[2] += z * z;
 }
 
 // one staged unit of A p (p formed on the fly from the gathered z and old p)
@@ -672,14 +699,11 @@ __device__ __forceinline__ void ap_unit(const CgView& d, const float* pin, float
 }
 
 __device__ __forceinline__ void ap_end(const CgView& d, const float* pin, float* pout, float beta, bool first,
-                                       int64_t ls, const Row& rw, double (&acc)[1], int lane) {
+                                       int64_t ls, const Row& rw, double (&acc)[3], int lane) {
     const int64_t row = ls * TCB_SLICE + lane;
     if (row >= d.n) return;
-    const float pn = p_update(__ldca(d.z + row), first ? 0.0f : __ldca(pin + row), beta, first);
-    __stwb(pout + row, pn);
-    const float a32 = (float)rw.v[0];
-    __stwb(d.ap + row, a32);
-    acc[0] += (double)pn * (double)a32;
+    const float z = __ldca(d.z + row);
+    ap_sums(d, row, z, p_update(z, first ? 0.0f : __ldca(pin + row), beta, first), (float)rw.v[0], pout, acc);
 }
 
 // every block: totals of every active simulation (warp per simulation, lanes over its blocks)
@@ -707,8 +731,8 @@ __device__ __forceinline__ void totals(const BatchWS* W, BatchShared& S, const d
 
 // bytes of the shared carve-out before the staging area (128-byte aligned)
 __host__ __device__ inline size_t carve_bytes(int n) {
-    const size_t b = (size_t)n * (4 * sizeof(double) + 6 * sizeof(int)) +
-                     sizeof(double) * kCgWarps * kBatchMaxPerBlock * 2 + sizeof(int64_t) * (n + 1) +
+    const size_t b = (size_t)n * (5 * sizeof(double) + 6 * sizeof(int)) +
+                     sizeof(double) * kCgWarps * kBatchMaxPerBlock * 3 + sizeof(int64_t) * (n + 1) +
                      sizeof(int64_t) * (kBatchMaxBlocks + 1) + sizeof(CgView) * kBatchMaxPerBlock;
     return (b + 127) / 128 * 128;
 }
@@ -729,8 +753,10 @@ __global__ void __launch_bounds__(kCgThreads, PER_SM) batch_cg_kernel(const Batc
     BatchShared S = carve(smd, n, gridDim.x);
     const int lane = threadIdx.x & 31;
     double* parts0 = W->parts;
-    double* parts1 = W->parts + 2 * (size_t)n * gridDim.x;
+    double* parts1 = W->parts + 3 * (size_t)n * gridDim.x;
     int32_t* err = W->err;
+    GridWait gw = grid_wait_begin(W->bar, err, W->wait);
+    if (*(volatile int32_t*)err != 0) return;   // an earlier launch gave up
     Pipe P = {};
     if constexpr (STAGED) {
         unsigned char* base = reinterpret_cast<unsigned char*>(smd) + carve_bytes(n);
@@ -760,7 +786,7 @@ __global__ void __launch_bounds__(kCgThreads, PER_SM) batch_cg_kernel(const Batc
     // ---- right-hand side, guess, r0, z0 (solver.py:46-55; monodomain.py:130-131)
     int64_t A = active_prefix(S, n, S.step);
     if constexpr (STAGED) {
-        sweep_staged<2, RhsStreams>(
+        const bool ok = sweep_staged<3, RhsStreams>(
             W, S, parts0, P, err,
             [&](int i, const CgView& d, int64_t ls, int nk, const unsigned char* buf, Row& rw) {
                 const int step = S.step[i];
@@ -769,21 +795,25 @@ __global__ void __launch_bounds__(kCgThreads, PER_SM) batch_cg_kernel(const Batc
                     rhs_unit<(F & 4) != 0, (F & 2) != 0, (F & 1) != 0>(d, step, ls, nk, buf, rw, lane);
                 });
             },
-            [&](int i, const CgView& d, int64_t ls, const Row& rw, double (&acc)[2]) {
+            [&](int i, const CgView& d, int64_t ls, const Row& rw, double (&acc)[3]) {
                 rhs_end(d, S.step[i], ls, rw, acc, lane);
             });
+        // a copy that did not come in time: the error word is set, and a block missing at the
+        // barrier makes the others look at it
+        if (__syncthreads_or(!ok)) return;
     } else
-    sweep<2>(W, S, parts0, [&](int i, const CgView& d, int64_t ls, double (&acc)[2]) {
+    sweep<3>(W, S, parts0, [&](int i, const CgView& d, int64_t ls, double (&acc)[3]) {
         const int step = S.step[i];
         with_flags<FLAGS>(d, [&](auto fl) {
             constexpr int F = decltype(fl)::value;
             rhs_slice<(F & 4) != 0, (F & 2) != 0, (F & 1) != 0>(d, step, ls, lane, acc);
         });
     });
-    if (!grid_barrier(W->bar, err, W->wait)) return;
-    totals<2>(W, S, parts0, [&](int i, double* t) {
+    if (!grid_barrier(gw)) return;
+    totals<3>(W, S, parts0, [&](int i, double* t) {
         S.bn[i] = sqrt(t[0]);
         S.rz[i] = t[1];
+        S.zz[i] = t[2];
         S.be[i] = 0.0;
         S.act[i] = W->dev[i].max_iter > 0;
     });
@@ -794,7 +824,7 @@ __global__ void __launch_bounds__(kCgThreads, PER_SM) batch_cg_kernel(const Batc
         const bool first_pass = pass == 0;
         // ---- p = z + beta p (on the fly), Ap, p.Ap
         if constexpr (STAGED) {
-            sweep_staged<1, ApStreams>(
+            const bool ok = sweep_staged<3, ApStreams>(
                 W, S, parts1, P, err,
                 [&](int i, const CgView& d, int64_t ls, int nk, const unsigned char* buf, Row& rw) {
                     const float* pin = (pass & 1) ? d.p2 : d.p;
@@ -805,12 +835,13 @@ __global__ void __launch_bounds__(kCgThreads, PER_SM) batch_cg_kernel(const Batc
                         else ap_unit<DC, false>(d, pin, beta, ls, nk, buf, rw, lane);
                     });
                 },
-                [&](int i, const CgView& d, int64_t ls, const Row& rw, double (&acc)[1]) {
+                [&](int i, const CgView& d, int64_t ls, const Row& rw, double (&acc)[3]) {
                     ap_end(d, (pass & 1) ? d.p2 : d.p, (pass & 1) ? d.p : d.p2, (float)S.be[i], first_pass, ls, rw, acc,
                            lane);
                 });
+            if (__syncthreads_or(!ok)) return;
         } else
-        sweep<1>(W, S, parts1, [&](int i, const CgView& d, int64_t ls, double (&acc)[1]) {
+        sweep<3>(W, S, parts1, [&](int i, const CgView& d, int64_t ls, double (&acc)[3]) {
             const float* pin = (pass & 1) ? d.p2 : d.p;
             float* pout = (pass & 1) ? d.p : d.p2;
             const float beta = (float)S.be[i];
@@ -820,10 +851,19 @@ __global__ void __launch_bounds__(kCgThreads, PER_SM) batch_cg_kernel(const Batc
                 else ap_slice<DC, false>(d, pin, pout, beta, ls, lane, acc);
             });
         });
-        if (!grid_barrier(W->bar, err, W->wait)) return;
-        totals<1>(W, S, parts1, [&](int i, double* t) { S.al[i] = S.rz[i] / t[0]; });
+        if (!grid_barrier(gw)) return;
+        // alpha, and |z'|^2 of z' = z - alpha w from the same sums: a simulation that this
+        // stops (solver.py:66-69) has only x left to update
+        totals<3>(W, S, parts1, [&](int i, double* t) {
+            const double alpha = S.rz[i] / t[0];
+            const double zz1 = S.zz[i] - alpha * (2.0 * t[1] - alpha * t[2]);
+            const double zn = sqrt(zz1 < 0.0 ? 0.0 : zz1);
+            const MonoDev& d = W->dev[i];
+            S.al[i] = alpha;
+            if (zn < d.a_tol || zn < d.r_tol * S.bn[i]) S.act[i] = 2;
+        });
 
-        // ---- x += alpha p, r -= alpha Ap, z = D r; ||z||^2, r.z
+        // ---- x += alpha p, r -= alpha Ap, z = D r; r.z, z.z
         sweep<2>(W, S, parts0, [&](int i, const CgView& d, int64_t ls, double (&acc)[2]) {
             const int64_t row = ls * TCB_SLICE + lane;
             if (row >= d.n) return;
@@ -831,25 +871,30 @@ __global__ void __launch_bounds__(kCgThreads, PER_SM) batch_cg_kernel(const Batc
             const double alpha = S.al[i];
             float* x = d.x + ring_next(S.step[i]) * d.n_pad;
             __stwb(x + row, (float)((double)__ldca(x + row) + alpha * (double)__ldca(pnew + row)));
+            if (S.act[i] == 2) return;
             const float r32 = (float)((double)__ldca(d.r + row) - alpha * (double)__ldca(d.ap + row));
             __stwb(d.r + row, r32);
-            const float z32 = (float)((double)__ldg(d.dinv + row) * (double)r32);
+            const float z32 = __fmul_rn(__ldg(d.dinv + row), r32);
             __stwb(d.z + row, z32);
-            acc[0] += (double)z32 * (double)z32;
-            acc[1] += (double)r32 * (double)z32;
+            const double z = (double)z32;
+            acc[0] += (double)r32 * z;
+            acc[1] += z * z;
         });
-        if (!grid_barrier(W->bar, err, W->wait)) return;
+        // (the sweeps of the next pass wait for this one's z; with nobody iterating, nothing is left)
+        bool more = false;
+        for (int i = threadIdx.x; i < n; i += blockDim.x) more |= S.act[i] == 1;
+        if (!__syncthreads_or(more)) break;
+        if (!grid_barrier(gw)) return;
         totals<2>(W, S, parts0, [&](int i, double* t) {
-            const MonoDev& d = W->dev[i];
-            const double zn = sqrt(t[0]);
-            if (zn < d.a_tol || (zn / S.bn[i]) < d.r_tol) {   // solver.py:66-69
+            if (S.act[i] != 1) {
                 S.act[i] = 0;
                 return;
             }
-            S.be[i] = t[1] / S.rz[i];
-            S.rz[i] = t[1];
+            S.be[i] = t[0] / S.rz[i];
+            S.rz[i] = t[0];
+            S.zz[i] = t[1];
             S.it[i] += 1;
-            if (S.it[i] >= d.max_iter) S.act[i] = 0;
+            if (S.it[i] >= W->dev[i].max_iter) S.act[i] = 0;
         });
     }
     // block 0 records the iterations and advances the step counters (every
@@ -860,6 +905,7 @@ __global__ void __launch_bounds__(kCgThreads, PER_SM) batch_cg_kernel(const Batc
                 W->dev[i].step_iters[S.step[i]] = S.it[i];
                 W->dev[i].counter[0] = S.step[i] + 1;
             }
+    grid_wait_end(gw, W->bar);
 }
 
 }  // namespace

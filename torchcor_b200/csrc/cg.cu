@@ -38,6 +38,8 @@ __global__ void __launch_bounds__(kCgThreads, 2) cg_kernel(MonoDev d) {
     const int64_t s_end = (int64_t)(blockIdx.x + 1) * d.n_slices / nb;
     const int64_t n = d.counter[0];
     int32_t* err = d.counter + 1;
+    GridWait gw = grid_wait_begin(d.bar, err, d.wait);
+    if (*(volatile int32_t*)err != 0) return;   // an earlier launch gave up
     const float* __restrict__ u = d.x + ring_cur(n) * d.n_pad;
     const float* __restrict__ xp = d.x + ring_prev(n) * d.n_pad;
     float* __restrict__ x = d.x + ring_next(n) * d.n_pad;
@@ -83,7 +85,7 @@ __global__ void __launch_bounds__(kCgThreads, 2) cg_kernel(MonoDev d) {
         acc2[1] += (double)r32 * z;
     }
     block_partial<2>(acc2, parts0, sh_part);
-    if (!grid_barrier(d.bar, err, d.wait)) return;
+    if (!grid_barrier(gw)) return;
     double tot[2];
     grid_total<2>(parts0, tot, sh_tot);
     const double b_norm = sqrt(tot[0]);
@@ -109,7 +111,7 @@ __global__ void __launch_bounds__(kCgThreads, 2) cg_kernel(MonoDev d) {
         }
         __syncthreads();
         block_partial<1>(acc1, parts1, sh_part);
-        if (!grid_barrier(d.bar, err, d.wait)) return;
+        if (!grid_barrier(gw)) return;
         double pap[1];
         grid_total<1>(parts1, pap, sh_tot);
         const double alpha = rz / pap[0];
@@ -128,7 +130,7 @@ __global__ void __launch_bounds__(kCgThreads, 2) cg_kernel(MonoDev d) {
         }
         __syncthreads();
         block_partial<2>(acc2, parts0, sh_part);
-        if (!grid_barrier(d.bar, err, d.wait)) return;
+        if (!grid_barrier(gw)) return;
         grid_total<2>(parts0, tot, sh_tot);
         const double zn = sqrt(tot[0]);
         if (zn < d.a_tol || (zn / b_norm) < d.r_tol) break;   // solver.py:66-69
@@ -141,13 +143,14 @@ __global__ void __launch_bounds__(kCgThreads, 2) cg_kernel(MonoDev d) {
             if (row >= d.n) continue;
             p[row] = (float)(beta * (double)p[row] + (double)dinv[row] * (double)r[row]);
         }
-        if (!grid_barrier(d.bar, err, d.wait)) return;
+        if (!grid_barrier(gw)) return;
         ++it;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         d.step_iters[n] = it;
         d.counter[0] = (int32_t)(n + 1);
     }
+    grid_wait_end(gw, d.bar);
 }
 
 struct DeviceInfo {

@@ -27,18 +27,6 @@ struct WaitLimit {
     uint32_t drop_first_copy;
 };
 
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long long* p) {
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-
 __device__ __forceinline__ uint64_t globaltimer() {
     uint64_t t;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -51,45 +39,124 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// Grid-wide barrier with a bounded wait: returns false (and the kernel must
-// return) if any block recorded an error or the wait ran past the timeout.
-// One 64-bit word (bar[0..1], 8-byte aligned): arrivals in the low half, the
-// generation in the high half.  A block's arrival (one atomic add) returns the
-// generation it waits to see change; the last arrival adds 2^32 - gridDim.x,
-// which clears the count and advances the generation in one operation, so no
-// block can arrive at the next barrier before the count is clear.
-__device__ __forceinline__ bool grid_barrier(uint32_t* bar, int32_t* err, const WaitLimit& w) {
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int good = 1;
-        unsigned long long* word = reinterpret_cast<unsigned long long*>(bar);
-        __threadfence();   // this block's writes before its arrival
-        const unsigned long long old = atomicAdd(word, 1ull);
-        const unsigned gen = (unsigned)(old >> 32);
-        if ((unsigned)old == gridDim.x - 1 + w.extra_arrivals) {
-            atomicAdd(word, (1ull << 32) - (unsigned long long)gridDim.x);
-        } else {
-            const uint64_t t0 = globaltimer();
-            while ((unsigned)(ld_acquire64(word) >> 32) == gen) {
-                if (*(volatile int32_t*)err != 0) {
-                    good = 0;
-                    break;
-                }
-                if (globaltimer() - t0 > w.timeout_ns) {
-                    atomicCAS(err, 0, TCB_ETIMEOUT);
-                    good = 0;
-                    break;
-                }
-                __nanosleep(32);
+// Grid-wide barrier with a bounded wait.  bar[2] counts arrivals and only ever
+// grows (modulo 2^32); bar[3] is its value between launches, which every block
+// reads as it starts and block 0 writes as it ends.  A block arrives with an add
+// that returns nothing and polls the same word until all have: a fence, an add and a
+// poll, where a counter with a generation beside it took two round trips more (the
+// add's result, and the last arrival's second add).  On B200 the last arrival is
+// seen after 1.3 us, before 2.6.
+struct GridWait {
+    uint32_t* word;
+    uint32_t target;
+    int32_t* err;
+    WaitLimit lim;
+};
+__device__ __forceinline__ GridWait grid_wait_begin(uint32_t* bar, int32_t* err, const WaitLimit& w) {
+    return GridWait{bar + 2, bar[3], err, w};
+}
+// (a launch whose wait ran out leaves its error word set, and nothing runs after that)
+__device__ __forceinline__ void grid_wait_end(const GridWait& g, uint32_t* bar) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) bar[3] = g.target;
+}
+
+// One thread's part; false if the wait ran past the limit or, while waiting, another
+// block recorded an error (reading the error word after every barrier would cost a
+// round trip; a block that gave up is missing at the next one).
+__device__ __forceinline__ bool grid_arrive_and_wait(const GridWait& g) {
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");   // the block's writes before its arrival
+    asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(g.word) : "memory");
+    const uint32_t target = g.target + g.lim.extra_arrivals;
+    uint64_t t0 = 0;
+    for (int spin = 1;; ++spin) {
+        uint32_t v;
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(g.word) : "memory");
+        if ((int32_t)(v - target) >= 0) break;
+        if ((spin & 31) == 0) {
+            if (*(volatile int32_t*)g.err != 0) return false;
+            const uint64_t now = globaltimer();
+            if (t0 == 0) t0 = now;
+            if (now - t0 > g.lim.timeout_ns) {
+                atomicCAS(g.err, 0, TCB_ETIMEOUT);
+                return false;
             }
         }
-        __threadfence();
-        if (*(volatile int32_t*)err != 0) good = 0;
-        ok = good;
+    }
+    asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    return true;
+}
+
+// Every block's earlier writes are visible to every block after it; false: return.
+__device__ __forceinline__ bool grid_barrier(GridWait& g) {
+    __syncthreads();
+    g.target += gridDim.x;
+    int bad = 0;
+    if (threadIdx.x == 0) bad = !grid_arrive_and_wait(g);
+    return !__syncthreads_or(bad);
+}
+
+// The barrier with the totals over all threads of NV (4 or 8) float64 values, in
+// sh.total[0..NV) after it.  A warp's values are added by halving exchanges (each step
+// hands half of the values to the partner lane), the warps' by warp 0; after the
+// barrier warp j adds the blocks' value j.  parts: NV * SLOTS doubles, at least
+// gridDim.x slots; two alternating sets of them.
+template <int NV>
+struct GridSums {
+    double part[kCgWarps][NV];
+    double total[NV];
+};
+template <int NV, int SLOTS>
+__device__ __forceinline__ bool grid_barrier_sums(const double (&v)[NV], GridSums<NV>& sh, double* parts, GridWait& g) {
+    static_assert((NV == 4 || NV == 8) && kCgWarps == 16 && SLOTS % 32 == 0, "exchange pattern");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double a[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) a[i] = v[i];
+    int bit = 16;
+#pragma unroll
+    for (int half = NV / 2; half > 0; half >>= 1, bit >>= 1) {
+        const bool up = lane & bit;
+#pragma unroll
+        for (int i = 0; i < half; ++i) {
+            const double give = up ? a[i] : a[i + half], mine = up ? a[i + half] : a[i];
+            a[i] = mine + __shfl_xor_sync(0xffffffffu, give, bit);
+        }
+    }
+#pragma unroll
+    for (; bit > 0; bit >>= 1) a[0] += __shfl_xor_sync(0xffffffffu, a[0], bit);
+    // value (bits 4, 3[, 2] of the lane) is complete in every lane
+    if ((lane & (32 / NV - 1)) == 0) sh.part[warp][lane / (32 / NV)] = a[0];
+    __syncthreads();
+    g.target += gridDim.x;
+    int bad = 0;
+    if (warp == 0) {
+        constexpr int kPer = kCgWarps * NV / 32;   // warps a lane adds
+        const int q = lane % NV, w = lane / NV * kPer;
+        double t = sh.part[w][q];
+#pragma unroll
+        for (int j = 1; j < kPer; ++j) t += sh.part[w + j][q];
+#pragma unroll
+        for (int o = NV; o < 32; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane < NV) parts[lane * SLOTS + blockIdx.x] = t;
+        __syncwarp();
+        if (lane == 0) bad = !grid_arrive_and_wait(g);
+    }
+    if (__syncthreads_or(bad)) return false;
+    if (warp < NV) {
+        double t[SLOTS / 32];
+#pragma unroll
+        for (int k = 0; k < SLOTS / 32; ++k) {
+            const int i = lane + 32 * k;
+            t[k] = i < (int)gridDim.x ? __ldcg(parts + warp * SLOTS + i) : 0.0;
+        }
+        double sum = 0.0;
+#pragma unroll
+        for (int k = 0; k < SLOTS / 32; ++k) sum += t[k];
+        sum = warp_sum(sum);
+        if (lane == 0) sh.total[warp] = sum;
     }
     __syncthreads();
-    return ok != 0;
+    return true;
 }
 
 // Block partial of NV float64 values -> parts[blockIdx.x * NV + i] (fixed order).

@@ -58,11 +58,11 @@ namespace {
 
 using namespace cgk;
 
-constexpr int kThreads = 512;
-constexpr int kWarps = kThreads / 32;
+constexpr int kThreads = kCgThreads;
+constexpr int kWarps = kCgWarps;
 constexpr int kSums = 8;                  // sums of a CG pass (see pass_sums)
 constexpr int kSlots = 160;               // most blocks of a launch
-constexpr size_t kHeadBytes = 256;        // arrivals of all launches so far; their number when the launch began
+constexpr size_t kHeadBytes = 256;        // barrier words
 constexpr size_t kPartBytes = 2 * (size_t)kSums * kSlots * sizeof(double);
 
 // no ionic update: b' comes from the caller (tcb_mono_cg_run)
@@ -82,112 +82,10 @@ struct Ionic {
 struct StepsPlan {
     int32_t n_steps, cap_rows, cap_entries;        // rows and matrix entries a block has at most
     int32_t smem_bytes, held_at, state_at;         // byte offsets of the matrix and the state (0: not held)
-    uint32_t *arrivals, *base;                     // barrier word; its value between launches
+    uint32_t* bar;                                 // barrier words (GridWait)
     double* parts;                                 // [2 parities][kSums][kSlots] block sums
     float4* rec[2];                                // per-row records, n_pad each
 };
-
-// ---------------------------------------------------------------- grid barrier
-struct Shared {
-    double part[kWarps][kSums];
-    double total[kSums];
-};
-
-// One thread announces its block and waits until all have: an add without a
-// result and a poll of the same word, which only ever grows (`target` = its value
-// once everybody has arrived, modulo 2^32).  Bounded: false after the time limit or
-// when another block has recorded an error.
-__device__ __forceinline__ bool arrive_and_wait(uint32_t* word, uint32_t target, int32_t* err, const WaitLimit& lim) {
-    asm volatile("fence.acq_rel.gpu;" ::: "memory");   // the block's writes before its arrival
-    asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(word) : "memory");
-    target += lim.extra_arrivals;
-    uint64_t t0 = 0;
-    for (int spin = 1;; ++spin) {
-        uint32_t v;
-        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
-        if ((int32_t)(v - target) >= 0) break;
-        if ((spin & 31) == 0) {
-            if (*(volatile int32_t*)err != 0) return false;
-            const uint64_t now = globaltimer();
-            if (t0 == 0) t0 = now;
-            if (now - t0 > lim.timeout_ns) {
-                atomicCAS(err, 0, TCB_ETIMEOUT);
-                return false;
-            }
-        }
-    }
-    asm volatile("fence.acq_rel.gpu;" ::: "memory");
-    return true;
-}
-
-// Grid barrier: every block's earlier writes are visible to every block after it.
-__device__ __forceinline__ bool barrier(const StepsPlan& pl, uint32_t& target, int32_t* err, const WaitLimit& lim) {
-    __syncthreads();
-    target += gridDim.x;
-    int bad = 0;
-    if (threadIdx.x == 0) bad = !arrive_and_wait(pl.arrivals, target, err, lim);
-    return !__syncthreads_or(bad);
-}
-
-// Grid barrier that also returns the totals of kSums float64 values per thread.
-// A warp's values are added by halving exchanges (16 lanes' worth of four values,
-// then eight lanes' worth of two, ...), the warps' by warp 0; after the barrier warp j
-// adds the blocks' value j.
-__device__ __forceinline__ bool barrier_sums(double (&v)[kSums], Shared& sh, const StepsPlan& pl, uint32_t& target,
-                                             int parity, int32_t* err, const WaitLimit& lim) {
-    static_assert(kSums == 8 && kWarps == 16, "exchange pattern");
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double a[4], b[2], c;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const bool up = lane & 16;
-        const double give = up ? v[i] : v[i + 4], mine = up ? v[i + 4] : v[i];
-        a[i] = mine + __shfl_xor_sync(0xffffffffu, give, 16);
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const bool up = lane & 8;
-        const double give = up ? a[i] : a[i + 2], mine = up ? a[i + 2] : a[i];
-        b[i] = mine + __shfl_xor_sync(0xffffffffu, give, 8);
-    }
-    {
-        const bool up = lane & 4;
-        const double give = up ? b[0] : b[1], mine = up ? b[1] : b[0];
-        c = mine + __shfl_xor_sync(0xffffffffu, give, 4);
-    }
-    c += __shfl_xor_sync(0xffffffffu, c, 2);
-    c += __shfl_xor_sync(0xffffffffu, c, 1);
-    if ((lane & 3) == 0) sh.part[warp][((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1)] = c;
-    __syncthreads();
-    double* parts = pl.parts + (size_t)parity * kSums * kSlots;
-    target += gridDim.x;
-    int bad = 0;
-    if (warp == 0) {
-        const int q = lane & 7, g = lane >> 3;
-        double t = (sh.part[4 * g][q] + sh.part[4 * g + 1][q]) + (sh.part[4 * g + 2][q] + sh.part[4 * g + 3][q]);
-        t += __shfl_xor_sync(0xffffffffu, t, 8);
-        t += __shfl_xor_sync(0xffffffffu, t, 16);
-        if (lane < kSums) parts[q * kSlots + blockIdx.x] = t;
-        __syncwarp();
-        if (lane == 0) bad = !arrive_and_wait(pl.arrivals, target, err, lim);
-    }
-    if (__syncthreads_or(bad)) return false;
-    if (warp < kSums) {
-        double t[kSlots / 32];
-#pragma unroll
-        for (int k = 0; k < kSlots / 32; ++k) {
-            const int i = lane + 32 * k;
-            t[k] = i < (int)gridDim.x ? __ldcg(parts + warp * kSlots + i) : 0.0;
-        }
-        double sum = 0.0;
-#pragma unroll
-        for (int k = 0; k < kSlots / 32; ++k) sum += t[k];
-        sum = warp_sum(sum);
-        if (lane == 0) sh.total[warp] = sum;
-    }
-    __syncthreads();
-    return true;
-}
 
 // alpha as a pair of float32 (high and low part) for advance()
 struct Alpha {
@@ -324,7 +222,7 @@ template <typename IDX, bool ASPLIT, class ION>
 __global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, const IDX* __restrict__ col, StepsPlan pl,
                                                                  ION ion) {
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ Shared sh;
+    __shared__ GridSums<kSums> sh;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t s_begin = (int64_t)blockIdx.x * d.n_slices / gridDim.x;
     const int64_t s_end = (int64_t)(blockIdx.x + 1) * d.n_slices / gridDim.x;
@@ -333,7 +231,7 @@ __global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, cons
     const int rows = (int)((d.n < s_end * TCB_SLICE ? d.n : s_end * TCB_SLICE) - row0);
     int32_t* err = d.counter + 1;
     const int first_step = d.counter[0];
-    uint32_t arrived = *pl.base;
+    GridWait g = grid_wait_begin(pl.bar, err, d.wait);
     int parity = 0;
     if (*(volatile int32_t*)err != 0) return;
 
@@ -420,7 +318,7 @@ __global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, cons
                 q4[row0 + i] = q;
             }
         }
-        if (!barrier(pl, arrived, err, d.wait)) return;
+        if (!grid_barrier(g)) return;
 
         // ---- right-hand side, r0, z0 (monodomain.py:130-131, solver.py:46-55)
         double sums[kSums];
@@ -447,7 +345,7 @@ __global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, cons
             const double db = (double)di * (double)rhs;
             sums[7] += db * db;
         }
-        if (!barrier(pl, arrived, err, d.wait)) return;
+        if (!grid_barrier(g)) return;
 
         int it = 0;
         Alpha alpha = {0.0f, 0.0f};
@@ -481,7 +379,7 @@ __global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, cons
                 rout[i] = out;
                 gout[row0 + i] = out;
             }
-            if (!barrier_sums(sums, sh, pl, arrived, parity ^= 1, err, d.wait)) return;
+            if (!grid_barrier_sums<kSums, kSlots>(sums, sh, pl.parts + (size_t)(parity ^= 1) * kSums * kSlots, g)) return;
             const double rz = sh.total[5];
             if (it == 0) b_norm = sqrt(sh.total[7]);
             const double al = rz / sh.total[0];
@@ -493,7 +391,7 @@ __global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, cons
                 if (i < rows) sx[i] = (float)((double)sx[i] + al * (double)rout[i].y);
             }
             const double zn = sqrt(zz < 0.0 ? 0.0 : zz);
-            if (zn < d.a_tol || (zn / b_norm) < d.r_tol) break;   // solver.py:66-69
+            if (zn < d.a_tol || zn < d.r_tol * b_norm) break;   // solver.py:66-69
             beta = (float)(rz1 / rz);
             ++it;
 #pragma unroll
@@ -517,8 +415,8 @@ __global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, cons
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         d.counter[0] = last_step;
-        *pl.base = arrived;
     }
+    grid_wait_end(g, pl.bar);
 }
 
 // ---------------------------------------------------------------- launch
@@ -532,7 +430,7 @@ const StepsInfo& steps_info() {
     StepsInfo& si = infos[dev & 63];
     if (si.sms == 0) {
         cudaDeviceGetAttribute(&si.max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        si.max_smem -= (int)sizeof(Shared) + 1024;
+        si.max_smem -= (int)sizeof(GridSums<kSums>) + 1024;
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         si.sms = sms;
@@ -574,8 +472,7 @@ bool steps_plan(const tcb_mono* m, const MonoDev& d, int states, StepsPlan* pl) 
     if (!m->work || m->work_entries <= 0 || m->fused_step != 0 || cg_forced_fallback()) return false;
     if (!steps_layout(d, m->work_entries, states, pl)) return false;
     unsigned char* w = static_cast<unsigned char*>(m->work);
-    pl->arrivals = reinterpret_cast<uint32_t*>(w);
-    pl->base = reinterpret_cast<uint32_t*>(w + kHeadBytes / 2);
+    pl->bar = reinterpret_cast<uint32_t*>(w);
     pl->parts = reinterpret_cast<double*>(w + kHeadBytes);
     pl->rec[0] = reinterpret_cast<float4*>(w + kHeadBytes + kPartBytes);
     pl->rec[1] = pl->rec[0] + d.n_pad;
