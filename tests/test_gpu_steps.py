@@ -65,6 +65,8 @@ def _run(sim, tol, max_iter, guess, fused_step, chunks, frames=False):
     ("cube", 9, "crn", 1e-8, 100, False, 0.5),      # many passes a step
     ("cube", 11, "ms", 1e-8, 2, True, 0.5),         # stopped by max_iter
     ("cube", 11, "ms", 1e-5, 0, True, 0.5),         # no pass at all
+    ("cube", 15, "crn", 1e-6, 100, True, 0.5),      # 4,096 nodes: a full cluster of 16 blocks, whole slices
+    ("cube", 16, "ttp", 1e-6, 100, True, 0.5),      # 4,913 nodes: the smallest grid
     ("cube", 13, "ttp", 1e-6, 100, True, 0.25),     # A is not M Cm + K'
     ("ico", 3, "crn", 1e-6, 100, True, 0.5),        # rows of 6 and 7 entries
     ("ico", 6, "ms", 1e-6, 100, True, 0.5),         # 32-bit columns

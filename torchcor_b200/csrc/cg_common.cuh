@@ -105,9 +105,10 @@ struct GridSums {
     double part[kCgWarps][NV];
     double total[NV];
 };
-template <int NV, int SLOTS>
-__device__ __forceinline__ bool grid_barrier_sums(const double (&v)[NV], GridSums<NV>& sh, double* parts, GridWait& g) {
-    static_assert((NV == 4 || NV == 8) && kCgWarps == 16 && SLOTS % 32 == 0, "exchange pattern");
+// every warp: its lanes' values into sh.part[warp]
+template <int NV>
+__device__ __forceinline__ void fold_warps(const double (&v)[NV], GridSums<NV>& sh) {
+    static_assert(NV == 4 || NV == 8, "exchange pattern");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double a[NV];
 #pragma unroll
@@ -126,17 +127,29 @@ __device__ __forceinline__ bool grid_barrier_sums(const double (&v)[NV], GridSum
     for (; bit > 0; bit >>= 1) a[0] += __shfl_xor_sync(0xffffffffu, a[0], bit);
     // value (bits 4, 3[, 2] of the lane) is complete in every lane
     if ((lane & (32 / NV - 1)) == 0) sh.part[warp][lane / (32 / NV)] = a[0];
+}
+// one warp, after the block has met: the block's value lane % NV, in every lane
+template <int NV>
+__device__ __forceinline__ double fold_block(const GridSums<NV>& sh) {
+    constexpr int kPer = kCgWarps * NV / 32;   // warps a lane adds
+    const int lane = threadIdx.x & 31, q = lane % NV, w = lane / NV * kPer;
+    double t = sh.part[w][q];
+#pragma unroll
+    for (int j = 1; j < kPer; ++j) t += sh.part[w + j][q];
+#pragma unroll
+    for (int o = NV; o < 32; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+}
+template <int NV, int SLOTS>
+__device__ __forceinline__ bool grid_barrier_sums(const double (&v)[NV], GridSums<NV>& sh, double* parts, GridWait& g) {
+    static_assert(SLOTS % 32 == 0, "whole strides");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    fold_warps<NV>(v, sh);
     __syncthreads();
     g.target += gridDim.x;
     int bad = 0;
     if (warp == 0) {
-        constexpr int kPer = kCgWarps * NV / 32;   // warps a lane adds
-        const int q = lane % NV, w = lane / NV * kPer;
-        double t = sh.part[w][q];
-#pragma unroll
-        for (int j = 1; j < kPer; ++j) t += sh.part[w + j][q];
-#pragma unroll
-        for (int o = NV; o < 32; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        const double t = fold_block<NV>(sh);
         if (lane < NV) parts[lane * SLOTS + blockIdx.x] = t;
         __syncwarp();
         if (lane == 0) bad = !grid_arrive_and_wait(g);

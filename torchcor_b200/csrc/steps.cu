@@ -29,11 +29,16 @@
 // 1.7 us, one of them with the sums 2.3 us; the ionic update's table reads 1-3 us;
 // column, gather and sum of a row 1-2 us a pass), not bytes.  Measured on B200, us a
 // step with x CG iterations, the two launches of a step replayed as a CUDA graph ->
-// here: TTP cube 1,000 nodes (0) 26.0 -> 10.8; MS cube 9,261 (0.4) 34.9 -> 12.1; TTP
+// here: TTP cube 1,000 nodes (1.15) 26 -> 10.7 (a cluster); MS cube 9,261 (0.4) 34.9 -> 12.1; TTP
 // cube 50,653 (1) 43.1 -> 17.7, 117,649 (0.8) 48.6 -> 26.0; CRN shell 40,962 (1) 36.6
 // -> 15.8, 163,842 (1) 51.7 -> 31.8.  The line to the two-launch form lies where the
 // matrix no longer fits (about 170,000 nodes of a tetrahedral mesh): reading it from
 // L2 instead, 262,144 nodes took 59.9 us here and 49.1 in two launches.
+//
+// The smallest meshes run as one thread-block cluster instead of a grid: its barrier
+// is the hardware's, sums and neighbours' records travel through distributed shared
+// memory and nothing goes through L2.  (A neighbour in the block itself is read the
+// same way: telling it apart with a predicate took half as long again.)
 //
 // Sums inside a row run in the order of the other CG kernels (M b' and K u in
 // float32, A x0 and A p in float64); sums over rows are float64 in an order that
@@ -42,6 +47,7 @@
 #include <math.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "cg_common.cuh"
@@ -80,7 +86,8 @@ struct Ionic {
 };
 
 struct StepsPlan {
-    int32_t n_steps, cap_rows, cap_entries;        // rows and matrix entries a block has at most
+    int32_t n_steps, blocks, cluster;              // cluster: the blocks are one cluster
+    int32_t cap_rows, cap_entries;                 // rows and matrix entries a block has at most
     int32_t smem_bytes, held_at, state_at;         // byte offsets of the matrix and the state (0: not held)
     uint32_t* bar;                                 // barrier words (GridWait)
     double* parts;                                 // [2 parities][kSums][kSlots] block sums
@@ -115,16 +122,18 @@ __device__ __forceinline__ void advance(const float4& f, const Alpha& alpha, flo
     p = __fmaf_rn(beta, f.y, z);
 }
 
-// the sums of one CG pass for a row
-__device__ __forceinline__ void pass_sums(double (&s)[kSums], float r, float z, float p, float ap, float di) {
-    const double d_ap = (double)ap, dap = (double)di * d_ap, dr = (double)di * (double)r;
+// The sums of one CG pass for a row.  All are of the unrounded D r and D A p: where
+// |z'| is far below |z| the identities cancel, and sums over the rounded z beside
+// unrounded products would leave 1e-5 of |z'|^2.
+__device__ __forceinline__ void pass_sums(double (&s)[kSums], float r, float p, float ap, float di) {
+    const double d_ap = (double)ap, d_r = (double)r, dap = (double)di * d_ap, dr = (double)di * d_r;
     s[0] += (double)p * d_ap;
     s[1] += dr * d_ap;
     s[2] += dap * d_ap;
     s[3] += dr * dap;
     s[4] += dap * dap;
-    s[5] += (double)r * (double)z;
-    s[6] += (double)z * (double)z;
+    s[5] += dr * d_r;
+    s[6] += dr * dr;
 }
 
 // copy `bytes` (a multiple of 64; both sides 16-byte aligned) into shared memory, whole block
@@ -133,30 +142,80 @@ __device__ __forceinline__ void hold(void* dst, const void* src, size_t bytes) {
         static_cast<uint4*>(dst)[i] = static_cast<const uint4*>(src)[i];
 }
 
-// The block's part of the matrix in shared memory and where its neighbours' values are.
-template <typename IDX>
+// Address in the cluster's shared memory of what is at `local` in this block's.
+__device__ __forceinline__ uint32_t peer_address(const void* local, uint32_t rank) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(local)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void peer_load(float& v, uint32_t a) {
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a));
+}
+__device__ __forceinline__ void peer_load(float4& v, uint32_t a) {
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// The block's part of the matrix in shared memory and where its neighbours' values
+// are.  CL: the blocks are one cluster, and a column is (block << 16 | row of the block).
+template <typename IDX, bool CL>
 struct Rows {
-    const IDX* col;       // int16: column - row; int32: column
+    const std::conditional_t<CL, uint32_t, IDX>* col;   // int16: column - row; int32: column
     const float *m, *k, *a;
     int row0, rows;
     float cm;
     __device__ __forceinline__ int column(int e, int i) const {
-        return sizeof(IDX) == 2 ? row0 + i + (int)col[e] : (int)col[e];
+        return !CL && sizeof(IDX) == 2 ? row0 + i + (int)col[e] : (int)col[e];
     }
-    // a neighbour's value: the block's own rows from shared memory, others through L1
+    // a neighbour's value: from the shared memory of its block (CL); else the block's own rows from
+    // shared memory, others through L1
     template <class T>
     __device__ __forceinline__ T value(const T* own, const T* all, int c) const {
+        if constexpr (CL) {
+            T v;
+            peer_load(v, peer_address(own + (c & 0xffff), (uint32_t)c >> 16));
+            return v;
+        }
         const int l = c - row0;
         const T* p = (unsigned)l < (unsigned)rows ? own + l : all + c;
         return *p;
     }
 };
 
+// grid_barrier_sums among the blocks of one cluster: warp 0 hands the block's sums to
+// every block, and each adds them in block order.
+constexpr int kMaxCluster = 16;
+struct ClusterSums {
+    double from[2][kMaxCluster][kSums];
+};
+__device__ __forceinline__ void cluster_barrier_sums(double (&v)[kSums], GridSums<kSums>& sh, ClusterSums& cs, int parity) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nb = (int)gridDim.x;
+    fold_warps<kSums>(v, sh);
+    __syncthreads();
+    if (warp == 0) {
+        const double t = fold_block<kSums>(sh);   // value lane % kSums, in every lane
+        for (int r = lane / kSums; r < nb; r += 32 / kSums)
+            asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(peer_address(&cs.from[parity][blockIdx.x][lane % kSums], (uint32_t)r)),
+                         "d"(t)
+                         : "memory");
+    }
+    cluster_barrier();
+    if (warp < kSums) {
+        double t = lane < nb ? cs.from[parity][lane][warp] : 0.0;
+#pragma unroll
+        for (int o = kMaxCluster / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) sh.total[warp] = t;
+    }
+    __syncthreads();
+}
+
 // Entries 0 .. w-1 of a row, C at a time, without branches: entries past the end
 // repeat the last one with a coefficient of zero.  All C gathers are in flight
 // before the first is used.
-template <int C, bool ASPLIT, typename IDX>
-__device__ __forceinline__ void row_rhs(const Rows<IDX>& R, const float4* own, const float4* all, int base, int w, int i,
+template <int C, bool ASPLIT, typename IDX, bool CL>
+__device__ __forceinline__ void row_rhs(const Rows<IDX, CL>& R, const float4* own, const float4* all, int base, int w, int i,
                                         float& mb, float& ku, double& ax) {
     for (int k0 = 0; k0 < w; k0 += C) {
         float4 q[C];
@@ -177,14 +236,14 @@ __device__ __forceinline__ void row_rhs(const Rows<IDX>& R, const float4* own, c
     }
 }
 
-template <bool ASPLIT, typename IDX>
-__device__ __forceinline__ float coefficient(const Rows<IDX>& R, int e) {
+template <bool ASPLIT, typename IDX, bool CL>
+__device__ __forceinline__ float coefficient(const Rows<IDX, CL>& R, int e) {
     if constexpr (ASPLIT) return __fadd_rn(__fmul_rn(R.m[e], R.cm), R.k[e]);
     else return R.a[e];
 }
 
-template <int C, bool ASPLIT, typename IDX>
-__device__ __forceinline__ double row_first(const Rows<IDX>& R, const float* own, const float* all, int base, int w, int i) {
+template <int C, bool ASPLIT, typename IDX, bool CL>
+__device__ __forceinline__ double row_first(const Rows<IDX, CL>& R, const float* own, const float* all, int base, int w, int i) {
     double acc = 0.0;
     for (int k0 = 0; k0 < w; k0 += C) {
         float z[C];
@@ -199,8 +258,8 @@ __device__ __forceinline__ double row_first(const Rows<IDX>& R, const float* own
     return acc;
 }
 
-template <int C, bool ASPLIT, typename IDX>
-__device__ __forceinline__ double row_next(const Rows<IDX>& R, const float4* own, const float4* all, int base, int w, int i,
+template <int C, bool ASPLIT, typename IDX, bool CL>
+__device__ __forceinline__ double row_next(const Rows<IDX, CL>& R, const float4* own, const float4* all, int base, int w, int i,
                                            const Alpha& alpha, float beta) {
     double acc = 0.0;
     for (int k0 = 0; k0 < w; k0 += C) {
@@ -218,11 +277,12 @@ __device__ __forceinline__ double row_next(const Rows<IDX>& R, const float4* own
     return acc;
 }
 
-template <typename IDX, bool ASPLIT, class ION>
+template <typename IDX, bool ASPLIT, bool CL, class ION>
 __global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, const IDX* __restrict__ col, StepsPlan pl,
                                                                  ION ion) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ GridSums<kSums> sh;
+    __shared__ std::conditional_t<CL, ClusterSums, char> cs;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t s_begin = (int64_t)blockIdx.x * d.n_slices / gridDim.x;
     const int64_t s_end = (int64_t)(blockIdx.x + 1) * d.n_slices / gridDim.x;
@@ -248,11 +308,12 @@ __global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, cons
     float* sm = reinterpret_cast<float*>(held);
     float* sk = reinterpret_cast<float*>(held + vals);
     float* sa = ASPLIT ? sk : reinterpret_cast<float*>(held + 2 * vals);
-    IDX* sc = reinterpret_cast<IDX*>(held + (ASPLIT ? 2 : 3) * vals);
+    using COL = std::conditional_t<CL, uint32_t, IDX>;
+    COL* sc = reinterpret_cast<COL*>(held + (ASPLIT ? 2 : 3) * vals);
     float* ss = reinterpret_cast<float*>(smem + pl.state_at);
     const int64_t e0 = d.slice_ptr[s_begin];
     const size_t ent = (size_t)(d.slice_ptr[s_end] - e0);   // multiple of 32, at most cap_entries
-    hold(sc, col + e0, ent * sizeof(IDX));
+    if constexpr (!CL) hold(sc, col + e0, ent * sizeof(IDX));
     hold(sm, d.mv + e0, ent * 4);
     hold(sk, d.kv + e0, ent * 4);
     if (!ASPLIT) hold(sa, d.av + e0, ent * 4);
@@ -269,12 +330,40 @@ __global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, cons
         rec0[i].w = d.dinv[row0 + i];
     }
     __syncthreads();
+    if constexpr (CL) {
+        // columns as (block, row of the block): block b has the slices from b*S/nb on
+        const uint32_t S = (uint32_t)d.n_slices, nb = gridDim.x;
+        for (int s = warp; s < slices; s += kWarps)
+            for (int e = off[s] + lane; e < off[s + 1]; e += TCB_SLICE) {
+                const uint32_t c = (uint32_t)(row0 + s * TCB_SLICE + lane + (int)col[e0 + e]);
+                const uint32_t b = ((c / TCB_SLICE + 1) * nb - 1) / S;
+                sc[e] = b << 16 | (c - b * S / nb * TCB_SLICE);
+            }
+    }
 
-    const Rows<IDX> R{sc, sm, sk, sa, row0, rows, d.cm};
+    const Rows<IDX, CL> R{sc, sm, sk, sa, row0, rows, d.cm};
     const bool lg = d.linear_guess != 0;
     float* zg = d.r;
     float4* q4 = pl.rec[1];        // {b', u, x0, -}; read before the first pass that writes rec[1]
     const int last_step = first_step + pl.n_steps;
+    // (the barriers of a cluster are the hardware's and need no limit)
+    auto barrier = [&] {
+        if constexpr (CL) {
+            cluster_barrier();
+            return true;
+        } else {
+            return grid_barrier(g);
+        }
+    };
+    auto barrier_sums = [&](double (&v)[kSums]) {
+        parity ^= 1;
+        if constexpr (CL) {
+            cluster_barrier_sums(v, sh, cs, parity);
+            return true;
+        } else {
+            return grid_barrier_sums<kSums, kSlots>(v, sh, pl.parts + (size_t)parity * kSums * kSlots, g);
+        }
+    };
     for (int n = first_step; n < last_step; ++n) {
         // ---- ionic update of the block's rows, b', guess (monodomain.py:117-128, solver.py:35-38)
         {
@@ -315,10 +404,10 @@ __global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, cons
                 }
                 const float4 q = make_float4(bp, u, lg ? 2.0f * u - sxp[i] : u, 0.0f);
                 rec1[i] = q;
-                q4[row0 + i] = q;
+                if constexpr (!CL) q4[row0 + i] = q;
             }
         }
-        if (!grid_barrier(g)) return;
+        if (!barrier()) return;
 
         // ---- right-hand side, r0, z0 (monodomain.py:130-131, solver.py:46-55)
         double sums[kSums];
@@ -341,11 +430,11 @@ __global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, cons
             const float z = __fmul_rn(di, r);
             rec0[i].x = r;
             sz[i] = z;
-            zg[row0 + i] = z;
+            if constexpr (!CL) zg[row0 + i] = z;
             const double db = (double)di * (double)rhs;
             sums[7] += db * db;
         }
-        if (!grid_barrier(g)) return;
+        if (!barrier()) return;
 
         int it = 0;
         Alpha alpha = {0.0f, 0.0f};
@@ -374,12 +463,12 @@ __global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, cons
                     advance(f, alpha, beta, r, z, p);
                     ap = (float)row_next<8, ASPLIT>(R, rin, gin, base, w, i, alpha, beta);
                 }
-                pass_sums(sums, r, z, p, ap, di);
+                pass_sums(sums, r, p, ap, di);
                 const float4 out = make_float4(r, p, ap, di);
                 rout[i] = out;
-                gout[row0 + i] = out;
+                if constexpr (!CL) gout[row0 + i] = out;
             }
-            if (!grid_barrier_sums<kSums, kSlots>(sums, sh, pl.parts + (size_t)(parity ^= 1) * kSums * kSlots, g)) return;
+            if (!barrier_sums(sums)) return;
             const double rz = sh.total[5];
             if (it == 0) b_norm = sqrt(sh.total[7]);
             const double al = rz / sh.total[0];
@@ -416,7 +505,7 @@ __global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, cons
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         d.counter[0] = last_step;
     }
-    grid_wait_end(g, pl.bar);
+    if constexpr (!CL) grid_wait_end(g, pl.bar);
 }
 
 // ---------------------------------------------------------------- launch
@@ -430,7 +519,7 @@ const StepsInfo& steps_info() {
     StepsInfo& si = infos[dev & 63];
     if (si.sms == 0) {
         cudaDeviceGetAttribute(&si.max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        si.max_smem -= (int)sizeof(GridSums<kSums>) + 1024;
+        si.max_smem -= (int)(sizeof(GridSums<kSums>) + sizeof(ClusterSums)) + 1024;
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         si.sms = sms;
@@ -441,24 +530,35 @@ const StepsInfo& steps_info() {
 constexpr int kMinSlices = 8;              // slices a block has at least
 constexpr int kHoldStateFrom = 4;          // shorter launches update the ionic state where it is
 constexpr int64_t kStepsPerLaunch = 128;   // about a millisecond or a few: other streams get their turn
+// Meshes of up to this many slices (4,608 nodes) run as one cluster of at most 16
+// blocks.  us a step with x CG iterations, grid -> cluster: TTP cube 1,000 nodes (1.15)
+// 14.4 -> 10.7, 2,197 (2.1) 18.7 -> 14.1, 4,096 (1.75) 19.3 -> 15.6; beyond, the rows of a
+// block weigh more than the barriers: 6,859 (1.4) 17.3 -> 19.0, MS 9,261 (0) 10.1 -> 12.5.
+constexpr int kClusterSlices = 144;
+constexpr int32_t kClusterWork = 1 << 30;  // tcb_mono.work_entries: entries are counted for a cluster's blocks
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
-unsigned steps_blocks(const MonoDev& d) {
-    const int64_t nb = std::min<int64_t>(ceil_div(d.n_slices, kMinSlices), std::min(steps_info().sms, kSlots));
-    return (unsigned)std::max<int64_t>(nb, 1);
+int64_t steps_blocks(const MonoDev& d, bool cluster) {
+    const int64_t nb = std::max<int64_t>(ceil_div(d.n_slices, kMinSlices), 1);
+    if (!cluster) return std::min<int64_t>(nb, std::min(steps_info().sms, kSlots));
+    int64_t p = 1;
+    while (p < nb && p < kMaxCluster) p *= 2;
+    return std::min(p, d.n_slices);
 }
 
 // Shared memory of a block with at most `entries` matrix entries; false where it
 // does not fit (the matrix has to; the ionic state stays in global memory if need be).
-bool steps_layout(const MonoDev& d, int64_t entries, int states, StepsPlan* pl) {
+bool steps_layout(const MonoDev& d, int64_t blocks, int64_t entries, int states, bool cluster, StepsPlan* pl) {
     const size_t max = (size_t)steps_info().max_smem;
     auto up = [](size_t b) { return (b + 127) / 128 * 128; };
-    const int64_t cap = ceil_div(d.n_slices, steps_blocks(d)) * TCB_SLICE;
+    const int64_t cap = ceil_div(d.n_slices, blocks) * TCB_SLICE;
     const size_t fixed = (size_t)cap * 44 + up((size_t)(cap / TCB_SLICE + 1) * 4);
-    const size_t per_entry = (d.a_split ? 8 : 12) + (d.dcol ? 2 : 4);
+    const size_t per_entry = (d.a_split ? 8 : 12) + (d.dcol && !cluster ? 2 : 4);
     const size_t matrix = up((size_t)entries * per_entry), state = (size_t)cap * 4 * states;
     if (cap > 16384 || entries > (1 << 20) || fixed + matrix > max) return false;
+    pl->blocks = (int)blocks;
+    pl->cluster = cluster;
     pl->cap_rows = (int)cap;
     pl->cap_entries = (int)entries;
     pl->held_at = (int)fixed;
@@ -468,9 +568,13 @@ bool steps_layout(const MonoDev& d, int64_t entries, int states, StepsPlan* pl) 
 }
 
 // false where the step-by-step launches run instead
-bool steps_plan(const tcb_mono* m, const MonoDev& d, int states, StepsPlan* pl) {
+bool steps_plan(const tcb_mono* m, const MonoDev& d, bool ionic, int states, StepsPlan* pl) {
     if (!m->work || m->work_entries <= 0 || m->fused_step != 0 || cg_forced_fallback()) return false;
-    if (!steps_layout(d, m->work_entries, states, pl)) return false;
+    const bool as_cluster = (m->work_entries & kClusterWork) != 0;
+    // the blocks counted for a cluster also run as a grid: where the cluster form is not compiled (ionic
+    // steps whose A is not M Cm + K'), and for the tests that let a grid barrier's wait run out
+    const bool cluster = as_cluster && (d.a_split || !ionic) && d.wait.extra_arrivals == 0;
+    if (!steps_layout(d, steps_blocks(d, as_cluster), m->work_entries & ~kClusterWork, states, cluster, pl)) return false;
     unsigned char* w = static_cast<unsigned char*>(m->work);
     pl->bar = reinterpret_cast<uint32_t*>(w);
     pl->parts = reinterpret_cast<double*>(w + kHeadBytes);
@@ -479,24 +583,31 @@ bool steps_plan(const tcb_mono* m, const MonoDev& d, int states, StepsPlan* pl) 
     return true;
 }
 
-template <typename IDX, bool ASPLIT, class ION>
+template <typename IDX, bool ASPLIT, bool CL, class ION>
 int launch(const MonoDev& d, const IDX* col, const StepsPlan& pl, const ION& ion, cudaStream_t s) {
     static bool configured[64] = {};
     int dev = 0;
     TCB_CHECK_CUDA(cudaGetDevice(&dev));
-    const void* fn = (const void*)mono_steps_kernel<IDX, ASPLIT, ION>;
+    const void* fn = (const void*)mono_steps_kernel<IDX, ASPLIT, CL, ION>;
     if (!configured[dev & 63]) {
         TCB_CHECK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, steps_info().max_smem));
+        if (CL) TCB_CHECK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         configured[dev & 63] = true;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(steps_blocks(d));
+    cfg.gridDim = dim3((unsigned)pl.blocks);
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = (size_t)pl.smem_bytes;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
+    if (CL) {   // one cluster: its blocks run together by themselves
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)pl.blocks;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    } else {
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+    }
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     void* args[] = {const_cast<MonoDev*>(&d), &col, const_cast<StepsPlan*>(&pl), const_cast<ION*>(&ion)};
@@ -507,9 +618,16 @@ int launch(const MonoDev& d, const IDX* col, const StepsPlan& pl, const ION& ion
 
 template <class ION>
 int launch_any(const MonoDev& d, const StepsPlan& pl, const ION& ion, cudaStream_t s) {
+    if (pl.cluster) {
+        if constexpr (!ION::kIonic)
+            if (!d.a_split) return launch<int16_t, false, true, ION>(d, d.dcol, pl, ion, s);
+        return launch<int16_t, true, true, ION>(d, d.dcol, pl, ion, s);
+    }
     if (d.dcol)
-        return d.a_split ? launch<int16_t, true, ION>(d, d.dcol, pl, ion, s) : launch<int16_t, false, ION>(d, d.dcol, pl, ion, s);
-    return d.a_split ? launch<int32_t, true, ION>(d, d.col, pl, ion, s) : launch<int32_t, false, ION>(d, d.col, pl, ion, s);
+        return d.a_split ? launch<int16_t, true, false, ION>(d, d.dcol, pl, ion, s)
+                         : launch<int16_t, false, false, ION>(d, d.dcol, pl, ion, s);
+    return d.a_split ? launch<int32_t, true, false, ION>(d, d.col, pl, ion, s)
+                     : launch<int32_t, false, false, ION>(d, d.col, pl, ion, s);
 }
 
 template <class M, class Q>
@@ -520,6 +638,34 @@ int launch_model(const tcb_mono* m, const MonoDev& d, const StepsPlan& pl, cudaS
     return launch_any(d, pl, ion, s);
 }
 
+// whether the device takes a cluster of kMaxCluster blocks with all of the shared memory
+bool cluster_fits() {
+    static int fits[64] = {};   // 0 not asked yet, 1 yes, 2 no
+    int dev = 0;
+    cudaGetDevice(&dev);
+    int& f = fits[dev & 63];
+    if (f == 0) {
+        const void* fn = (const void*)mono_steps_kernel<int16_t, true, true, GivenRhs>;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kMaxCluster);
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = (size_t)steps_info().max_smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = kMaxCluster;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        const bool ok = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, steps_info().max_smem) == cudaSuccess &&
+                        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess && clusters >= 1;
+        if (!ok) cudaGetLastError();
+        f = ok ? 1 : 2;
+    }
+    return f == 1;
+}
+
 }  // namespace
 
 // Steps [counter, counter + n_steps) as persistent launches of up to kStepsPerLaunch steps:
@@ -528,7 +674,7 @@ int launch_steps(const tcb_mono* m, const MonoDev& d, int64_t n_steps, bool ioni
     StepsPlan pl;
     constexpr int kStates[4] = {0, MS::kStates, TTP::kStates, CRN::kStates};
     if (ionic && (m->model < TCB_MODEL_MS || m->model > TCB_MODEL_CRN)) return 0;
-    if (!steps_plan(m, d, ionic ? kStates[m->model] : 0, &pl)) return 0;
+    if (!steps_plan(m, d, ionic, ionic ? kStates[m->model] : 0, &pl)) return 0;
     int32_t count, v, b, fast = 0, staged;
     if (ionic) {
         // the chosen instance's division policy
@@ -561,18 +707,29 @@ extern "C" int64_t tcb_mono_work_bytes(const tcb_mono* m, int32_t* entries, void
     *entries = 0;
     const MonoDev d = make_dev(m);
     StepsPlan pl;
-    // (16-byte copies of the matrix; nothing to ask the device for where even an empty matrix would not fit)
+    // (16-byte copies of the matrix; nothing to ask the device for where even one entry a row would not fit)
     if (m->fused_step != 0 || cg_forced_fallback() || !aligned16(d.dcol ? (const void*)d.dcol : (const void*)d.col) ||
-        !aligned16(d.mv) || !aligned16(d.kv) || !aligned16(d.av) || !steps_layout(d, TCB_SLICE * ceil_div(d.n_slices, steps_blocks(d)), 0, &pl))
+        !aligned16(d.mv) || !aligned16(d.kv) || !aligned16(d.av))
         return 0;
+    const int64_t grid = steps_blocks(d, false);
+    if (!steps_layout(d, grid, TCB_SLICE * ceil_div(d.n_slices, grid), 0, false, &pl)) return 0;
     std::vector<int64_t> sp((size_t)d.n_slices + 1);
     cudaStream_t s = as_stream(stream);
     TCB_CHECK_CUDA(cudaMemcpyAsync(sp.data(), d.slice_ptr, sp.size() * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     TCB_CHECK_CUDA(cudaStreamSynchronize(s));
-    const int64_t nb = steps_blocks(d);
-    int64_t most = 0;
-    for (int64_t b = 0; b < nb; ++b) most = std::max(most, sp[(b + 1) * d.n_slices / nb] - sp[b * d.n_slices / nb]);
-    if (!steps_layout(d, most, 0, &pl)) return 0;
-    *entries = (int32_t)most;
+    auto most = [&](int64_t nb) {
+        int64_t e = 0;
+        for (int64_t b = 0; b < nb; ++b) e = std::max(e, sp[(b + 1) * d.n_slices / nb] - sp[b * d.n_slices / nb]);
+        return e;
+    };
+    if (d.dcol && d.n_slices <= kClusterSlices && cluster_fits()) {
+        const int64_t nb = steps_blocks(d, true), e = most(nb);
+        if (steps_layout(d, nb, e, 0, true, &pl)) *entries = (int32_t)e | kClusterWork;
+    }
+    if (*entries == 0) {
+        const int64_t e = most(grid);
+        if (!steps_layout(d, grid, e, 0, false, &pl)) return 0;
+        *entries = (int32_t)e;
+    }
     return (int64_t)(kHeadBytes + kPartBytes + 2 * (size_t)m->n_pad * sizeof(float4));
 }
