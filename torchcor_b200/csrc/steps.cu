@@ -346,6 +346,7 @@ __global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, cons
     float* zg = d.r;
     float4* q4 = pl.rec[1];        // {b', u, x0, -}; read before the first pass that writes rec[1]
     const int last_step = first_step + pl.n_steps;
+    const double stop_a = d.a_tol > 0.0 ? d.a_tol * d.a_tol : 0.0;
     // (the barriers of a cluster are the hardware's and need no limit)
     auto barrier = [&] {
         if constexpr (CL) {
@@ -438,7 +439,8 @@ __global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, cons
 
         int it = 0;
         Alpha alpha = {0.0f, 0.0f};
-        double b_norm = 0.0;
+        double stop_b = 0.0;   // (r_tol |D b|)^2
+        bool zero_stops = false;
         float beta = 0.0f;
         while (it < d.max_iter) {
             // ---- p, A p; the sums that give alpha, beta and the stopping test
@@ -461,7 +463,8 @@ __global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, cons
                     const float4 f = rin[i];
                     di = f.w;
                     advance(f, alpha, beta, r, z, p);
-                    ap = (float)row_next<8, ASPLIT>(R, rin, gin, base, w, i, alpha, beta);
+                    ap = (float)(w <= 8 ? row_next<8, ASPLIT>(R, rin, gin, base, w, i, alpha, beta)
+                                        : row_next<16, ASPLIT>(R, rin, gin, base, w, i, alpha, beta));
                 }
                 pass_sums(sums, r, p, ap, di);
                 const float4 out = make_float4(r, p, ap, di);
@@ -470,18 +473,22 @@ __global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, cons
             }
             if (!barrier_sums(sums)) return;
             const double rz = sh.total[5];
-            if (it == 0) b_norm = sqrt(sh.total[7]);
-            const double al = rz / sh.total[0];
+            if (it == 0) {
+                stop_b = d.r_tol > 0.0 ? d.r_tol * d.r_tol * sh.total[7] : 0.0;
+                zero_stops = d.a_tol > 0.0 || (d.r_tol > 0.0 && sh.total[7] > 0.0);
+            }
+            const double al = rz / sh.total[0], inv_rz = 1.0 / rz;   // (side by side)
             alpha = split(al);
-            const double zz = sh.total[6] - al * (2.0 * sh.total[3] - al * sh.total[4]);
+            double zz = sh.total[6] - al * (2.0 * sh.total[3] - al * sh.total[4]);
+            if (zz < 0.0) zz = 0.0;
             const double rz1 = rz - al * (2.0 * sh.total[1] - al * sh.total[2]);
             for (int s = warp; s < slices; s += kWarps) {
                 const int i = s * TCB_SLICE + lane;
                 if (i < rows) sx[i] = (float)((double)sx[i] + al * (double)rout[i].y);
             }
-            const double zn = sqrt(zz < 0.0 ? 0.0 : zz);
-            if (zn < d.a_tol || zn < d.r_tol * b_norm) break;   // solver.py:66-69
-            beta = (float)(rz1 / rz);
+            // |z'| below a_tol or r_tol |D b| (solver.py:66-69), squared
+            if (zz < stop_a || zz < stop_b || (zz == 0.0 && zero_stops)) break;
+            beta = (float)(rz1 * inv_rz);
             ++it;
 #pragma unroll
             for (int j = 0; j < kSums; ++j) sums[j] = 0.0;
