@@ -38,6 +38,7 @@ struct CgView {
     const int16_t* dcol;       // int16 column offsets from the row, or null
     const float *mv, *kv, *av, *dinv;
     float *x, *bp, *r, *p, *ap, *z, *p2;
+    float *u, *xprev, *xnext;  // the step's slots of the ring x (set by the kernel in its own copy)
     float cm;
     int32_t linear_guess, a_split, pad;
 };

@@ -20,8 +20,10 @@
 // Stopping test.  A pass's sums tell which simulations it stops (as in the
 // single-simulation kernel); those update x alone, and where none goes on the
 // launch ends without another barrier.  24 cubes of 2.0 M nodes (one or two passes)
-// take 213 us a launch on B200, 245 before this, the unpredicated chunks of 5 and
-// the shorter barrier; 12 cubes and shells of 340,000 nodes 85, 99 before.
+// take 210 us a launch on B200, 245 before this, the unpredicated chunks of 5, the
+// shorter barrier and the views and limits kept in shared memory for the whole launch
+// (a pass read them through two dependent global loads each time); 12 cubes and
+// shells of 340,000 nodes 79, 99 before.
 //
 // Reductions are per simulation and deterministic: each lane accumulates its
 // rows of one simulation in slice order, a warp reduces its lanes with a fixed
@@ -110,11 +112,11 @@ constexpr int kRhsChunk = 5;
 // DC: int16 column offsets; AS: A rebuilt as fp32(fp32(M*Cm) + K'); LG: linear
 // extrapolation guess.  Vectors other than x's next slot are read-only here.
 template <bool DC, bool AS, bool LG>
-__device__ __forceinline__ void rhs_slice(const CgView& d, int step, int64_t ls, int lane, double (&acc)[3]) {
+__device__ __forceinline__ void rhs_slice(const CgView& d, int64_t ls, int lane, double (&acc)[3]) {
     const int64_t row = ls * TCB_SLICE + lane;
     if (row >= d.n) return;
-    const float* __restrict__ u = d.x + ring_cur(step) * d.n_pad;
-    const float* __restrict__ xp = d.x + ring_prev(step) * d.n_pad;
+    const float* __restrict__ u = d.u;
+    const float* __restrict__ xp = d.xprev;
     const float* __restrict__ bp = d.bp;
     const int64_t s0 = __ldg(d.slice_ptr + ls);
     const int w = (int)((__ldg(d.slice_ptr + ls + 1) - s0) / TCB_SLICE);
@@ -162,7 +164,7 @@ __device__ __forceinline__ void rhs_slice(const CgView& d, int step, int64_t ls,
     float xg0;
     if constexpr (LG) xg0 = 2.0f * ui - __ldg(xp + row);
     else xg0 = ui;
-    __stwb(d.x + ring_next(step) * d.n_pad + row, xg0);
+    __stwb(d.xnext + row, xg0);
     const float r32 = (float)((double)rhs - ax);
     const float di = __ldg(d.dinv + row);
     const float z32 = __fmul_rn(di, r32);
@@ -310,11 +312,12 @@ struct ApStreams {
 
 struct BatchShared {
     double *rz, *zz, *bn, *al, *be;   // [n] per simulation
+    double *at, *rt;             // [n] tolerances
     double* wp;                  // [warps][kBatchMaxPerBlock][3] warp partials of the staged simulations
     int64_t* pre;                // [n+1] prefix of the active simulations' slice counts
     int64_t* bb;                 // [nb+1] first virtual slice of each block
     CgView* cg;                  // [kBatchMaxPerBlock] staged views
-    int *it, *act, *step, *ns;   // [n]; act: 0 done, 1 iterating, 2 in its last pass
+    int *it, *act, *step, *ns, *most;   // [n]; act: 0 done, 1 iterating, 2 in its last pass; most: max_iter
     int *w0, *w1;                // [n] first and last block holding each active simulation's slices
 };
 
@@ -325,7 +328,9 @@ __device__ __forceinline__ BatchShared carve(double* smd, int n, int nb) {
     s.bn = s.zz + n;
     s.al = s.bn + n;
     s.be = s.al + n;
-    s.wp = s.be + n;
+    s.at = s.be + n;
+    s.rt = s.at + n;
+    s.wp = s.rt + n;
     s.pre = reinterpret_cast<int64_t*>(s.wp + kCgWarps * kBatchMaxPerBlock * 3);
     s.bb = s.pre + n + 1;
     s.cg = reinterpret_cast<CgView*>(s.bb + nb + 1);
@@ -333,7 +338,8 @@ __device__ __forceinline__ BatchShared carve(double* smd, int n, int nb) {
     s.act = s.it + n;
     s.step = s.act + n;
     s.ns = s.step + n;
-    s.w0 = s.ns + n;
+    s.most = s.ns + n;
+    s.w0 = s.most + n;
     s.w1 = s.w0 + n;
     return s;
 }
@@ -413,12 +419,30 @@ __device__ __forceinline__ void flush(BatchShared& S, int warp, int lane, int j,
     }
 }
 
+// The views of simulations [j0, j1), with their step's slots of the solution ring, into
+// S.cg[0..j1-j0).  Up to kBatchMaxPerBlock simulations are staged once a launch, more
+// by every sweep that walks them.
+__device__ __forceinline__ void stage_views(const BatchWS* W, BatchShared& S, int j0, int j1) {
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(W->cg + j0);
+    uint32_t* dst = reinterpret_cast<uint32_t*>(S.cg);
+    const int words = (j1 - j0) * (int)(sizeof(CgView) / 4);
+    for (int t = threadIdx.x; t < words; t += blockDim.x) dst[t] = src[t];
+    __syncthreads();
+    for (int t = threadIdx.x; t < j1 - j0; t += blockDim.x) {
+        CgView& d = S.cg[t];
+        const int step = S.step[j0 + t];
+        d.u = d.x + ring_cur(step) * d.n_pad;
+        d.xprev = d.x + ring_prev(step) * d.n_pad;
+        d.xnext = d.x + ring_next(step) * d.n_pad;
+    }
+}
+
 // One sweep over this block's share of the active slices: body(i, view, local
 // slice, acc) adds each lane's row into acc; the block's per-simulation sums go
 // to parts[v][i][block].
 template <int NV, class Body>
-__device__ __forceinline__ void sweep(const BatchWS* W, BatchShared& S, double* parts, Body&& body) {
-    const int nb = gridDim.x, b = blockIdx.x, n = W->n;
+__device__ __forceinline__ void sweep(const BatchWS* W, BatchShared& S, int n, double* parts, Body&& body) {
+    const int nb = gridDim.x, b = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t vb = S.bb[b], ve = S.bb[b + 1];
     if (vb >= ve) return;
@@ -426,14 +450,10 @@ __device__ __forceinline__ void sweep(const BatchWS* W, BatchShared& S, double* 
     for (int j0 = first; j0 <= last; j0 += kBatchMaxPerBlock) {
         const int j1 = min(last + 1, j0 + kBatchMaxPerBlock);
         __syncthreads();   // earlier users of the staged views and slots are done
-        {
-            const uint32_t* src = reinterpret_cast<const uint32_t*>(W->cg + j0);
-            uint32_t* dst = reinterpret_cast<uint32_t*>(S.cg);
-            const int words = (j1 - j0) * (int)(sizeof(CgView) / 4);
-            for (int t = threadIdx.x; t < words; t += blockDim.x) dst[t] = src[t];
-            for (int t = threadIdx.x; t < kCgWarps * kBatchMaxPerBlock * 3; t += blockDim.x) S.wp[t] = 0.0;
-        }
+        if (n > kBatchMaxPerBlock) stage_views(W, S, j0, j1);
+        for (int t = threadIdx.x; t < kCgWarps * kBatchMaxPerBlock * 3; t += blockDim.x) S.wp[t] = 0.0;
         __syncthreads();
+        const CgView* views = S.cg + (n > kBatchMaxPerBlock ? -j0 : 0);   // of simulation i at views[i]
         const int64_t sb = max(vb, S.pre[j0]), se = min(ve, S.pre[j1]);
         double acc[NV];
 #pragma unroll
@@ -445,7 +465,7 @@ __device__ __forceinline__ void sweep(const BatchWS* W, BatchShared& S, double* 
                 if (ci >= 0) flush<NV>(S, warp, lane, ci - j0, acc);
                 ci = i;
             }
-            body(i, S.cg[i - j0], vs - S.pre[i], acc);
+            body(i, views[i], vs - S.pre[i], acc);
         }
         if (ci >= 0) flush<NV>(S, warp, lane, ci - j0, acc);
         __syncthreads();
@@ -469,11 +489,11 @@ struct Walk {
     int64_t vs, se, ls, s0;
     int i, w, k0, nk;
     bool ok;
-    __device__ void load(const BatchShared& S, int j0, int stage_bytes) {
+    __device__ void load(const BatchShared& S, const CgView* views, int stage_bytes) {
         ok = vs < se;
         if (!ok) return;
         while (S.pre[i + 1] <= vs) ++i;
-        const CgView& d = S.cg[i - j0];
+        const CgView& d = views[i];
         ls = vs - S.pre[i];
         s0 = __ldg(d.slice_ptr + ls);
         w = (int)((__ldg(d.slice_ptr + ls + 1) - s0) / TCB_SLICE);
@@ -481,11 +501,11 @@ struct Walk {
         nk = fit < kMaxUnitEntries ? fit : kMaxUnitEntries;
         k0 = 0;
     }
-    __device__ void next(const BatchShared& S, int j0, int stage_bytes) {
+    __device__ void next(const BatchShared& S, const CgView* views, int stage_bytes) {
         k0 += nk;
         if (k0 >= w) {
             vs += kCgWarps;
-            load(S, j0, stage_bytes);
+            load(S, views, stage_bytes);
         }
     }
     __device__ int count() const { return nk < w - k0 ? nk : w - k0; }
@@ -510,9 +530,9 @@ __device__ __forceinline__ void issue(Pipe& P, int s, const CgView& d, const Wal
 // finishes a row after its slice's last unit.  Returns false after a timed-out
 // wait (the error word is set; the block returns).
 template <int NV, class Streams, class Unit, class End>
-__device__ __forceinline__ bool sweep_staged(const BatchWS* W, BatchShared& S, double* parts, Pipe& P,
+__device__ __forceinline__ bool sweep_staged(const BatchWS* W, BatchShared& S, int n, double* parts, Pipe& P,
                                              int32_t* err, Unit&& unit, End&& end) {
-    const int nb = gridDim.x, b = blockIdx.x, n = W->n;
+    const int nb = gridDim.x, b = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t vb = S.bb[b], ve = S.bb[b + 1];
     if (vb >= ve) return true;
@@ -521,23 +541,19 @@ __device__ __forceinline__ bool sweep_staged(const BatchWS* W, BatchShared& S, d
     for (int j0 = first; j0 <= last; j0 += kBatchMaxPerBlock) {
         const int j1 = min(last + 1, j0 + kBatchMaxPerBlock);
         __syncthreads();   // earlier users of the staged views and slots are done
-        {
-            const uint32_t* src = reinterpret_cast<const uint32_t*>(W->cg + j0);
-            uint32_t* dst = reinterpret_cast<uint32_t*>(S.cg);
-            const int words = (j1 - j0) * (int)(sizeof(CgView) / 4);
-            for (int t = threadIdx.x; t < words; t += blockDim.x) dst[t] = src[t];
-            for (int t = threadIdx.x; t < kCgWarps * kBatchMaxPerBlock * 3; t += blockDim.x) S.wp[t] = 0.0;
-        }
+        if (n > kBatchMaxPerBlock) stage_views(W, S, j0, j1);
+        for (int t = threadIdx.x; t < kCgWarps * kBatchMaxPerBlock * 3; t += blockDim.x) S.wp[t] = 0.0;
         __syncthreads();
+        const CgView* views = S.cg + (n > kBatchMaxPerBlock ? -j0 : 0);   // of simulation i at views[i]
         Walk<Streams> cons;
         cons.vs = max(vb, S.pre[j0]) + warp;
         cons.se = min(ve, S.pre[j1]);
         cons.i = j0;
-        cons.load(S, j0, P.stage_bytes);
+        cons.load(S, views, P.stage_bytes);
         Walk<Streams> prod = cons;
         for (int st = 0; st < kStages && prod.ok; ++st) {
-            issue(P, st, S.cg[prod.i - j0], prod, lane);
-            prod.next(S, j0, P.stage_bytes);
+            issue(P, st, views[prod.i], prod, lane);
+            prod.next(S, views, P.stage_bytes);
         }
         double acc[NV];
 #pragma unroll
@@ -553,7 +569,7 @@ __device__ __forceinline__ bool sweep_staged(const BatchWS* W, BatchShared& S, d
             }
             P.inflight &= ~(1u << st);
             P.phase ^= 1u << st;
-            const CgView& d = S.cg[cons.i - j0];
+            const CgView& d = views[cons.i];
             if (cons.i != ci) {
                 if (ci >= 0) flush<NV>(S, warp, lane, ci - j0, acc);
                 ci = cons.i;
@@ -564,10 +580,10 @@ __device__ __forceinline__ bool sweep_staged(const BatchWS* W, BatchShared& S, d
             if (cons.k0 + cnt >= cons.w) end(cons.i, d, cons.ls, rw, acc);
             __syncwarp();   // every lane is done with this stage's buffer
             if (prod.ok) {
-                issue(P, st, S.cg[prod.i - j0], prod, lane);
-                prod.next(S, j0, P.stage_bytes);
+                issue(P, st, views[prod.i], prod, lane);
+                prod.next(S, views, P.stage_bytes);
             }
-            cons.next(S, j0, P.stage_bytes);
+            cons.next(S, views, P.stage_bytes);
         }
         if (ci >= 0) flush<NV>(S, warp, lane, ci - j0, acc);
         __syncthreads();
@@ -588,13 +604,13 @@ __device__ __forceinline__ bool sweep_staged(const BatchWS* W, BatchShared& S, d
 // one staged unit of the right-hand side (entries in slice order, the same
 // float64 accumulation sequence as rhs_slice)
 template <bool DC, bool AS, bool LG>
-__device__ __forceinline__ void rhs_unit(const CgView& d, int step, int64_t ls, int nk, const unsigned char* buf,
+__device__ __forceinline__ void rhs_unit(const CgView& d, int64_t ls, int nk, const unsigned char* buf,
                                          Row& rw, int lane) {
     const int64_t row = ls * TCB_SLICE + lane;
     if (row >= d.n) return;
     const int r = (int)row;
-    const float* __restrict__ u = d.x + ring_cur(step) * d.n_pad;
-    const float* __restrict__ xp = d.x + ring_prev(step) * d.n_pad;
+    const float* __restrict__ u = d.u;
+    const float* __restrict__ xp = d.xprev;
     const float* __restrict__ bp = d.bp;
     const int m = nk * TCB_SLICE;
     const int16_t* c16 = reinterpret_cast<const int16_t*>(buf);
@@ -642,15 +658,15 @@ __device__ __forceinline__ void rhs_unit(const CgView& d, int step, int64_t ls, 
 }
 
 // the end of a right-hand-side row (as the tail of rhs_slice)
-__device__ __forceinline__ void rhs_end(const CgView& d, int step, int64_t ls, const Row& rw, double (&acc)[3],
+__device__ __forceinline__ void rhs_end(const CgView& d, int64_t ls, const Row& rw, double (&acc)[3],
                                         int lane) {
     const int64_t row = ls * TCB_SLICE + lane;
     if (row >= d.n) return;
-    const float* __restrict__ u = d.x + ring_cur(step) * d.n_pad;
+    const float* __restrict__ u = d.u;
     const float rhs = (float)rw.v[0] - (float)rw.v[1];   // float32 sums carried in the row state
     const float ui = __ldg(u + row);
-    const float xg0 = d.linear_guess ? 2.0f * ui - __ldg(d.x + ring_prev(step) * d.n_pad + row) : ui;
-    __stwb(d.x + ring_next(step) * d.n_pad + row, xg0);
+    const float xg0 = d.linear_guess ? 2.0f * ui - __ldg(d.xprev + row) : ui;
+    __stwb(d.xnext + row, xg0);
     const float r32 = (float)((double)rhs - rw.v[2]);
     const float di = __ldg(d.dinv + row);
     const float z32 = __fmul_rn(di, r32);
@@ -708,8 +724,8 @@ __device__ __forceinline__ void ap_end(const CgView& d, const float* pin, float*
 
 // every block: totals of every active simulation (warp per simulation, lanes over its blocks)
 template <int NV, class F>
-__device__ __forceinline__ void totals(const BatchWS* W, BatchShared& S, const double* parts, F&& consume) {
-    const int nb = gridDim.x, n = W->n;
+__device__ __forceinline__ void totals(BatchShared& S, int n, const double* parts, F&& consume) {
+    const int nb = gridDim.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int i = warp; i < n; i += kCgWarps) {
         const int b0 = S.w0[i], b1 = S.w1[i];
@@ -731,7 +747,7 @@ __device__ __forceinline__ void totals(const BatchWS* W, BatchShared& S, const d
 
 // bytes of the shared carve-out before the staging area (128-byte aligned)
 __host__ __device__ inline size_t carve_bytes(int n) {
-    const size_t b = (size_t)n * (5 * sizeof(double) + 6 * sizeof(int)) +
+    const size_t b = (size_t)n * (7 * sizeof(double) + 7 * sizeof(int)) +
                      sizeof(double) * kCgWarps * kBatchMaxPerBlock * 3 + sizeof(int64_t) * (n + 1) +
                      sizeof(int64_t) * (kBatchMaxBlocks + 1) + sizeof(CgView) * kBatchMaxPerBlock;
     return (b + 127) / 128 * 128;
@@ -775,47 +791,51 @@ __global__ void __launch_bounds__(kCgThreads, PER_SM) batch_cg_kernel(const Batc
     }
 
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const int64_t st = W->dev[i].counter[0];
-        S.step[i] = (st >= 1 && st <= W->dev[i].nt) ? (int)st : 0;   // 0 = not stepping
+        const MonoDev& d = W->dev[i];
+        const int64_t st = d.counter[0];
+        S.step[i] = (st >= 1 && st <= d.nt) ? (int)st : 0;   // 0 = not stepping
+        S.at[i] = d.a_tol;
+        S.rt[i] = d.r_tol;
+        S.most[i] = d.max_iter;
         S.ns[i] = W->slices[i];
         S.act[i] = 0;
         S.it[i] = 0;
     }
     __syncthreads();
 
+    if (n <= kBatchMaxPerBlock) stage_views(W, S, 0, n);
+
     // ---- right-hand side, guess, r0, z0 (solver.py:46-55; monodomain.py:130-131)
     int64_t A = active_prefix(S, n, S.step);
     if constexpr (STAGED) {
         const bool ok = sweep_staged<3, RhsStreams>(
-            W, S, parts0, P, err,
+            W, S, n, parts0, P, err,
             [&](int i, const CgView& d, int64_t ls, int nk, const unsigned char* buf, Row& rw) {
-                const int step = S.step[i];
                 with_flags<FLAGS>(d, [&](auto fl) {
                     constexpr int F = decltype(fl)::value;
-                    rhs_unit<(F & 4) != 0, (F & 2) != 0, (F & 1) != 0>(d, step, ls, nk, buf, rw, lane);
+                    rhs_unit<(F & 4) != 0, (F & 2) != 0, (F & 1) != 0>(d, ls, nk, buf, rw, lane);
                 });
             },
             [&](int i, const CgView& d, int64_t ls, const Row& rw, double (&acc)[3]) {
-                rhs_end(d, S.step[i], ls, rw, acc, lane);
+                rhs_end(d, ls, rw, acc, lane);
             });
         // a copy that did not come in time: the error word is set, and a block missing at the
         // barrier makes the others look at it
         if (__syncthreads_or(!ok)) return;
     } else
-    sweep<3>(W, S, parts0, [&](int i, const CgView& d, int64_t ls, double (&acc)[3]) {
-        const int step = S.step[i];
+    sweep<3>(W, S, n, parts0, [&](int i, const CgView& d, int64_t ls, double (&acc)[3]) {
         with_flags<FLAGS>(d, [&](auto fl) {
             constexpr int F = decltype(fl)::value;
-            rhs_slice<(F & 4) != 0, (F & 2) != 0, (F & 1) != 0>(d, step, ls, lane, acc);
+            rhs_slice<(F & 4) != 0, (F & 2) != 0, (F & 1) != 0>(d, ls, lane, acc);
         });
     });
     if (!grid_barrier(gw)) return;
-    totals<3>(W, S, parts0, [&](int i, double* t) {
+    totals<3>(S, n, parts0, [&](int i, double* t) {
         S.bn[i] = sqrt(t[0]);
         S.rz[i] = t[1];
         S.zz[i] = t[2];
         S.be[i] = 0.0;
-        S.act[i] = W->dev[i].max_iter > 0;
+        S.act[i] = S.most[i] > 0;
     });
 
     for (int pass = 0;; ++pass) {
@@ -825,7 +845,7 @@ __global__ void __launch_bounds__(kCgThreads, PER_SM) batch_cg_kernel(const Batc
         // ---- p = z + beta p (on the fly), Ap, p.Ap
         if constexpr (STAGED) {
             const bool ok = sweep_staged<3, ApStreams>(
-                W, S, parts1, P, err,
+                W, S, n, parts1, P, err,
                 [&](int i, const CgView& d, int64_t ls, int nk, const unsigned char* buf, Row& rw) {
                     const float* pin = (pass & 1) ? d.p2 : d.p;
                     const float beta = (float)S.be[i];
@@ -841,7 +861,7 @@ __global__ void __launch_bounds__(kCgThreads, PER_SM) batch_cg_kernel(const Batc
                 });
             if (__syncthreads_or(!ok)) return;
         } else
-        sweep<3>(W, S, parts1, [&](int i, const CgView& d, int64_t ls, double (&acc)[3]) {
+        sweep<3>(W, S, n, parts1, [&](int i, const CgView& d, int64_t ls, double (&acc)[3]) {
             const float* pin = (pass & 1) ? d.p2 : d.p;
             float* pout = (pass & 1) ? d.p : d.p2;
             const float beta = (float)S.be[i];
@@ -854,22 +874,21 @@ __global__ void __launch_bounds__(kCgThreads, PER_SM) batch_cg_kernel(const Batc
         if (!grid_barrier(gw)) return;
         // alpha, and |z'|^2 of z' = z - alpha w from the same sums: a simulation that this
         // stops (solver.py:66-69) has only x left to update
-        totals<3>(W, S, parts1, [&](int i, double* t) {
+        totals<3>(S, n, parts1, [&](int i, double* t) {
             const double alpha = S.rz[i] / t[0];
             const double zz1 = S.zz[i] - alpha * (2.0 * t[1] - alpha * t[2]);
             const double zn = sqrt(zz1 < 0.0 ? 0.0 : zz1);
-            const MonoDev& d = W->dev[i];
             S.al[i] = alpha;
-            if (zn < d.a_tol || zn < d.r_tol * S.bn[i]) S.act[i] = 2;
+            if (zn < S.at[i] || zn < S.rt[i] * S.bn[i]) S.act[i] = 2;
         });
 
         // ---- x += alpha p, r -= alpha Ap, z = D r; r.z, z.z
-        sweep<2>(W, S, parts0, [&](int i, const CgView& d, int64_t ls, double (&acc)[2]) {
+        sweep<2>(W, S, n, parts0, [&](int i, const CgView& d, int64_t ls, double (&acc)[2]) {
             const int64_t row = ls * TCB_SLICE + lane;
             if (row >= d.n) return;
             const float* pnew = (pass & 1) ? d.p : d.p2;
             const double alpha = S.al[i];
-            float* x = d.x + ring_next(S.step[i]) * d.n_pad;
+            float* x = d.xnext;
             __stwb(x + row, (float)((double)__ldca(x + row) + alpha * (double)__ldca(pnew + row)));
             if (S.act[i] == 2) return;
             const float r32 = (float)((double)__ldca(d.r + row) - alpha * (double)__ldca(d.ap + row));
@@ -885,7 +904,7 @@ __global__ void __launch_bounds__(kCgThreads, PER_SM) batch_cg_kernel(const Batc
         for (int i = threadIdx.x; i < n; i += blockDim.x) more |= S.act[i] == 1;
         if (!__syncthreads_or(more)) break;
         if (!grid_barrier(gw)) return;
-        totals<2>(W, S, parts0, [&](int i, double* t) {
+        totals<2>(S, n, parts0, [&](int i, double* t) {
             if (S.act[i] != 1) {
                 S.act[i] = 0;
                 return;
@@ -894,7 +913,7 @@ __global__ void __launch_bounds__(kCgThreads, PER_SM) batch_cg_kernel(const Batc
             S.rz[i] = t[0];
             S.zz[i] = t[1];
             S.it[i] += 1;
-            if (S.it[i] >= W->dev[i].max_iter) S.act[i] = 0;
+            if (S.it[i] >= S.most[i]) S.act[i] = 0;
         });
     }
     // block 0 records the iterations and advances the step counters (every
