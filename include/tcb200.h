@@ -80,7 +80,8 @@ int tcb_sell_layout_device(const int32_t* rowptr, int64_t n_rows, int64_t* slice
  * parse exactly are counted in *bad (device int64, caller-zeroed).
  * Pattern: tcb_pattern_device with work = 2*(N+1) int64, keys = k*k*E uint64,
  * iwork = 2*N+1 int32 returns nnz; tcb_pattern_device_emit writes the same arrays
- * as tcb_pattern_build (device pointers). */
+ * as tcb_pattern_build (device pointers).  slot_src may be the first k*k*E int32 of
+ * keys, where the first call leaves it: nothing is copied then. */
 int64_t tcb_text_scratch(int64_t n_bytes);
 int tcb_text_newlines(const char* text, int64_t n_bytes, int64_t* scratch, int64_t* pos, int64_t cap, int64_t* count,
                       void* stream);

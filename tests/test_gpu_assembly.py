@@ -46,6 +46,27 @@ def test_rows_of_every_sort(lib, cuda, k, degrees):
     _equal(el, n, cuda)
 
 
+@pytest.mark.parametrize("k,shift,inplace", [(4, 0, False), (4, 1, False), (4, 1, True), (3, 1, False)])
+def test_contributions_beside_and_inside_the_keys(lib, cuda, k, shift, inplace):
+    """slot_src in the keys' own buffer or in another; a buffer aligned to 8 bytes only
+    takes single stores instead of 16-byte ones."""
+    from torchcor_b200._lib import check, ptr, stream_ptr
+    from torchcor_b200.core.assemble import build_pattern
+    el, n = _fans(k, [1, 5, 8, 16, 17, 32, 33, 64, 65, 200], np.random.default_rng(7 + k))
+    E, h, d = len(el), build_pattern(el, n), torch.from_numpy(el).to(cuda)
+    work = torch.empty(2 * (n + 1), device=cuda, dtype=torch.int64)
+    keys = torch.empty(k * k * E + shift, device=cuda, dtype=torch.int64)[shift:]
+    iwork = torch.empty(2 * n + 1, device=cuda, dtype=torch.int32)
+    nnz = C.c_int64()
+    check(lib.tcb_pattern_device(ptr(d), E, k, n, ptr(work), ptr(keys), ptr(iwork), C.byref(nnz), stream_ptr()))
+    i32 = dict(device=cuda, dtype=torch.int32)
+    src = keys.view(torch.int32)[:k * k * E] if inplace else torch.empty(k * k * E, **i32)
+    got = [torch.empty(n + 1, **i32), torch.empty(nnz.value, **i32), torch.empty(nnz.value + 1, **i32), src, torch.empty(n, **i32)]
+    check(lib.tcb_pattern_device_emit(ptr(work), ptr(keys), E, k, n, *(ptr(t) for t in got), stream_ptr()))
+    for name, t in zip(NAMES, got):
+        assert np.array_equal(t.cpu().numpy(), h.host(name)), name
+
+
 def test_far_columns_and_multi_block_scans(lib, cuda):
     """A strip of triangles over 4.3 million nodes, some joined to nodes millions of
     rows away: beyond the 22- and 23-bit column offsets of the register sorts."""

@@ -95,7 +95,7 @@ def build_pattern_device(elems: torch.Tensor, n_nodes: int) -> Pattern:
     check(lib.tcb_pattern_device(ptr(el), E, k, n_nodes, ptr(work), ptr(keys), ptr(iwork), C.byref(nnz), s))
     i32 = dict(device=dev, dtype=torch.int32)
     rowptr, col = torch.empty(n_nodes + 1, **i32), torch.empty(nnz.value, **i32)
-    slot_ptr, slot_src = torch.empty(nnz.value + 1, **i32), torch.empty(k * k * E, **i32)
+    slot_ptr, slot_src = torch.empty(nnz.value + 1, **i32), keys.view(torch.int32)[:k * k * E]   # where the sort left it
     diag = torch.empty(n_nodes, **i32)
     check(lib.tcb_pattern_device_emit(ptr(work), ptr(keys), E, k, n_nodes, ptr(rowptr), ptr(col), ptr(slot_ptr),
                                       ptr(slot_src), ptr(diag), s))

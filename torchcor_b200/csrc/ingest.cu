@@ -362,48 +362,78 @@ __global__ void pattern_count_kernel(const int32_t* __restrict__ el, int64_t E, 
     }
 }
 
-// e*k + a of every element corner, in its node's segment (any order; the segment
-// has room for k entries a corner, the first ones are used)
+// The two halves of the 64-bit keys' buffer, row_off + i a row's i-th word in each: `src` gets the
+// contributions in their final order (flat element-matrix indices e*k*k + a*k + b), so
+// that the emit kernel need not read them again; `list` holds the row's element corners
+// (e*k + a, any order) until the sort, then its distinct columns.
+struct KeyHalves {
+    uint32_t* src;
+    uint32_t* list;
+};
+
+inline KeyHalves key_halves(uint64_t* keys, int64_t E, int k) {
+    uint32_t* p = reinterpret_cast<uint32_t*>(keys);
+    return {p, p + (int64_t)k * k * E};
+}
+
 __global__ void pattern_fill_kernel(const int32_t* __restrict__ el, int64_t E, int k, int64_t N, const int64_t* __restrict__ row_off,
-                                    int32_t* __restrict__ fill, uint64_t* __restrict__ keys) {
+                                    int32_t* __restrict__ fill, uint32_t* __restrict__ list) {
     const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= E) return;
     for (int a = 0; a < k; ++a) {
         const int32_t row = el[e * k + a];
         if (row < 0 || row >= N) return;   // recorded by the count
-        keys[row_off[row] + atomicAdd(fill + row, 1)] = (uint64_t)(e * k + a);
+        list[row_off[row] + atomicAdd(fill + row, 1)] = (uint32_t)(e * k + a);
     }
 }
 
-// A row's contributions as the emit kernel reads them: column in the high half, the
-// flat element-matrix index e*k*k + a*k + b in the low half, its top bit set at
-// the first contribution of a column.
-constexpr uint64_t kFirstOfColumn = 0x80000000ull;
+// A distinct column in `list`: its distance from the row (23 bits) above its first contribution's
+// place in the row (8 bits).  Rows of the shared-memory sort have the column itself with the top
+// bit set, and the top bit of `src` at the first contribution of a column.
+constexpr int kStartBits = 8;
+constexpr int32_t kFar = 1 << 22;
+constexpr uint32_t kRestRow = 0x80000000u, kFirstOfColumn = 0x80000000u;
 
-// ascending bitonic sort of 32*R keys in registers, key r of a lane at lane*R + r
+// Ascending bitonic sort of 32*R keys in registers, key r of a lane at lane*R + r.  A merge starts by
+// comparing mirrored places, so every exchange goes the same way: the lower place keeps the smaller key.
 template <int R>
 __device__ __forceinline__ void warp_sort(uint32_t (&key)[R]) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int size = 2; size <= 32 * R; size <<= 1) {
+        if (size <= R) {
 #pragma unroll
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            for (int r = 0; r < R; ++r) {
+                const int q = r ^ (size - 1);
+                if (q < r) continue;
+                const uint32_t x = key[r], y = key[q];
+                key[r] = min(x, y);
+                key[q] = max(x, y);
+            }
+        } else {
+            const bool lower = (lane & (size / R / 2)) == 0;
+            uint32_t o[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) o[r] = __shfl_xor_sync(0xffffffffu, key[R - 1 - r], size / R - 1);
+#pragma unroll
+            for (int r = 0; r < R; ++r) key[r] = lower ? min(key[r], o[r]) : max(key[r], o[r]);
+        }
+#pragma unroll
+        for (int stride = size >> 2; stride > 0; stride >>= 1) {
             if (stride >= R) {
                 const bool lower = (lane & (stride / R)) == 0;
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
-                    const bool up = ((lane * R + r) & size) == 0;
                     const uint32_t o = __shfl_xor_sync(0xffffffffu, key[r], stride / R);
-                    key[r] = lower == up ? min(key[r], o) : max(key[r], o);
+                    key[r] = lower ? min(key[r], o) : max(key[r], o);
                 }
             } else {
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
                     if (r & stride) continue;
-                    const bool up = ((lane * R + r) & size) == 0;
                     const uint32_t x = key[r], y = key[r | stride];
-                    key[r] = up ? min(x, y) : max(x, y);
-                    key[r | stride] = up ? max(x, y) : min(x, y);
+                    key[r] = min(x, y);
+                    key[r | stride] = max(x, y);
                 }
             }
         }
@@ -416,16 +446,17 @@ __device__ __forceinline__ void warp_sort(uint32_t (&key)[R]) {
 // A = corners a lane.  false (nothing written) if a column is too far from the row for
 // the key's 23 (A = 1) or 22 bits.
 template <int R, int A, int K>
-__device__ __forceinline__ bool sort_row(const int32_t* __restrict__ el, int64_t row, int deg, uint64_t* __restrict__ seg,
-                                         int32_t* uniq) {
+__device__ __forceinline__ bool sort_row(const int32_t* __restrict__ el, int64_t row, int deg, uint32_t* __restrict__ src,
+                                         uint32_t* __restrict__ list, int32_t* uniq) {
     constexpr uint32_t k = K;
     constexpr int kRankBits = A == 1 ? 5 : 6, kLow = 4 + kRankBits;
     constexpr int kHalf = 1 << (31 - kLow);   // |column - row| below this
+    static_assert(kHalf <= kFar && 32 * R <= 1 << kStartBits, "columns of the list");
     const int lane = threadIdx.x & 31;
     const int cnt = deg * K;
     uint32_t corner[A];
 #pragma unroll
-    for (int r = 0; r < A; ++r) corner[r] = lane * A + r < deg ? (uint32_t)seg[lane * A + r] : 0xffffffffu;
+    for (int r = 0; r < A; ++r) corner[r] = lane * A + r < deg ? list[lane * A + r] : 0xffffffffu;
     warp_sort<A>(corner);
     uint32_t key[R];
     bool ok = true;
@@ -447,7 +478,9 @@ __device__ __forceinline__ bool sort_row(const int32_t* __restrict__ el, int64_t
     }
     if (!__all_sync(0xffffffffu, ok)) return false;
     warp_sort<R>(key);
-    uint32_t before = __shfl_up_sync(0xffffffffu, key[R - 1], 1);
+    const uint32_t last = __shfl_up_sync(0xffffffffu, key[R - 1], 1);
+    uint32_t out[R];
+    bool first[R];
     int u = 0;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -458,44 +491,62 @@ __device__ __forceinline__ bool sort_row(const int32_t* __restrict__ el, int64_t
             const uint32_t c1 = __shfl_sync(0xffffffffu, corner[1], j / A);
             if (j & 1) c = c1;
         }
-        if (p < cnt) {
-            const bool first = p == 0 || (key[r] >> kLow) != (before >> kLow);
-            u += first;
-            const uint32_t col = (uint32_t)(row + (int64_t)(key[r] >> kLow) - kHalf);
-            seg[p] = ((uint64_t)col << 32) | (first ? kFirstOfColumn : 0ull) | (uint64_t)((c / k) * (k * k) + ab);
-        }
-        before = key[r];
+        out[r] = (c / k) * (k * k) + ab;
+        first[r] = p < cnt && (p == 0 || (key[r] >> kLow) != ((r ? key[r - 1] : last) >> kLow));
+        u += first[r];
     }
+    // (a tetrahedron's four contributions keep the places of a row in multiples of four)
+    constexpr int V = K == 4 ? (R < 4 ? R : 4) : 1;
+    if (V > 1 && (reinterpret_cast<uintptr_t>(src) & (4 * V - 1)) == 0) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) u += __shfl_xor_sync(0xffffffffu, u, o);
-    if (lane == 0) *uniq = u;
+        for (int r = 0; r < R; r += V) {
+            if (lane * R + r >= cnt) break;
+            if constexpr (V == 4) *reinterpret_cast<uint4*>(src + lane * R + r) = make_uint4(out[r], out[r + 1], out[r + 2], out[r + 3]);
+            if constexpr (V == 2) *reinterpret_cast<uint2*>(src + lane * R + r) = make_uint2(out[r], out[r + 1]);
+        }
+    } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (lane * R + r < cnt) src[lane * R + r] = out[r];
+    }
+    int at = u;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) at += v;
+    }
+    if (lane == 31) *uniq = at;
+    at -= u;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        if (first[r]) list[at++] = (((key[r] >> kLow) + (kFar - kHalf)) << kStartBits) | (uint32_t)(lane * R + r);
     return true;
 }
 
 // Rows of up to 64 corners whose columns are near enough (all rows of meshes below two
 // million nodes), one warp each; the others go to `rest` (rest[0] counts).  Bound by
-// integer issue: 28 exchange steps of 128 keys in registers (one 32-bit shuffle and one
-// minimum a key) where the 64-bit keys took as many round trips through shared memory.
+// the exchanges: 28 steps of 128 keys in registers, one 32-bit shuffle and one minimum a key.
+// 531,441 nodes, 50 M contributions: 482 -> 378 us with exchanges that all go one way
+// (no select of a direction) and 4 bytes a contribution written in 16-byte stores.
 template <int K>
 __global__ void __launch_bounds__(256) pattern_sort_kernel(const int32_t* __restrict__ el, const int64_t* __restrict__ row_off, int64_t N,
-                                                           uint64_t* __restrict__ keys, int32_t* __restrict__ uniq,
-                                                           int64_t* __restrict__ rest) {
+                                                           KeyHalves keys, int32_t* __restrict__ uniq, int64_t* __restrict__ rest) {
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= N) return;
     const int64_t b = row_off[row];
     const int cnt = (int)(row_off[row + 1] - b), deg = cnt / K;
     bool done = false;
-    if (cnt <= 32) done = sort_row<1, 1, K>(el, row, deg, keys + b, uniq + row);
-    else if (cnt <= 64) done = sort_row<2, 1, K>(el, row, deg, keys + b, uniq + row);
-    else if (deg <= 32) done = sort_row<4, 1, K>(el, row, deg, keys + b, uniq + row);
-    else if (deg <= 64) done = sort_row<8, 2, K>(el, row, deg, keys + b, uniq + row);
+    if (cnt <= 32) done = sort_row<1, 1, K>(el, row, deg, keys.src + b, keys.list + b, uniq + row);
+    else if (cnt <= 64) done = sort_row<2, 1, K>(el, row, deg, keys.src + b, keys.list + b, uniq + row);
+    else if (deg <= 32) done = sort_row<4, 1, K>(el, row, deg, keys.src + b, keys.list + b, uniq + row);
+    else if (deg <= 64) done = sort_row<8, 2, K>(el, row, deg, keys.src + b, keys.list + b, uniq + row);
     if (!done && (threadIdx.x & 31) == 0)
         rest[1 + atomicAdd(reinterpret_cast<unsigned long long*>(rest), 1ull)] = row;
 }
 
 // The remaining rows: 64-bit keys (column, COO order) sorted in shared memory, one warp a row
 __global__ void pattern_rest_kernel(const int32_t* __restrict__ el, int64_t E, int k, const int64_t* __restrict__ row_off,
-                                    uint64_t* __restrict__ keys, int32_t* __restrict__ uniq, const int64_t* __restrict__ rest,
+                                    KeyHalves keys, int32_t* __restrict__ uniq, const int64_t* __restrict__ rest,
                                     int32_t* __restrict__ err) {
     __shared__ uint64_t sh[kSortWarps][kRowCap];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -517,7 +568,7 @@ __global__ void pattern_rest_kernel(const int32_t* __restrict__ el, int64_t E, i
         for (int i = lane; i < p2; i += 32) {
             uint64_t v = ~0ull;
             if (i < cnt) {
-                const int64_t corner = (int64_t)keys[b + i / k], e = corner / k, a = corner - e * k, c = i % k;
+                const int64_t corner = keys.list[b + i / k], e = corner / k, a = corner - e * k, c = i % k;
                 v = ((uint64_t)(uint32_t)el[e * k + c] << 32) | ((uint64_t)(a * k + c) * (uint64_t)E + (uint64_t)e);
             }
             s[i] = v;
@@ -539,54 +590,61 @@ __global__ void pattern_rest_kernel(const int32_t* __restrict__ el, int64_t E, i
                 __syncwarp();
             }
         int u = 0;
-        for (int i = lane; i < cnt; i += 32) {
-            const bool first = i == 0 || (s[i] >> 32) != (s[i - 1] >> 32);
-            const uint64_t order = s[i] & 0xffffffffull, ab = order / (uint64_t)E, e = order - ab * (uint64_t)E;
-            keys[b + i] = (s[i] & 0xffffffff00000000ull) | (first ? kFirstOfColumn : 0ull) | (e * k * k + ab);
-            u += first;
+        for (int i0 = 0; i0 < cnt; i0 += 32) {
+            const int i = i0 + lane;
+            const uint64_t v = i < cnt ? s[i] : 0ull;
+            const bool first = i < cnt && (i == 0 || (v >> 32) != (s[i - 1] >> 32));
+            const unsigned m = __ballot_sync(0xffffffffu, first);
+            const uint64_t order = v & 0xffffffffull, ab = order / (uint64_t)E, e = order - ab * (uint64_t)E;
+            if (i < cnt) keys.src[b + i] = (first ? kFirstOfColumn : 0u) | (uint32_t)(e * k * k + ab);
+            if (first) keys.list[b + u + __popc(m & ((1u << lane) - 1))] = kRestRow | (uint32_t)(v >> 32);
+            u += __popc(m);
         }
-        for (int o = 16; o > 0; o >>= 1) u += __shfl_xor_sync(0xffffffffu, u, o);
         if (lane == 0) uniq[row] = u;
         __syncwarp();
     }
 }
 
-// one warp per row: CSR columns, slot boundaries, contributions and the diagonal slot
+// CSR columns, slot boundaries and the diagonal slot, half a warp a row (a cube's interior rows have
+// 15 columns): it reads the 15, not the 96 contributions, which are in place (531,441 nodes: 145 -> 55 us).
+// `src` is rewritten only in rows that the shared-memory sort left flagged.
 __global__ void __launch_bounds__(256) pattern_emit_kernel(const int64_t* __restrict__ row_off, const int64_t* __restrict__ rowptr64,
-                                                           int64_t N, const uint64_t* __restrict__ keys,
+                                                           int64_t N, const uint32_t* __restrict__ list,
                                                            int32_t* __restrict__ rowptr, int32_t* __restrict__ col,
-                                                           int32_t* __restrict__ slot_ptr, int32_t* __restrict__ slot_src,
+                                                           int32_t* __restrict__ slot_ptr, int32_t* __restrict__ src,
                                                            int32_t* __restrict__ diag) {
-    const int lane = threadIdx.x & 31;
-    const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 15;
+    const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 4) + (threadIdx.x >> 4);
     if (row >= N) return;
-    const int64_t b = row_off[row];
-    const int cnt = (int)(row_off[row + 1] - b);
-    int64_t w = rowptr64[row];
+    const int64_t b = row_off[row], w = rowptr64[row];
+    const int u = (int)(rowptr64[row + 1] - w);
     if (lane == 0) rowptr[row] = (int32_t)w;
-    constexpr int U = 4;   // rounds in flight (a cube's interior rows have three)
-    for (int i0 = 0; i0 < cnt; i0 += 32 * U) {
-        uint64_t key[U];
-#pragma unroll
-        for (int r = 0; r < U; ++r) {
-            const int i = i0 + 32 * r + lane;
-            key[r] = i < cnt ? keys[b + i] : 0ull;
+    bool flagged = false;
+    for (int i = lane; i < u; i += 16) {
+        const uint32_t v = list[b + i];
+        flagged = (v & kRestRow) != 0;
+        int32_t c = (int32_t)(v & ~kRestRow);
+        if (!flagged) {
+            c = (int32_t)row + (int32_t)(v >> kStartBits) - kFar;
+            slot_ptr[w + i] = (int32_t)(b + (v & ((1u << kStartBits) - 1)));
         }
-#pragma unroll
-        for (int r = 0; r < U; ++r) {
-            const int i = i0 + 32 * r + lane;
-            const bool first = (key[r] & kFirstOfColumn) != 0;
-            const unsigned m = __ballot_sync(0xffffffffu, first);
-            if (i < cnt) slot_src[b + i] = (int32_t)(key[r] & 0x7fffffffull);
-            if (first) {
-                const int64_t j = w + __popc(m & ((1u << lane) - 1));
-                const int32_t c = (int32_t)(key[r] >> 32);
-                col[j] = c;
-                slot_ptr[j] = (int32_t)(b + i);
-                if (c == row) diag[row] = (int32_t)j;
-            }
-            w += __popc(m);
+        col[w + i] = c;
+        if (c == row) diag[row] = (int32_t)(w + i);
+    }
+    const unsigned half = 0xffffu << (threadIdx.x & 16);
+    if (!__any_sync(half, flagged)) return;
+    const int64_t end = row_off[row + 1];
+    int64_t j = w;
+    for (int64_t q0 = b; q0 < end; q0 += 16) {
+        const int64_t q = q0 + lane;
+        const uint32_t v = q < end ? (uint32_t)src[q] : 0u;
+        const bool first = (v & kFirstOfColumn) != 0;
+        const unsigned m = __ballot_sync(half, first) >> (threadIdx.x & 16);
+        if (first) {
+            slot_ptr[j + __popc(m & ((1u << lane) - 1))] = (int32_t)q;
+            src[q] = (int32_t)(v & ~kFirstOfColumn);
         }
+        j += __popc(m);
     }
 }
 
@@ -674,13 +732,14 @@ extern "C" int tcb_pattern_device(const int32_t* elems, int64_t E, int32_t k, in
     if (st) return st;
     TCB_CHECK_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int32_t) * N, s));
     TCB_CHECK_CUDA(cudaMemsetAsync(rowptr64, 0, sizeof(int64_t), s));
-    pattern_fill_kernel<<<blocks(E, kThreads), kThreads, 0, s>>>(elems, E, k, N, row_off, cnt, keys);
+    const KeyHalves halves = key_halves(keys, E, k);
+    pattern_fill_kernel<<<blocks(E, kThreads), kThreads, 0, s>>>(elems, E, k, N, row_off, cnt, halves.list);
     TCB_CHECK_LAUNCH("pattern fill kernel");
-    if (k == 4) pattern_sort_kernel<4><<<blocks(N, 8), 256, 0, s>>>(elems, row_off, N, keys, uniq, rowptr64);
-    else pattern_sort_kernel<3><<<blocks(N, 8), 256, 0, s>>>(elems, row_off, N, keys, uniq, rowptr64);
+    if (k == 4) pattern_sort_kernel<4><<<blocks(N, 8), 256, 0, s>>>(elems, row_off, N, halves, uniq, rowptr64);
+    else pattern_sort_kernel<3><<<blocks(N, 8), 256, 0, s>>>(elems, row_off, N, halves, uniq, rowptr64);
     TCB_CHECK_LAUNCH("pattern sort kernel");
     pattern_rest_kernel<<<(unsigned)std::min<int64_t>(blocks(N, kSortWarps), 592), kSortWarps * 32, 0, s>>>(
-        elems, E, k, row_off, keys, uniq, rowptr64, err);
+        elems, E, k, row_off, halves, uniq, rowptr64, err);
     TCB_CHECK_LAUNCH("pattern rest kernel");
     // (the tile sums of this scan go where the corner counts were: 8-byte aligned, read no more)
     int64_t* tmp = reinterpret_cast<int64_t*>(((uintptr_t)cnt + 7) & ~(uintptr_t)7);
@@ -705,7 +764,10 @@ extern "C" int tcb_pattern_device_emit(const int64_t* work, const uint64_t* keys
     cudaStream_t s = as_stream(stream);
     const int64_t* row_off = work;
     const int64_t* rowptr64 = work + N + 1;
-    pattern_emit_kernel<<<blocks(N, 8), 256, 0, s>>>(row_off, rowptr64, N, keys, rowptr, col, slot_ptr, slot_src, diag);
+    const KeyHalves halves = key_halves(const_cast<uint64_t*>(keys), E, k);
+    if (reinterpret_cast<uint32_t*>(slot_src) != halves.src)
+        TCB_CHECK_CUDA(cudaMemcpyAsync(slot_src, halves.src, sizeof(int32_t) * k * k * E, cudaMemcpyDeviceToDevice, s));
+    pattern_emit_kernel<<<blocks(N, 16), 256, 0, s>>>(row_off, rowptr64, N, halves.list, rowptr, col, slot_ptr, slot_src, diag);
     TCB_CHECK_LAUNCH("pattern emit kernel");
     pattern_tail_kernel<<<1, 1, 0, s>>>(rowptr64, row_off, N, rowptr, slot_ptr);
     TCB_CHECK_LAUNCH("pattern tail kernel");
