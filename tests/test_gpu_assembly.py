@@ -48,12 +48,13 @@ def test_rows_of_every_sort(lib, cuda, k, degrees):
 
 @pytest.mark.parametrize("k,shift,inplace", [(4, 0, False), (4, 1, False), (4, 1, True), (3, 1, False)])
 def test_contributions_beside_and_inside_the_keys(lib, cuda, k, shift, inplace):
-    """slot_src in the keys' own buffer or in another; a buffer aligned to 8 bytes only
-    takes single stores instead of 16-byte ones."""
+    """slot_src in the keys' own buffer or in another; buffers that are not aligned to 16
+    bytes take single loads and stores instead of 16-byte ones."""
     from torchcor_b200._lib import check, ptr, stream_ptr
     from torchcor_b200.core.assemble import build_pattern
     el, n = _fans(k, [1, 5, 8, 16, 17, 32, 33, 64, 65, 200], np.random.default_rng(7 + k))
-    E, h, d = len(el), build_pattern(el, n), torch.from_numpy(el).to(cuda)
+    E, h = len(el), build_pattern(el, n)
+    d = torch.from_numpy(np.concatenate([np.zeros(shift, np.int32), el.reshape(-1)])).to(cuda)[shift:]
     work = torch.empty(2 * (n + 1), device=cuda, dtype=torch.int64)
     keys = torch.empty(k * k * E + shift, device=cuda, dtype=torch.int64)[shift:]
     iwork = torch.empty(2 * n + 1, device=cuda, dtype=torch.int32)

@@ -394,13 +394,14 @@ constexpr int kStartBits = 8;
 constexpr int32_t kFar = 1 << 22;
 constexpr uint32_t kRestRow = 0x80000000u, kFirstOfColumn = 0x80000000u;
 
-// Ascending bitonic sort of 32*R keys in registers, key r of a lane at lane*R + r.  A merge starts by
-// comparing mirrored places, so every exchange goes the same way: the lower place keeps the smaller key.
-template <int R>
-__device__ __forceinline__ void warp_sort(uint32_t (&key)[R]) {
-    const int lane = threadIdx.x & 31;
+// Ascending bitonic sort of G*R keys in the registers of G lanes, key r of a lane at lane*R + r.  A merge
+// starts by comparing mirrored places, so every exchange goes the same way: the lower place keeps
+// the smaller key.
+template <int G, int R>
+__device__ __forceinline__ void group_sort(uint32_t (&key)[R]) {
+    const int lane = threadIdx.x & (G - 1);
 #pragma unroll
-    for (int size = 2; size <= 32 * R; size <<= 1) {
+    for (int size = 2; size <= G * R; size <<= 1) {
         if (size <= R) {
 #pragma unroll
             for (int r = 0; r < R; ++r) {
@@ -440,107 +441,143 @@ __device__ __forceinline__ void warp_sort(uint32_t (&key)[R]) {
     }
 }
 
-// One warp sorts a row's contributions in registers: its element corners first (so
-// that a corner's rank orders elements as the reference's COO list does), then
-// one 32-bit key per contribution, (column - row, a*k + b, corner rank), R a lane.
-// A = corners a lane.  false (nothing written) if a column is too far from the row for
-// the key's 23 (A = 1) or 22 bits.
-template <int R, int A, int K>
-__device__ __forceinline__ bool sort_row(const int32_t* __restrict__ el, int64_t row, int deg, uint32_t* __restrict__ src,
-                                         uint32_t* __restrict__ list, int32_t* uniq) {
+// G lanes sort a row's contributions in registers (the other groups of the warp their own rows'):
+// its element corners first, A a lane (so that a corner's rank orders elements as the
+// reference's COO list does), then one 32-bit key per contribution, (column - row, a*k + b,
+// corner rank); a lane's first keys are those of its own corners.  shared: G*A words of the group.
+// false (nothing written) if a column is too far from the row for the key's 23 (up to 32
+// corners) or 22 bits, or the group has no row (`active`).
+template <int G, int A, int K>
+__device__ __forceinline__ bool sort_row(bool active, const int32_t* __restrict__ el, int64_t row, int deg, uint32_t* __restrict__ src,
+                                         uint32_t* __restrict__ list, int32_t* uniq, uint32_t* shared) {
     constexpr uint32_t k = K;
-    constexpr int kRankBits = A == 1 ? 5 : 6, kLow = 4 + kRankBits;
+    constexpr int R = 4 * A;   // (a triangle's fourth key is padding)
+    constexpr int kRankBits = G * A <= 32 ? 5 : 6, kLow = 4 + kRankBits;
     constexpr int kHalf = 1 << (31 - kLow);   // |column - row| below this
-    static_assert(kHalf <= kFar && 32 * R <= 1 << kStartBits, "columns of the list");
-    const int lane = threadIdx.x & 31;
+    static_assert(G * A <= 1 << kRankBits && kHalf <= kFar && G * R <= 1 << kStartBits, "fields of the keys");
+    const int lane = threadIdx.x & (G - 1);
     const int cnt = deg * K;
     uint32_t corner[A];
 #pragma unroll
     for (int r = 0; r < A; ++r) corner[r] = lane * A + r < deg ? list[lane * A + r] : 0xffffffffu;
-    warp_sort<A>(corner);
+    group_sort<G, A>(corner);
+    const bool wide = K == 4 && (reinterpret_cast<uintptr_t>(el) & 15) == 0;
     uint32_t key[R];
-    bool ok = true;
+    bool ok = active;
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-        const int i = r * 32 + lane, j = i / K, b = i - j * K;
-        uint32_t c = __shfl_sync(0xffffffffu, corner[0], A == 1 ? j & 31 : (j / A) & 31);
-        if constexpr (A == 2) {
-            const uint32_t c1 = __shfl_sync(0xffffffffu, corner[1], (j / A) & 31);
-            if (j & 1) c = c1;
+    for (int r = 0; r < A; ++r) {
+        const int j = lane * A + r;
+        const uint32_t e = corner[r] / k, a = corner[r] - e * k;
+        int32_t v[4] = {};
+        if (j < deg) {
+            if (wide) {
+                const int4 q = *reinterpret_cast<const int4*>(el + (size_t)e * k);
+                v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+            } else {
+#pragma unroll
+                for (int b = 0; b < K; ++b) v[b] = el[(size_t)e * k + b];
+            }
         }
-        key[r] = 0xffffffffu;
-        if (i < cnt) {
-            const uint32_t e = c / k, a = c - e * k;
-            const int64_t d = (int64_t)el[e * k + b] - row;
-            ok = ok && d > -kHalf && d < kHalf - 1;   // (kHalf - 1 with all low bits set would be the padding)
-            key[r] = ((uint32_t)(int32_t)(d + kHalf) << kLow) | ((a * k + b) << kRankBits) | (uint32_t)j;
+        shared[j] = e * (k * k);
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            key[r * 4 + b] = 0xffffffffu;
+            if (b < K && j < deg) {
+                const int64_t d = (int64_t)v[b] - row;
+                ok = ok && d > -kHalf && d < kHalf - 1;   // (kHalf - 1 with all low bits set would be the padding)
+                key[r * 4 + b] = ((uint32_t)(int32_t)(d + kHalf) << kLow) | ((a * k + b) << kRankBits) | (uint32_t)j;
+            }
         }
     }
-    if (!__all_sync(0xffffffffu, ok)) return false;
-    warp_sort<R>(key);
-    const uint32_t last = __shfl_up_sync(0xffffffffu, key[R - 1], 1);
-    uint32_t out[R];
+    group_sort<G, R>(key);
+    const uint32_t last = __shfl_up_sync(0xffffffffu, key[R - 1], 1, G);
+    const unsigned group = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1) << (threadIdx.x & 31 & ~(G - 1));
+    ok = (__ballot_sync(0xffffffffu, ok) & group) == group;   // (also orders `shared`)
+    __syncwarp();
     bool first[R];
     int u = 0;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int p = lane * R + r;
-        const int j = key[r] & ((1 << kRankBits) - 1), ab = (key[r] >> kRankBits) & 15;
-        uint32_t c = __shfl_sync(0xffffffffu, corner[0], A == 1 ? j : j / A);
-        if constexpr (A == 2) {
-            const uint32_t c1 = __shfl_sync(0xffffffffu, corner[1], j / A);
-            if (j & 1) c = c1;
-        }
-        out[r] = (c / k) * (k * k) + ab;
         first[r] = p < cnt && (p == 0 || (key[r] >> kLow) != ((r ? key[r - 1] : last) >> kLow));
         u += first[r];
     }
-    // (a tetrahedron's four contributions keep the places of a row in multiples of four)
-    constexpr int V = K == 4 ? (R < 4 ? R : 4) : 1;
-    if (V > 1 && (reinterpret_cast<uintptr_t>(src) & (4 * V - 1)) == 0) {
-#pragma unroll
-        for (int r = 0; r < R; r += V) {
-            if (lane * R + r >= cnt) break;
-            if constexpr (V == 4) *reinterpret_cast<uint4*>(src + lane * R + r) = make_uint4(out[r], out[r + 1], out[r + 2], out[r + 3]);
-            if constexpr (V == 2) *reinterpret_cast<uint2*>(src + lane * R + r) = make_uint2(out[r], out[r + 1]);
-        }
-    } else {
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-            if (lane * R + r < cnt) src[lane * R + r] = out[r];
-    }
     int at = u;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, at, o);
+    for (int o = 1; o < G; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, at, o, G);
         if (lane >= o) at += v;
     }
-    if (lane == 31) *uniq = at;
+    if (!ok) return false;
+    if (lane == G - 1) *uniq = at;
     at -= u;
 #pragma unroll
     for (int r = 0; r < R; ++r)
         if (first[r]) list[at++] = (((key[r] >> kLow) + (kFar - kHalf)) << kStartBits) | (uint32_t)(lane * R + r);
+    // (a tetrahedron's four contributions keep the places of a row in multiples of four)
+    const bool wide_out = K == 4 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+#pragma unroll
+    for (int r = 0; r < R; r += 4) {
+        const int p = lane * R + r;
+        if (p >= cnt) break;
+        uint32_t out[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t v = key[r + q];
+            out[q] = shared[v & (G * A - 1)] + ((v >> kRankBits) & 15);
+        }
+        if (wide_out) {
+            *reinterpret_cast<uint4*>(src + p) = make_uint4(out[0], out[1], out[2], out[3]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (p + q < cnt) src[p + q] = out[q];
+        }
+    }
     return true;
 }
 
 // Rows of up to 64 corners whose columns are near enough (all rows of meshes below two
-// million nodes), one warp each; the others go to `rest` (rest[0] counts).  Bound by
-// the exchanges: 28 steps of 128 keys in registers, one 32-bit shuffle and one minimum a key.
-// 531,441 nodes, 50 M contributions: 482 -> 378 us with exchanges that all go one way
-// (no select of a direction) and 4 bytes a contribution written in 16-byte stores.
+// million nodes); the others go to `rest` (rest[0] counts).  Four rows a warp, 8 lanes each, where
+// they have up to 32 corners, else a warp a row.  Bound by the exchanges: of the 28 steps of a
+// 128-key sort 6 leave a lane's 16 registers with 8 lanes a row, 15 with a warp a row and 4
+// registers, and a shuffle costs as much issue as four other instructions.
+// Measured on B200: 531,441 nodes, 50 M contributions, a warp a row 378 -> 297 us (482 with exchanges that
+// selected a direction and 8-byte keys written back); the whole pattern 633 -> 554 us, of a
+// level-8 icosphere (655,362 nodes) 454 -> 309 us, of a 20-cube even (140, launches).
 template <int K>
 __global__ void __launch_bounds__(256) pattern_sort_kernel(const int32_t* __restrict__ el, const int64_t* __restrict__ row_off, int64_t N,
                                                            KeyHalves keys, int32_t* __restrict__ uniq, int64_t* __restrict__ rest) {
-    const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (row >= N) return;
-    const int64_t b = row_off[row];
-    const int cnt = (int)(row_off[row + 1] - b), deg = cnt / K;
-    bool done = false;
-    if (cnt <= 32) done = sort_row<1, 1, K>(el, row, deg, keys.src + b, keys.list + b, uniq + row);
-    else if (cnt <= 64) done = sort_row<2, 1, K>(el, row, deg, keys.src + b, keys.list + b, uniq + row);
-    else if (deg <= 32) done = sort_row<4, 1, K>(el, row, deg, keys.src + b, keys.list + b, uniq + row);
-    else if (deg <= 64) done = sort_row<8, 2, K>(el, row, deg, keys.src + b, keys.list + b, uniq + row);
-    if (!done && (threadIdx.x & 31) == 0)
+    constexpr int G = 8, kRows = 32 / G;
+    __shared__ uint32_t shared[8][128];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t row0 = ((int64_t)blockIdx.x * 8 + warp) * kRows;
+    if (row0 >= N) return;
+    const int64_t row = row0 + lane / G;
+    const bool in = row < N;
+    const int64_t b = in ? row_off[row] : 0;
+    const int64_t deg64 = in ? (row_off[row + 1] - b) / K : 0;
+    const bool small = in && deg64 <= 32;
+    const int deg = small ? (int)deg64 : 0;
+    int most = deg;
+#pragma unroll
+    for (int o = G; o < 32; o <<= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+    uint32_t* mine = shared[warp] + lane / G * 32;
+    bool done;
+    if (most <= 8) done = sort_row<G, 1, K>(small, el, row, deg, keys.src + b, keys.list + b, uniq + row, mine);
+    else if (most <= 16) done = sort_row<G, 2, K>(small, el, row, deg, keys.src + b, keys.list + b, uniq + row, mine);
+    else done = sort_row<G, 4, K>(small, el, row, deg, keys.src + b, keys.list + b, uniq + row, mine);
+    unsigned large = __ballot_sync(0xffffffffu, in && deg64 > 32 && deg64 <= 64 && lane % G == 0);
+    while (large) {
+        const int from = __ffs(large) - 1;
+        large &= large - 1;
+        const int64_t r = row0 + from / G, rb = __shfl_sync(0xffffffffu, b, from);
+        const int rd = __shfl_sync(0xffffffffu, (int)deg64, from);
+        __syncwarp();   // the words of the sort before have been read
+        const bool ok = sort_row<32, 2, K>(true, el, r, rd, keys.src + rb, keys.list + rb, uniq + r, shared[warp]);
+        if (lane / G == from / G) done = ok;
+    }
+    if (in && !done && lane % G == 0)
         rest[1 + atomicAdd(reinterpret_cast<unsigned long long*>(rest), 1ull)] = row;
 }
 
@@ -735,8 +772,8 @@ extern "C" int tcb_pattern_device(const int32_t* elems, int64_t E, int32_t k, in
     const KeyHalves halves = key_halves(keys, E, k);
     pattern_fill_kernel<<<blocks(E, kThreads), kThreads, 0, s>>>(elems, E, k, N, row_off, cnt, halves.list);
     TCB_CHECK_LAUNCH("pattern fill kernel");
-    if (k == 4) pattern_sort_kernel<4><<<blocks(N, 8), 256, 0, s>>>(elems, row_off, N, halves, uniq, rowptr64);
-    else pattern_sort_kernel<3><<<blocks(N, 8), 256, 0, s>>>(elems, row_off, N, halves, uniq, rowptr64);
+    if (k == 4) pattern_sort_kernel<4><<<blocks(N, 32), 256, 0, s>>>(elems, row_off, N, halves, uniq, rowptr64);
+    else pattern_sort_kernel<3><<<blocks(N, 32), 256, 0, s>>>(elems, row_off, N, halves, uniq, rowptr64);
     TCB_CHECK_LAUNCH("pattern sort kernel");
     pattern_rest_kernel<<<(unsigned)std::min<int64_t>(blocks(N, kSortWarps), 592), kSortWarps * 32, 0, s>>>(
         elems, E, k, row_off, halves, uniq, rowptr64, err);
