@@ -114,3 +114,24 @@ def test_sliced_ell_on_the_device(lib, cuda, n, widest):
     assert np.array_equal(scol.cpu().numpy(), pc)
     for t, p in zip(sell, pv):
         assert np.array_equal(t.cpu().numpy(), p)
+
+
+@pytest.mark.parametrize("nnz,shift", [(1, 0), (4, 0), (1023, 0), (4099, 0), (4099, 1)])
+def test_system_values_in_vectors_and_one_by_one(lib, cuda, nnz, shift):
+    """A, K / chi and K' at vector remainders and on arrays that are not aligned to 16 bytes,
+    each float32 operation rounded by itself as in numpy: equal to the bit."""
+    from torchcor_b200._lib import check, ptr, stream_ptr
+    rng = np.random.default_rng(nnz)
+    k, m = rng.normal(size=nnz).astype(np.float32), rng.uniform(0.1, 1, nnz).astype(np.float32)
+    kd, md = (torch.from_numpy(np.concatenate([np.zeros(shift, np.float32), v])).to(cuda)[shift:] for v in (k, m))
+    a, kr = (torch.zeros(nnz + shift, device=cuda)[shift:] for _ in range(2))
+    d, diag = torch.zeros(1, device=cuda), torch.zeros(1, device=cuda, dtype=torch.int32)
+    chi, cm, dt, theta = 140.0, 0.01, 0.01, 0.5
+    split = torch.ones(1, device=cuda, dtype=torch.int32)
+    check(lib.tcb_assemble_system(nnz, 1, 1, ptr(diag), ptr(kd), ptr(md), chi, cm, dt, theta, ptr(a), ptr(kr), ptr(d),
+                                  ptr(split), stream_ptr()))
+    f = np.float32
+    kc, mc = k / f(chi), m * f(cm)
+    want, wr = mc + kc * f(dt) * f(theta), kc * f((1 - theta) * dt)
+    assert np.array_equal(kd.cpu().numpy(), kc) and np.array_equal(a.cpu().numpy(), want)
+    assert np.array_equal(kr.cpu().numpy(), wr) and bool(split.item()) == bool(np.all(mc + wr == want))

