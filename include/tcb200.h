@@ -249,6 +249,9 @@ int64_t tcb_mono_scratch_doubles(void);
  * case: meshes whose matrix does not fit in the GPU's shared memory, fused_step != 0.
  * Negative = error status. */
 int64_t tcb_mono_work_bytes(const tcb_mono* m, int32_t* entries, void* stream);
+/* The same with the n_slices + 1 offsets of m->slice_ptr given on the host: no copy, no
+ * synchronisation, nothing on any stream (callable while a stream is being recorded). */
+int64_t tcb_mono_work_bytes_host(const tcb_mono* m, const int64_t* slice_ptr, int32_t* entries);
 /* Run steps [step_begin, step_end) (1-based, step_begin must equal the device
  * counter).  Non-convergence is not an error (n_iter == max_iter), as in the
  * reference. */

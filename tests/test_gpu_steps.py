@@ -118,3 +118,58 @@ def test_step_graph_recorded_while_garbage_holds_device_memory(lib, cuda):
     finally:
         gc.set_threshold(*old)
     torch.cuda.synchronize(cuda)
+
+
+def test_first_steps_on_a_stream_of_the_callers(lib, cuda):
+    """The first steps of a simulation on a stream other than the current one, which is busy:
+    they neither wait for it nor read an exchange buffer that it has yet to zero, so they are those on
+    the current stream bit for bit.  Freed memory of that size is full of ones."""
+    sim = _sim("cube", 20, "ttp", cuda)
+    ref = _run(sim, 1e-6, 100, True, 0, [20])
+    nbytes = sim._sim["work"].numel()
+    sim.prepare(1e-6, 1e-6, 100, snapshot_interval=sim.T)
+    dirty = [torch.full((nbytes,), 255, device=cuda, dtype=torch.uint8) for _ in range(4)]
+    big = torch.empty((2, 1 << 30), device=cuda, dtype=torch.uint8)
+    side = torch.cuda.Stream(cuda)
+    torch.cuda.synchronize(cuda)
+    del dirty
+    for _ in range(300):          # about 0.1 s
+        big[1].copy_(big[0])
+    busy = torch.cuda.Event()
+    busy.record()
+    assert sim.run_steps(20, stream=side) == 20
+    side.synchronize()
+    assert not busy.query()       # the steps did not wait for the copies
+    assert sim._sim["work"] is not None
+    torch.cuda.synchronize(cuda)
+    assert torch.equal(sim._sim["x"][:, : sim.n_nodes], ref["x"])
+    assert torch.equal(sim._sim["step_iters"], ref["iters"])
+
+
+def test_steps_recorded_by_the_caller_right_after_prepare(lib, cuda):
+    """run_steps under a recording of the caller's own allocates, copies and waits for nothing: the
+    recorded steps are the ones launched one by one, and later steps run as stretches again."""
+    sim = _sim("cube", 10, "ttp", cuda)
+    ref = _run(sim, 1e-6, 100, True, 2, [10])
+    sim.prepare(1e-6, 1e-6, 100, snapshot_interval=sim.T)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        assert sim.run_steps(10) == 10
+    assert sim._sim["work"] is None
+    graph.replay()
+    torch.cuda.synchronize(cuda)
+    assert torch.equal(sim._sim["x"][:, : sim.n_nodes], ref["x"])
+    sim.run_steps(3)
+    assert sim._sim["work"] is not None and int(sim._sim["counter"][0].item()) == 14
+
+
+def test_launch_shape_taken_back_before_the_first_stretch(lib, cuda):
+    """Steps under a pinned launch shape ask for no exchange buffer; without it the next ones do."""
+    sim = _sim("cube", 6, "ms", cuda)
+    sim.prepare(1e-6, 1e-6, 100, snapshot_interval=sim.T)
+    sim.set_launch(fused_step=1)
+    sim.run_steps(2)
+    assert sim._sim["work"] is None
+    sim.set_launch(fused_step=0)
+    sim.run_steps(2)
+    assert sim._sim["work"] is not None and int(sim._sim["counter"][0].item()) == 5

@@ -140,20 +140,29 @@ class System:
     sell_a: torch.Tensor
     sell_dcol: torch.Tensor = None   # int16 col - row, or None
     a_split: bool = False            # every A value == fp32(fp32(M*Cm) + K')
+    host_slices: np.ndarray = None   # slice_ptr on the host, for meshes of up to HOST_SLICES slices
 
     def csr(self, values):
         return torch.sparse_csr_tensor(self.rowptr, self.col, values, size=(self.n, self.n))
 
 
+# Meshes of up to this many slices (524,288 nodes) keep a host copy of slice_ptr: whether, and with how
+# much shared memory a block, their steps run as persistent launches follows from it.  A row takes 44
+# bytes there and 10 for each of its three or more entries, 39 MB for so many nodes, and the GPU's
+# shared memory is 34 MB: larger meshes need none.
+HOST_SLICES = 1 << 14
+
+
 def _sliced_ell(pat, rowptr, col, values, dev, flag=None):
-    """Sliced-ELL copy of CSR values on the device: (n_slices, slice_ptr, columns, int16
-    column offsets or None, [values...], flag as a bool).  ``flag``: an int32 device scalar read in
-    the same synchronisation as the width of the columns."""
+    """Sliced-ELL copy of CSR values on the device, as fields of ``System``, and ``flag`` as a
+    bool.  ``flag``: an int32 device scalar read in the same copy as the width of the columns."""
     lib = _lib.load()
     s = stream_ptr()
     n = pat.n_nodes
     n_slices = (n + _lib.TCB_SLICE - 1) // _lib.TCB_SLICE
-    slice_ptr = torch.empty(n_slices + 1, device=dev, dtype=torch.int64)
+    # the two flags behind the offsets: one copy to the host for all of them
+    ends = torch.empty(n_slices + 2, device=dev, dtype=torch.int64)
+    slice_ptr, flags = ends[:n_slices + 1], ends[n_slices + 1:].view(torch.int32)
     scratch = torch.empty(int(lib.tcb_sell_layout_scratch(n)), device=dev, dtype=torch.int64)
     n_entries = C.c_int64()
     check(lib.tcb_sell_layout_device(ptr(rowptr), n, ptr(slice_ptr), ptr(scratch), C.byref(n_entries), s))
@@ -165,12 +174,16 @@ def _sliced_ell(pat, rowptr, col, values, dev, flag=None):
     check(lib.tcb_sell_pack(n, ptr(rowptr), ptr(col), ptr(slice_ptr), n_slices, len(values), vin, ptr(sell_col), vout, s))
     # int16 column offsets when the mesh ordering keeps every |col - row| < 32768
     dcol = torch.empty(ne, device=dev, dtype=torch.int16)
-    flags = torch.zeros(2, device=dev, dtype=torch.int32)
+    flags.zero_()
     check(lib.tcb_sell_delta(n, ptr(slice_ptr), n_slices, ptr(sell_col), ptr(dcol), ptr(flags), s))
     if flag is not None:
         flags[1:] = flag
-    width, flag = flags.tolist()
-    return n_slices, slice_ptr, sell_col, dcol if width < 32768 else None, sell, bool(flag)
+    small = n_slices <= HOST_SLICES
+    host = (ends if small else ends[n_slices + 1:]).cpu().numpy()
+    width, flag = host[-1:].view(np.int32).tolist()
+    fields = dict(n_slices=n_slices, slice_ptr=slice_ptr, sell_col=sell_col, sell_dcol=dcol if width < 32768 else None,
+                  sell_m=sell[0], sell_k=sell[1], sell_a=sell[2], host_slices=host[:-1] if small else None)
+    return fields, bool(flag)
 
 
 def assemble_system(nodes, elems_np, sl, st, fibres, dt, chi=140, cm=0.01, theta=0.5, pattern=None) -> System:
@@ -199,10 +212,9 @@ def assemble_system(nodes, elems_np, sl, st, fibres, dt, chi=140, cm=0.01, theta
     check(lib.tcb_assemble_system(nnz, n, n_pad, ptr(diag), ptr(k_val), ptr(m_val), float(chi), float(cm), float(dt),
                                   float(theta), ptr(a_val), ptr(krhs), ptr(d_inv), ptr(a_split), s))
     rowptr, col = pat.on("rowptr", dev), pat.on("col", dev)
-    n_slices, slice_ptr, sell_col, dcol, sell, split = _sliced_ell(pat, rowptr, col, [m_val, krhs, a_val], dev, a_split)
+    sell, split = _sliced_ell(pat, rowptr, col, [m_val, krhs, a_val], dev, a_split)
     return System(n=n, n_pad=n_pad, nnz=nnz, rowptr=rowptr, col=col, m_val=m_val, k_val=k_val, a_val=a_val,
-                  krhs_val=krhs, d_inv=d_inv, n_slices=n_slices, slice_ptr=slice_ptr, sell_col=sell_col,
-                  sell_m=sell[0], sell_k=sell[1], sell_a=sell[2], sell_dcol=dcol, a_split=split)
+                  krhs_val=krhs, d_inv=d_inv, a_split=split, **sell)
 
 
 def assemble_phie(nodes, elems_np, sl_i, st_i, sl_e, st_e, fibres) -> System:
@@ -238,10 +250,9 @@ def assemble_phie(nodes, elems_np, sl_i, st_i, sl_e, st_e, fibres) -> System:
     check(lib.tcb_assemble_system(nnz, n, n_pad, ptr(diag), ptr(kie), ptr(mass), 1.0, 0.0, 1.0, 1.0,
                                   ptr(a_val), ptr(zero), ptr(d_inv), None, s))
     rowptr, col = pat.on("rowptr", dev), pat.on("col", dev)
-    n_slices, slice_ptr, sell_col, dcol, sell, _ = _sliced_ell(pat, rowptr, col, [ki, zero, a_val], dev)
+    sell, _ = _sliced_ell(pat, rowptr, col, [ki, zero, a_val], dev)
     return System(n=n, n_pad=n_pad, nnz=nnz, rowptr=rowptr, col=col, m_val=ki, k_val=kie, a_val=a_val,
-                  krhs_val=zero, d_inv=d_inv, n_slices=n_slices, slice_ptr=slice_ptr, sell_col=sell_col,
-                  sell_m=sell[0], sell_k=sell[1], sell_a=sell[2], sell_dcol=dcol, a_split=False)
+                  krhs_val=zero, d_inv=d_inv, a_split=False, **sell)
 
 
 class _Matrices:

@@ -706,7 +706,8 @@ int launch_steps(const tcb_mono* m, const MonoDev& d, int64_t n_steps, bool ioni
 
 }  // namespace tcb
 
-extern "C" int64_t tcb_mono_work_bytes(const tcb_mono* m, int32_t* entries, void* stream) {
+// `host_slices`: slice_ptr on the host, or null (read from the device on `stream`, which is synchronised)
+static int64_t work_bytes(const tcb_mono* m, const int64_t* host_slices, int32_t* entries, cudaStream_t s) {
     using namespace tcb;
     const int st = validate_mono(m);
     if (st) return st;
@@ -720,10 +721,13 @@ extern "C" int64_t tcb_mono_work_bytes(const tcb_mono* m, int32_t* entries, void
         return 0;
     const int64_t grid = steps_blocks(d, false);
     if (!steps_layout(d, grid, TCB_SLICE * ceil_div(d.n_slices, grid), 0, false, &pl)) return 0;
-    std::vector<int64_t> sp((size_t)d.n_slices + 1);
-    cudaStream_t s = as_stream(stream);
-    TCB_CHECK_CUDA(cudaMemcpyAsync(sp.data(), d.slice_ptr, sp.size() * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-    TCB_CHECK_CUDA(cudaStreamSynchronize(s));
+    std::vector<int64_t> copy;
+    if (!host_slices) {
+        copy.resize((size_t)d.n_slices + 1);
+        TCB_CHECK_CUDA(cudaMemcpyAsync(copy.data(), d.slice_ptr, copy.size() * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+        TCB_CHECK_CUDA(cudaStreamSynchronize(s));
+    }
+    const int64_t* sp = host_slices ? host_slices : copy.data();
     auto most = [&](int64_t nb) {
         int64_t e = 0;
         for (int64_t b = 0; b < nb; ++b) e = std::max(e, sp[(b + 1) * d.n_slices / nb] - sp[b * d.n_slices / nb]);
@@ -739,4 +743,13 @@ extern "C" int64_t tcb_mono_work_bytes(const tcb_mono* m, int32_t* entries, void
         *entries = (int32_t)e;
     }
     return (int64_t)(kHeadBytes + kPartBytes + 2 * (size_t)m->n_pad * sizeof(float4));
+}
+
+extern "C" int64_t tcb_mono_work_bytes(const tcb_mono* m, int32_t* entries, void* stream) {
+    return work_bytes(m, nullptr, entries, tcb::as_stream(stream));
+}
+
+extern "C" int64_t tcb_mono_work_bytes_host(const tcb_mono* m, const int64_t* slice_ptr, int32_t* entries) {
+    if (!slice_ptr) return tcb::fail(TCB_EINVAL, "tcb_mono_work_bytes_host: null slice_ptr");
+    return work_bytes(m, slice_ptr, entries, nullptr);
 }

@@ -45,16 +45,18 @@ def rcm_order(elems, n_nodes):
     return np.asarray(reverse_cuthill_mckee(g, symmetric_mode=True), dtype=np.int64)
 
 
-def _work_buffer(m, device):
-    """Zeroed ``tcb_mono.work`` of the struct ``m`` (set in it), or None where steps are
-    launched one by one in any case."""
+def _work_buffer(m, system):
+    """``tcb_mono.work`` of the struct ``m`` (set in it), made and zeroed on the current stream, or
+    None where steps are launched one by one in any case.  Nothing is synchronised."""
     entries = C.c_int32()
-    nbytes = int(_lib.load().tcb_mono_work_bytes(C.byref(m), C.byref(entries), stream_ptr()))
+    if system.host_slices is None:
+        return None
+    nbytes = int(_lib.load().tcb_mono_work_bytes_host(C.byref(m), ptr(system.host_slices), C.byref(entries)))
     if nbytes < 0:
         check(nbytes)
     if nbytes == 0:
         return None
-    work = torch.zeros(nbytes, device=device, dtype=torch.uint8)
+    work = torch.zeros(nbytes, device=system.slice_ptr.device, dtype=torch.uint8)
     m.work, m.work_entries = ptr(work), entries.value
     return work
 
@@ -223,7 +225,7 @@ class Monodomain:
             counter=torch.tensor([1, 0, 0, 0], device=dev, dtype=torch.int32),
             scratch=torch.zeros(int(_lib.load().tcb_mono_scratch_doubles()), device=dev, dtype=torch.float64),
             barrier=torch.zeros(4, device=dev, dtype=torch.int32),
-            params=im.param_array(), per_frame=per_frame, next_step=1,
+            params=im.param_array(), per_frame=per_frame, next_step=1, work=None, work_asked=False,
         )
         m = _lib.tcb_mono()
         m.n_nodes, m.n_pad, m.n_slices, m.nt = n, n_pad, s.n_slices, nt
@@ -260,18 +262,28 @@ class Monodomain:
         if (m.node_params or None) != want:
             m.node_params = want
 
-    def _sync_launch(self):
+    def _sync_launch(self, stream=None):
         """What a launch reads besides the buffers of ``_setup``: the per-node parameters,
         and the exchange buffer of the many-steps-per-launch kernel where it applies
-        (allocated when the simulation is first stepped by itself; batches do without)."""
+        (made when the simulation is first stepped by itself; batches do without).  Its
+        zeroes are written on the stream that the steps go to, so they come before
+        them whatever the caller ordered.  While that stream is being recorded nothing is
+        allocated: the steps of the recording are then launched one by one."""
         self._sync_node_params()
         sim = self._sim
-        if "work" not in sim:
-            sim["work"] = _work_buffer(sim["struct"], self.device)
+        # (not asked under a pinned launch shape, which may be taken back later)
+        if not sim["work_asked"] and not sim["struct"].fused_step:
+            if stream is not None and not isinstance(stream, torch.cuda.Stream):
+                stream = torch.cuda.ExternalStream(stream.cuda_stream, device=self.device)
+            with torch.cuda.stream(stream):
+                if not torch.cuda.is_current_stream_capturing():
+                    sim["work"] = _work_buffer(sim["struct"], self.system)
+                    sim["work_asked"] = True
 
     def run_steps(self, n_steps, stream=None):
-        """Advance the prepared simulation by ``n_steps`` steps (asynchronous)."""
-        self._sync_launch()
+        """Advance the prepared simulation by ``n_steps`` steps on ``stream`` (default: the current
+        one), asynchronously; also while the stream is being recorded in a CUDA graph."""
+        self._sync_launch(stream)
         sim = self._sim
         a = sim["next_step"]
         b = min(a + n_steps, self.nt + 1)
@@ -521,7 +533,7 @@ class Monodomain:
         m.step_iters, m.counter = ptr(buf["step_iters"]), ptr(buf["counter"])
         m.scratch, m.barrier = ptr(buf["scratch"]), ptr(buf["barrier"])
         m.params = buf["params"].ctypes.data
-        buf["work"] = _work_buffer(m, dev)
+        buf["work"] = _work_buffer(m, s)
         lib = _lib.load()
         out = torch.empty((F, n), **f32)
         for k in range(F):

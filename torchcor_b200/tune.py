@@ -243,7 +243,8 @@ def tune_single(sim, steps=5, cache=None, force=False):
     lib = _lib.load()
     # where a stretch of steps is one persistent launch (tcb_mono.work), the fused step is no candidate
     m.fused_step = 0
-    stretches = int(lib.tcb_mono_work_bytes(C.byref(m), C.byref(C.c_int32()), _lib.stream_ptr())) > 0
+    slices = sim.system.host_slices
+    stretches = slices is not None and int(lib.tcb_mono_work_bytes_host(C.byref(m), _lib.ptr(slices), C.byref(C.c_int32()))) > 0
     if hit is not None and 0 <= int(hit.get("ionic_variant", 0)) <= len(shapes):
         m.ionic_variant, m.cg_per_sm = int(hit["ionic_variant"]), int(hit.get("cg_per_sm", 0))
         m.fused_step = 0 if stretches else int(hit.get("fused_step", 0))
