@@ -173,3 +173,23 @@ def test_launch_shape_taken_back_before_the_first_stretch(lib, cuda):
     sim.set_launch(fused_step=0)
     sim.run_steps(2)
     assert sim._sim["work"] is not None and int(sim._sim["counter"][0].item()) == 5
+
+
+def test_replay_on_another_stream_follows_what_came_before_the_recording(lib, cuda):
+    """Steps queued behind other work before the recording, replayed right after it on an idle stream
+    that nothing orders with the first: the replay comes after them."""
+    sim = _sim("cube", 20, "ttp", cuda)
+    ref = _run(sim, 1e-6, 100, True, 0, [8])
+    sim.prepare(1e-6, 1e-6, 100, snapshot_interval=sim.T)
+    sim.run_steps(1)
+    big = torch.empty((2, 1 << 30), device=cuda, dtype=torch.uint8)
+    for _ in range(100):
+        big[1].copy_(big[0])
+    sim.run_steps(2)
+    replay = sim.capture_steps(5)
+    side = torch.cuda.Stream(cuda)
+    with torch.cuda.stream(side):
+        replay()
+    side.synchronize()
+    assert torch.equal(sim._sim["x"][:, : sim.n_nodes], ref["x"])
+    assert torch.equal(sim._sim["step_iters"], ref["iters"])

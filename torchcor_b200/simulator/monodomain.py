@@ -310,17 +310,21 @@ class Monodomain:
 
     def capture_steps(self, n_steps):
         """Record ``n_steps`` steps of the prepared simulation in a CUDA graph;
-        returns a callable replaying them (with the step bookkeeping)."""
+        returns a callable replaying them (with the step bookkeeping) on the stream that
+        is current at the replay.  The device is synchronised before the recording, so a
+        replay on any stream comes after everything queued until then."""
         self._sync_launch()
         sim = self._sim
         lib = _lib.load()
         # the first launch on a device configures kernel attributes: keep it outside capture
         graph = torch.cuda.CUDAGraph()
-        # recorded on a stream of its own without the garbage collection, device
-        # synchronisation and release of cached memory that torch.cuda.graph() begins
-        # with (2 to 60 ms): nothing is allocated while the launches are recorded, and
-        # the collector, which could free another graph or tensor in the middle of it
-        # on this thread, waits until it is over
+        # the buffers' set-up and earlier steps, on whatever stream they were queued
+        torch.cuda.synchronize(self.device)
+        # recorded on a stream of its own without the garbage collection and release of
+        # cached memory that torch.cuda.graph() begins with (2 to 60 ms): nothing is
+        # allocated while the launches are recorded, and the collector, which could free
+        # another graph or tensor in the middle of it on this thread, waits until it is
+        # over
         side = torch.cuda.Stream(self.device)
         struct, stream = C.byref(sim["struct"]), side.cuda_stream
         with _recording, torch.cuda.stream(side):
