@@ -154,8 +154,14 @@ HOST_SLICES = 1 << 14
 
 
 def _sliced_ell(pat, rowptr, col, values, dev, flag=None):
-    """Sliced-ELL copy of CSR values on the device, as fields of ``System``, and ``flag`` as a
-    bool.  ``flag``: an int32 device scalar read in the same copy as the width of the columns."""
+    """Sliced-ELL copy of CSR values on the device: (n_slices, slice_ptr, columns, int16
+    column offsets or None, [values...], flag as a bool).  ``flag``: an int32 device scalar read in
+    the same copy as the width of the columns."""
+    return _sliced_ell_host(pat, rowptr, col, values, dev, flag)[:-1]
+
+
+def _sliced_ell_host(pat, rowptr, col, values, dev, flag=None):
+    """``_sliced_ell`` with ``System.host_slices`` behind its values."""
     lib = _lib.load()
     s = stream_ptr()
     n = pat.n_nodes
@@ -181,9 +187,8 @@ def _sliced_ell(pat, rowptr, col, values, dev, flag=None):
     small = n_slices <= HOST_SLICES
     host = (ends if small else ends[n_slices + 1:]).cpu().numpy()
     width, flag = host[-1:].view(np.int32).tolist()
-    fields = dict(n_slices=n_slices, slice_ptr=slice_ptr, sell_col=sell_col, sell_dcol=dcol if width < 32768 else None,
-                  sell_m=sell[0], sell_k=sell[1], sell_a=sell[2], host_slices=host[:-1] if small else None)
-    return fields, bool(flag)
+    return (n_slices, slice_ptr, sell_col, dcol if width < 32768 else None, sell, bool(flag),
+            host[:-1] if small else None)
 
 
 def assemble_system(nodes, elems_np, sl, st, fibres, dt, chi=140, cm=0.01, theta=0.5, pattern=None) -> System:
@@ -212,9 +217,11 @@ def assemble_system(nodes, elems_np, sl, st, fibres, dt, chi=140, cm=0.01, theta
     check(lib.tcb_assemble_system(nnz, n, n_pad, ptr(diag), ptr(k_val), ptr(m_val), float(chi), float(cm), float(dt),
                                   float(theta), ptr(a_val), ptr(krhs), ptr(d_inv), ptr(a_split), s))
     rowptr, col = pat.on("rowptr", dev), pat.on("col", dev)
-    sell, split = _sliced_ell(pat, rowptr, col, [m_val, krhs, a_val], dev, a_split)
+    n_slices, slice_ptr, sell_col, dcol, sell, split, host = _sliced_ell_host(pat, rowptr, col, [m_val, krhs, a_val], dev,
+                                                                              a_split)
     return System(n=n, n_pad=n_pad, nnz=nnz, rowptr=rowptr, col=col, m_val=m_val, k_val=k_val, a_val=a_val,
-                  krhs_val=krhs, d_inv=d_inv, a_split=split, **sell)
+                  krhs_val=krhs, d_inv=d_inv, n_slices=n_slices, slice_ptr=slice_ptr, sell_col=sell_col,
+                  sell_m=sell[0], sell_k=sell[1], sell_a=sell[2], sell_dcol=dcol, a_split=split, host_slices=host)
 
 
 def assemble_phie(nodes, elems_np, sl_i, st_i, sl_e, st_e, fibres) -> System:
@@ -250,9 +257,10 @@ def assemble_phie(nodes, elems_np, sl_i, st_i, sl_e, st_e, fibres) -> System:
     check(lib.tcb_assemble_system(nnz, n, n_pad, ptr(diag), ptr(kie), ptr(mass), 1.0, 0.0, 1.0, 1.0,
                                   ptr(a_val), ptr(zero), ptr(d_inv), None, s))
     rowptr, col = pat.on("rowptr", dev), pat.on("col", dev)
-    sell, _ = _sliced_ell(pat, rowptr, col, [ki, zero, a_val], dev)
+    n_slices, slice_ptr, sell_col, dcol, sell, _, host = _sliced_ell_host(pat, rowptr, col, [ki, zero, a_val], dev)
     return System(n=n, n_pad=n_pad, nnz=nnz, rowptr=rowptr, col=col, m_val=ki, k_val=kie, a_val=a_val,
-                  krhs_val=zero, d_inv=d_inv, a_split=False, **sell)
+                  krhs_val=zero, d_inv=d_inv, n_slices=n_slices, slice_ptr=slice_ptr, sell_col=sell_col,
+                  sell_m=sell[0], sell_k=sell[1], sell_a=sell[2], sell_dcol=dcol, a_split=False, host_slices=host)
 
 
 class _Matrices:
