@@ -135,3 +135,33 @@ def test_system_values_in_vectors_and_one_by_one(lib, cuda, nnz, shift):
     want, wr = mc + kc * f(dt) * f(theta), kc * f((1 - theta) * dt)
     assert np.array_equal(kd.cpu().numpy(), kc) and np.array_equal(a.cpu().numpy(), want)
     assert np.array_equal(kr.cpu().numpy(), wr) and bool(split.item()) == bool(np.all(mc + wr == want))
+
+
+@pytest.mark.parametrize("k", [3, 4])
+def test_gather_of_the_last_contributions_below_2_31(lib, cuda, k):
+    """Slots whose contributions end at 2^31 - 2, the most that the pattern build takes: sums of
+    the last 5,000, in windows that an int32 counter would step over the end of."""
+    from torchcor_b200._lib import check, ptr, stream_ptr
+    rng = np.random.default_rng(k)
+    total, tail, nnz, E = 2 ** 31 - 2, 5000, 300, 50
+    cuts = np.sort(rng.choice(np.arange(1, tail), nnz - 1, replace=False))
+    cuts = np.concatenate([[0], cuts, [tail]])
+    src = rng.integers(0, k * k * E, tail).astype(np.int32)
+    ke, mw = rng.normal(size=k * k * E).astype(np.float32), rng.normal(size=E).astype(np.float32)
+    slot_ptr = torch.from_numpy((total - tail + cuts).astype(np.int32)).to(cuda)
+    slot_src = torch.zeros(total, device=cuda, dtype=torch.int32)
+    slot_src[total - tail:] = torch.from_numpy(src).to(cuda)
+    d_ke, d_mw = torch.from_numpy(ke).to(cuda), torch.from_numpy(mw).to(cuda)
+    out = torch.zeros((2, nnz), device=cuda, dtype=torch.float32)
+    check(lib.tcb_assemble_gather(k, ptr(slot_ptr), ptr(slot_src), nnz, ptr(d_ke), ptr(d_mw), ptr(out[0]), ptr(out[1]),
+                                  stream_ptr()))
+    ab = src % (k * k)
+    mass = mw[src // (k * k)] * np.where(ab // k == ab % k, np.float32(2), np.float32(1))
+    want = np.zeros((2, nnz), dtype=np.float32)
+    for s in range(nnz):
+        for j, v in enumerate((ke[src], mass)):
+            # float32 sums one by one, in order
+            want[j, s] = np.add.accumulate(v[cuts[s]: cuts[s + 1]], dtype=np.float32)[-1]
+    assert np.array_equal(out.cpu().numpy(), want)
+    del slot_src
+    torch.cuda.empty_cache()

@@ -172,19 +172,22 @@ __global__ void __launch_bounds__(kThreads) gather_kernel(const int32_t* __restr
     const int32_t c0 = slot_ptr[s0], c1 = slot_ptr[s1];
     const int32_t q0 = s < nnz ? slot_ptr[s] : c1, q1 = s < nnz ? slot_ptr[s + 1] : c1;
     float ks = 0.0f, ms = 0.0f;
-    for (int32_t w0 = c0; w0 < c1; w0 += kWindow) {
-        const int32_t w1 = c1 - w0 < kWindow ? c1 : w0 + kWindow;
+    // (offsets within a window: up to 2^31 - 2 contributions, an int32 beyond the last one would overflow)
+    for (int64_t w0 = c0; w0 < c1; w0 += kWindow) {
+        const int32_t len = c1 - w0 < kWindow ? (int32_t)(c1 - w0) : kWindow;
+        const int32_t* from = slot_src + w0;
 #pragma unroll 4
-        for (int32_t q = w0 + (int32_t)threadIdx.x; q < w1; q += kThreads) {
-            const int32_t src = slot_src[q], e = src / (K * K), ab = src - e * (K * K);
+        for (int32_t i = (int32_t)threadIdx.x; i < len; i += kThreads) {
+            const int32_t src = from[i], e = src / (K * K), ab = src - e * (K * K);
             const float m = mw[e];
-            sh[q - w0] = make_float2(ke[src], (ab / K == ab % K) ? __fmul_rn(m, 2.0f) : m);
+            sh[i] = make_float2(ke[src], (ab / K == ab % K) ? __fmul_rn(m, 2.0f) : m);
         }
         __syncthreads();
-        for (int32_t q = q0 > w0 ? q0 : w0; q < (q1 < w1 ? q1 : w1); ++q) {
-            const float2 v = sh[q - w0];
-            ks = q == q0 ? v.x : __fadd_rn(ks, v.x);
-            ms = q == q0 ? v.y : __fadd_rn(ms, v.y);
+        const int32_t i0 = (int32_t)(q0 - w0), i1 = q1 - w0 < len ? (int32_t)(q1 - w0) : len;
+        for (int32_t i = i0 > 0 ? i0 : 0; i < i1; ++i) {
+            const float2 v = sh[i];
+            ks = i == i0 ? v.x : __fadd_rn(ks, v.x);
+            ms = i == i0 ? v.y : __fadd_rn(ms, v.y);
         }
         __syncthreads();
     }
