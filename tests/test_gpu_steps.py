@@ -193,3 +193,51 @@ def test_replay_on_another_stream_follows_what_came_before_the_recording(lib, cu
     side.synchronize()
     assert torch.equal(sim._sim["x"][:, : sim.n_nodes], ref["x"])
     assert torch.equal(sim._sim["step_iters"], ref["iters"])
+
+
+FIRST_CALLS = """
+import ctypes as C, threading, torch
+from tests.test_gpu_steps import _sim
+from torchcor_b200 import _lib
+lib, cuda = _lib.load(), torch.device("cuda", 0)
+sims = [_sim("cube", 12 + k % 3, "ttp", cuda) for k in range(12)]
+for s in sims:
+    s.prepare(1e-6, 1e-6, 100, snapshot_interval=s.T)
+torch.cuda.synchronize()
+together = threading.Barrier(len(sims))
+asked, failed = [None] * len(sims), []
+def work(s):
+    n = C.c_int32()
+    slices = _lib.ptr(s.system.host_slices)
+    return lib.tcb_mono_work_bytes_host(C.byref(s._sim["struct"]), slices, C.byref(n)), n.value
+def first(k):
+    try:
+        stream = torch.cuda.Stream()
+        together.wait()
+        asked[k] = work(sims[k])                 # the first questions about the device
+        sims[k].run_steps(3, stream=stream)      # the first launches
+        stream.synchronize()
+        _lib.check(lib.tcb_mono_check(C.byref(sims[k]._sim["struct"]), stream.cuda_stream))
+    except BaseException as e:
+        failed.append(repr(e))
+threads = [threading.Thread(target=first, args=(k,)) for k in range(len(sims))]
+for t in threads: t.start()
+for t in threads: t.join()
+assert not failed, failed
+assert asked == [work(s) for s in sims] and all(b > 0 for b, _ in asked), asked
+for s in sims[3:]:
+    ref = sims[sims.index(s) % 3]
+    assert torch.equal(s._sim["x"], ref._sim["x"])
+print("same")
+"""
+
+
+def test_first_calls_from_several_threads(lib, cuda):
+    """The limits of a device and the kernels' attributes are set by whichever thread comes first;
+    the others wait for the finished values."""
+    import subprocess
+    import sys
+    from pathlib import Path
+    root = Path(__file__).resolve().parent.parent
+    r = subprocess.run([sys.executable, "-c", FIRST_CALLS], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "same" in r.stdout, r.stderr[-2000:]

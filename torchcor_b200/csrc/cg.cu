@@ -16,9 +16,6 @@
 #include <stdlib.h>
 #include <string.h>
 
-#include <mutex>
-#include <vector>
-
 #include "cg_common.cuh"
 #include "l2_hint.cuh"
 #include "mono.cuh"
@@ -158,19 +155,12 @@ struct DeviceInfo {
     int cg_blocks_per_sm = 0;
 };
 
-DeviceInfo& device_info() {
-    static std::mutex mu;
-    static std::vector<DeviceInfo> infos;
-    std::lock_guard<std::mutex> g(mu);
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if ((int)infos.size() <= dev) infos.resize(dev + 1);
-    DeviceInfo& di = infos[dev];
-    if (di.sms == 0) {
-        cudaDeviceGetAttribute(&di.sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&di.cg_blocks_per_sm, cg_kernel, kCgThreads, 0);
-    }
-    return di;
+DeviceInfo device_info() {
+    static PerDevice<DeviceInfo> infos;
+    return infos.get([](DeviceInfo& di, int dev) {
+        return cudaDeviceGetAttribute(&di.sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+               cudaOccupancyMaxActiveBlocksPerMultiprocessor(&di.cg_blocks_per_sm, cg_kernel, kCgThreads, 0) == cudaSuccess;
+    });
 }
 
 }  // namespace
@@ -188,7 +178,7 @@ static bool env_is(const char* name, const char* value) {
 int cg_blocks(const MonoDev& d) {
     int r = env_is("TCB_CG_KERNEL", "streaming") ? 0 : resident_blocks(d);
     if (r > 0) return r;
-    DeviceInfo& di = device_info();
+    const DeviceInfo di = device_info();
     int64_t want = ceil_div(d.n_slices, kMinSlicesPerBlock);
     int64_t cap = (int64_t)di.sms * di.cg_blocks_per_sm;
     if (cap > kMaxBlocks) cap = kMaxBlocks;
@@ -210,7 +200,7 @@ int launch_cg(const MonoDev& d, cudaStream_t s) {
         if (r < 0) return r;
         if (r == 1) return TCB_OK;
     }
-    DeviceInfo& di = device_info();
+    const DeviceInfo di = device_info();
     if (di.cg_blocks_per_sm <= 0) return fail(TCB_ECUDA, "CG kernel cannot be resident on this device");
     int64_t want = ceil_div(d.n_slices, kMinSlicesPerBlock);
     int64_t cap = (int64_t)di.sms * di.cg_blocks_per_sm;

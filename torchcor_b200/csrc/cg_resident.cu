@@ -471,17 +471,14 @@ PickFn cg_pick(bool i16) { return i16 ? pick<int16_t> : pick<int32_t>; }
 struct ResidentInfo {
     int sms = 0;
     int max_smem = 0;
-    bool configured = false;
 };
 
-ResidentInfo& resident_info() {
-    static ResidentInfo infos[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    ResidentInfo& ri = infos[dev & 63];
-    if (!ri.configured) {
-        cudaDeviceGetAttribute(&ri.sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaDeviceGetAttribute(&ri.max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+ResidentInfo resident_info() {
+    static PerDevice<ResidentInfo> infos;
+    return infos.get([](ResidentInfo& ri, int dev) {
+        if (cudaDeviceGetAttribute(&ri.sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&ri.max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+            return false;
         int reserve = (int)(sizeof(GridSums<4>)) + 1024;
         ri.max_smem -= reserve;
         const PickFn picks[5] = {pick<int16_t>, pick<int32_t>, kFusedPick[1], kFusedPick[2], kFusedPick[3]};
@@ -489,16 +486,15 @@ ResidentInfo& resident_info() {
             for (int ps = 1; ps <= 2; ++ps)
                 for (int as = 0; as < 2; ++as)
                     cudaFuncSetAttribute(pk(ps, as), cudaFuncAttributeMaxDynamicSharedMemorySize, ri.max_smem);
-        ri.configured = true;
-    }
-    return ri;
+        return true;
+    });
 }
 
 constexpr int kResidentBytesPerRow = 6 * sizeof(float);
 
 // Grid of the resident kernel: the most blocks per SM (2, else 1) whose rows fit.
 bool resident_plan(const MonoDev& d, unsigned* nb_out, int* cap_out, size_t* smem_out, int* per_sm_out, PickFn pk) {
-    ResidentInfo& ri = resident_info();
+    const ResidentInfo ri = resident_info();
     // d.cg_per_sm = 1 or 2 pins the blocks per SM (a tuning choice); 0: 2 if the rows fit, else 1
     const int hi = d.cg_per_sm == 1 ? 1 : 2, lo = d.cg_per_sm == 2 ? 2 : 1;
     for (int per_sm = hi; per_sm >= lo; --per_sm) {

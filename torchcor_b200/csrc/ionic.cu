@@ -207,13 +207,14 @@ __global__ void __launch_bounds__(kThreads, MINB) mono_ionic_staged_kernel(MonoD
 template <class M, int V, int MINB, class Q>
 int launch_staged(const MonoDev& d, const typename M::C& c, const typename M::Tables& T, cudaStream_t s) {
     using ST = StagedTile<M, V>;
-    static bool configured[64] = {};
-    int dev = 0;
-    TCB_CHECK_CUDA(cudaGetDevice(&dev));
-    if (!configured[dev & 63]) {
-        TCB_CHECK_CUDA(cudaFuncSetAttribute(mono_ionic_staged_kernel<M, V, MINB, Q>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ST::kBytes));
-        configured[dev & 63] = true;
+    static PerDevice<bool> configured;
+    const bool ok = configured.get([](bool& done, int) {
+        return done = cudaFuncSetAttribute(mono_ionic_staged_kernel<M, V, MINB, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)ST::kBytes) == cudaSuccess;
+    });
+    if (!ok) {
+        const cudaError_t e = cudaGetLastError();
+        return cuda_fail(e != cudaSuccess ? e : cudaErrorUnknown, "staged ionic kernel attributes");
     }
     const int64_t n_tiles = ceil_div(d.n_pad, ST::kTile);
     const int64_t grid = std::min<int64_t>(n_tiles, (int64_t)num_sms() * MINB);

@@ -519,19 +519,15 @@ __global__ void __launch_bounds__(kThreads, 1) mono_steps_kernel(MonoDev d, cons
 struct StepsInfo {
     int sms = 0, max_smem = 0;
 };
-const StepsInfo& steps_info() {
-    static StepsInfo infos[64];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    StepsInfo& si = infos[dev & 63];
-    if (si.sms == 0) {
-        cudaDeviceGetAttribute(&si.max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+StepsInfo steps_info() {
+    static PerDevice<StepsInfo> infos;
+    return infos.get([](StepsInfo& si, int dev) {
+        if (cudaDeviceGetAttribute(&si.max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&si.sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+            return false;
         si.max_smem -= (int)(sizeof(GridSums<kSums>) + sizeof(ClusterSums)) + 1024;
-        int sms = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        si.sms = sms;
-    }
-    return si;
+        return true;
+    });
 }
 
 constexpr int kMinSlices = 8;              // slices a block has at least
@@ -548,7 +544,7 @@ bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
 int64_t steps_blocks(const MonoDev& d, bool cluster) {
     const int64_t nb = std::max<int64_t>(ceil_div(d.n_slices, kMinSlices), 1);
-    if (!cluster) return std::min<int64_t>(nb, std::min(steps_info().sms, kSlots));
+    if (!cluster) return std::min<int64_t>(nb, std::max(1, std::min(steps_info().sms, kSlots)));
     int64_t p = 1;
     while (p < nb && p < kMaxCluster) p *= 2;
     return std::min(p, d.n_slices);
@@ -592,14 +588,15 @@ bool steps_plan(const tcb_mono* m, const MonoDev& d, bool ionic, int states, Ste
 
 template <typename IDX, bool ASPLIT, bool CL, class ION>
 int launch(const MonoDev& d, const IDX* col, const StepsPlan& pl, const ION& ion, cudaStream_t s) {
-    static bool configured[64] = {};
-    int dev = 0;
-    TCB_CHECK_CUDA(cudaGetDevice(&dev));
+    static PerDevice<bool> configured;
     const void* fn = (const void*)mono_steps_kernel<IDX, ASPLIT, CL, ION>;
-    if (!configured[dev & 63]) {
-        TCB_CHECK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, steps_info().max_smem));
-        if (CL) TCB_CHECK_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        configured[dev & 63] = true;
+    const bool ok = configured.get([fn](bool& done, int) {
+        return done = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, steps_info().max_smem) == cudaSuccess &&
+                      (!CL || cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess);
+    });
+    if (!ok) {
+        const cudaError_t e = cudaGetLastError();
+        return cuda_fail(e != cudaSuccess ? e : cudaErrorUnknown, "steps kernel attributes");
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)pl.blocks);
@@ -647,11 +644,8 @@ int launch_model(const tcb_mono* m, const MonoDev& d, const StepsPlan& pl, cudaS
 
 // whether the device takes a cluster of kMaxCluster blocks with all of the shared memory
 bool cluster_fits() {
-    static int fits[64] = {};   // 0 not asked yet, 1 yes, 2 no
-    int dev = 0;
-    cudaGetDevice(&dev);
-    int& f = fits[dev & 63];
-    if (f == 0) {
+    static PerDevice<bool> fits;
+    return fits.get([](bool& fit, int) {
         const void* fn = (const void*)mono_steps_kernel<int16_t, true, true, GivenRhs>;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(kMaxCluster);
@@ -664,13 +658,12 @@ bool cluster_fits() {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int clusters = 0;
-        const bool ok = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, steps_info().max_smem) == cudaSuccess &&
-                        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                        cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess && clusters >= 1;
-        if (!ok) cudaGetLastError();
-        f = ok ? 1 : 2;
-    }
-    return f == 1;
+        fit = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, steps_info().max_smem) == cudaSuccess &&
+              cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+              cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess && clusters >= 1;
+        if (!fit) cudaGetLastError();
+        return true;
+    });
 }
 
 }  // namespace
