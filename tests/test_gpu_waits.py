@@ -10,6 +10,10 @@ TCB_TEST_WAIT_STALL makes such a wait run out on purpose (limit 10 ms):
 of the batched CG kernel, the first block of the staged batched ionic kernel)
 unissued while their mbarrier still expects the bytes.  The tests check the reported
 status and that the next normal run on the same GPU is correct.
+
+The exception is the barrier of a thread-block cluster (persistent steps of the smallest
+meshes): the hardware's, without a limit, among blocks that the hardware starts together or not at
+all, so that none of them can be missing.  Under "grid" those meshes run as a grid.
 """
 import ctypes as C
 
@@ -61,6 +65,32 @@ def test_grid_barrier_timeout_is_reported(lib, cuda, tmp_path, monkeypatch, kern
     monkeypatch.delenv("TCB_TEST_WAIT_STALL")
     # the context is usable: a fresh solve on the same GPU is correct
     _clean_solve_matches_reference(case, d, cuda)
+
+
+@pytest.mark.parametrize("size", [6, 20])     # 343 nodes, a cluster's blocks as a grid; 9,261, a grid
+def test_grid_barrier_timeout_of_persistent_steps_is_reported(lib, cuda, monkeypatch, size):
+    """A stretch of steps in one launch whose grid barrier waits for an arrival that never comes: the
+    status, the step counter where it was, nothing run after it, and a clean run of the same
+    simulation set up anew."""
+    from tests.test_gpu_steps import _run, _sim as cube
+    from torchcor_b200 import _lib
+    sim = cube("cube", size, "ms", cuda)
+    ref = _run(sim, 1e-6, 100, True, 0, [7])
+    sim.prepare(1e-6, 1e-6, 100, snapshot_interval=sim.T)
+    st, counter = sim._sim["struct"], sim._sim["counter"]
+    sim.run_steps(2)
+    assert sim._sim["work"] is not None
+    assert lib.tcb_mono_check(C.byref(st), _lib.stream_ptr()) == 0 and int(counter[0].item()) == 3
+    monkeypatch.setenv("TCB_TEST_WAIT_STALL", "grid")
+    sim.run_steps(5)                                                     # the launch itself succeeds
+    assert lib.tcb_mono_check(C.byref(st), _lib.stream_ptr()) == _lib.TCB_ETIMEOUT
+    assert counter[:2].tolist() == [3, _lib.TCB_ETIMEOUT]
+    monkeypatch.delenv("TCB_TEST_WAIT_STALL")
+    _lib.check(lib.tcb_mono_run(C.byref(st), 3, 5, _lib.stream_ptr()))   # gives up at once: the error word is set
+    assert lib.tcb_mono_check(C.byref(st), _lib.stream_ptr()) == _lib.TCB_ETIMEOUT
+    assert counter[:2].tolist() == [3, _lib.TCB_ETIMEOUT]
+    again = _run(sim, 1e-6, 100, True, 0, [7])
+    assert all(bool((again[k] == ref[k]).all()) for k in ref)
 
 
 def test_bulk_copy_wait_timeout_is_reported(lib, cuda, tmp_path, monkeypatch):
