@@ -42,6 +42,8 @@ extern "C" {
 #define TCB_MODEL_TTP 2     /* TenTusscherPanfilov */
 #define TCB_MODEL_CRN 3     /* CourtemancheRamirezNattel */
 
+/* Of this header; a caller built against another one must not pass its structs.
+ * 2: tcb_mono ends in work and work_entries, and fused_step = 2 is the two launches. */
 int tcb_version(void);
 const char* tcb_status_string(int status);
 /* Copies the last error message of this thread into buf (truncated). */
@@ -220,12 +222,14 @@ typedef struct tcb_mono {
                                 and stim_bits aligned to the vector (else the first one-node instance runs) */
     int32_t cg_per_sm;       /* blocks per SM of the CG kernel that keeps rows in shared memory: 0 = the
                                 most whose rows fit (2, else 1); 1 or 2 pins it */
-    int32_t fused_step;      /* 1: each step is one launch, the ionic update fused into the CG kernel that
-                                keeps rows in shared memory (where that kernel applies: int16 column
-                                offsets, rows that fit); 2: the ionic and CG kernels as two launches;
-                                0: many steps in one persistent launch for meshes it suits (given `work`),
-                                else two launches.  The values are the same either way up to the order of
-                                the float64 sums */
+    int32_t fused_step;      /* 0: many steps in one persistent launch for meshes it suits (given `work`),
+                                else two launches; 2: the ionic and CG kernels as two launches; 1 (or any
+                                other value): each step is one launch, the ionic update fused into the CG
+                                kernel that keeps rows in shared memory (where that kernel applies: int16
+                                column offsets, rows that fit), else two launches.  The last two give the
+                                same values up to the compiler's multiply-add contractions; the persistent
+                                form also takes its float64 sums over unrounded products, in another order,
+                                and the residual from pairs of float32 (a relative 2^-46 before its rounding) */
     /* device bookkeeping (caller-allocated, zero-initialised) */
     int32_t* step_iters;     /* [nt+1] CG iterations of each step */
     int32_t* counter;        /* [4]: next step, error code, 2 spare */

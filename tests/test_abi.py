@@ -37,6 +37,13 @@ def test_status_strings(lib):
     assert lib.tcb_status_string(-3) == b"device wait timed out"
 
 
+def test_version_tells_the_longer_struct(lib):
+    """tcb_mono grew by two fields behind node_params: a caller built for version 1 can tell."""
+    from torchcor_b200 import _lib
+    assert [n for n, _ in _lib.tcb_mono._fields_][-3:] == ["node_params", "work", "work_entries"]
+    assert lib.tcb_version() == 2
+
+
 def test_struct_layout_matches_header(lib):
     from torchcor_b200 import _lib
     # the ctypes mirror must be as large as the C struct the library reads

@@ -89,6 +89,15 @@ def test_persistent_steps_match_single_launches(lib, cuda, mesh, size, model, to
     assert (a["at"] - b["at"]).abs().max().item() <= 0.0201 and (a["rt"] - b["rt"]).abs().max().item() <= 0.0201
 
 
+@pytest.mark.parametrize("fused_step,kernel", [(-1, 2), (0, 1), (1, 2), (2, 1), (3, 2)])
+def test_forms_of_a_single_step(lib, cuda, fused_step, kernel):
+    """2 asks for two launches; every other value but 0 for the fused one, as before there was a 2."""
+    sim = _sim("cube", 6, "ttp", cuda)
+    sim.prepare(1e-6, 1e-6, 100, snapshot_interval=sim.T)
+    sim.set_launch(fused_step=fused_step)
+    assert lib.tcb_mono_cg_kernel(C.byref(sim._sim["struct"])) == kernel
+
+
 def test_stretches_of_any_length_are_the_same(lib, cuda):
     """Where a launch begins and ends changes nothing, bit for bit: 145 steps at once
     (more than one launch's limit), and in stretches with and without the state held on chip."""

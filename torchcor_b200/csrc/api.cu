@@ -121,7 +121,7 @@ int validate_mono(const tcb_mono* m) { return validate(m); }
 
 using namespace tcb;
 
-extern "C" int tcb_version(void) { return 1; }
+extern "C" int tcb_version(void) { return 2; }
 
 extern "C" const char* tcb_status_string(int status) {
     switch (status) {

@@ -60,7 +60,7 @@ int launch_steps(const tcb_mono* m, const MonoDev& d, int64_t n_steps, bool ioni
 bool cg_forced_fallback();
 // 1 if tcb_mono_run runs this simulation's steps as the fused kernel
 inline int uses_fused_step(const tcb_mono* m, const MonoDev& d) {
-    return m->fused_step == 1 && !cg_forced_fallback() && mono_step_fusable(m, d);
+    return m->fused_step != 0 && m->fused_step != 2 && !cg_forced_fallback() && mono_step_fusable(m, d);
 }
 int cg_uses_resident(const MonoDev& d);
 

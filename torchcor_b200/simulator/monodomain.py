@@ -565,7 +565,9 @@ class Monodomain:
 
     def set_launch(self, ionic_variant=None, cg_per_sm=None, fused_step=None):
         """Set the prepared simulation's launch shapes: ionic kernel instance (1..,
-        0 = default), CG blocks per SM (0, 1, 2), fused step (0 or 1)."""
+        0 = default), CG blocks per SM (0, 1, 2), and the form of a step: fused_step 0
+        (default) runs stretches of steps as one launch where the mesh suits it, else two
+        launches a step; 1 one fused launch a step; 2 two launches a step."""
         m = self._sim["struct"]
         if ionic_variant is not None:
             m.ionic_variant = int(ionic_variant)
