@@ -112,3 +112,30 @@ def test_fused_step_matches_two_launches(lib, cuda, tmp_path, name):
         err = (a[k] - b[k]).abs().max().item() / a[k].abs().max().item()
         assert err <= tol, (k, err)
     assert (a["at_rt"] - b["at_rt"]).abs().max().item() <= case["dt"] * 1.001
+
+
+def test_tuner_times_the_stretches_that_run(lib, cuda, tmp_path):
+    """A mesh whose steps run as persistent launches: the tuner times those, with a buffer of its
+    own, under a key of its own; a launch pinned before stays where too few steps are left."""
+    from torchcor_b200 import tune
+    case = CS.case("cube8_ttp_f32")
+    sim = _prepared(case, case_mesh_dir(case, tmp_path), cuda)
+    sim.run_steps(4)
+    st, work = sim._sim["struct"], sim._sim["work"]
+    assert work is not None
+    torch.cuda.synchronize(cuda)
+    before = work.clone()
+    cache = tune.TuneCache(tmp_path / "tune.json")
+    key = tune.single_key(sim.device, int(st.n_nodes), int(sim.system.nnz), sim.ionic_model.name)
+    cache.put(key, {"ionic_variant": 2, "cg_per_sm": 2, "fused_step": 1})     # of a mesh of that size class launched step by step
+    got = tune.tune_single(sim, steps=4, cache=cache)
+    assert got["measured"] and sorted(got["step_ms"]) == ["stretch_fast0", "stretch_fast1"]
+    assert got["fused_step"] == st.fused_step == 0 and st.ionic_variant == got["ionic_variant"]
+    assert got["ionic_ms"][str(got["ionic_variant"])] == min(got["step_ms"].values())
+    assert torch.equal(work, before) and st.work == work.data_ptr()
+    st.ionic_variant, st.fused_step = 0, 2
+    again = tune.tune_single(sim, steps=4, cache=cache)
+    assert again["cached"] and again["fused_step"] == st.fused_step == 0 and st.ionic_variant == got["ionic_variant"]
+    st.fused_step = 2
+    few = tune.tune_single(sim, steps=10 ** 6, cache=cache, force=True)
+    assert not few["measured"] and few["fused_step"] == st.fused_step == 2

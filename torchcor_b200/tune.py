@@ -4,7 +4,9 @@ Single simulations (``tune_single``): the instance of the ionic kernel (1, 2
 or 4 consecutive nodes per thread, each compiled for a register budget of some
 blocks per SM and a division policy; ``_lib.ionic_variants``), the blocks per SM
 of the CG kernel that keeps rows in shared memory (1 or 2, where the rows fit),
-and whether a step runs as two launches or as the fused one.  Each
+and whether a step runs as two launches or as the fused one.  Where stretches of steps run
+as one persistent launch, which has the division policy alone from those, the
+candidates are the policies and what is timed is that launch.  Each
 candidate is timed with CUDA events on a scratch copy of the simulation's
 mutable device buffers, from the simulation's current step, so the simulation
 itself is untouched; the key is the device, the model and log2 buckets of the
@@ -198,6 +200,7 @@ class ScratchSim:
                                                             ("state", "x", "bp", "r", "p", "ap", "z", "p2"))
         m.at, m.rt = _lib.ptr(b["at_rt"][0]), _lib.ptr(b["at_rt"][1])
         m.snapshots, m.snap_ring = None, 0
+        m.work, m.work_entries = None, 0      # (the simulation's own; trials of stretches make theirs)
         m.step_iters, m.counter = _lib.ptr(b["step_iters"]), _lib.ptr(b["counter"])
         m.scratch, m.barrier = _lib.ptr(b["scratch"]), _lib.ptr(b["barrier"])
         self.struct = m
@@ -223,6 +226,25 @@ def time_steps(scratch, first, steps, stream):
     return mi.value / steps, mc.value / steps
 
 
+def time_stretch(scratch, first, steps, stream):
+    """ms a step over ``steps`` steps from ``first`` on the scratch copy in one call of
+    ``tcb_mono_run``: the best of three after an untimed one."""
+    import ctypes as C
+    from torchcor_b200 import _lib
+    lib = _lib.load()
+    ms = []
+    for _ in range(4):
+        scratch.reset()
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        e[0].record(stream)
+        _lib.check(lib.tcb_mono_run(C.byref(scratch.struct), first, first + steps, stream.cuda_stream))
+        e[1].record(stream)
+        _lib.check(lib.tcb_mono_check(C.byref(scratch.struct), stream.cuda_stream))
+        e[1].synchronize()
+        ms.append(e[0].elapsed_time(e[1]) / steps)
+    return min(ms[1:])
+
+
 def tune_single(sim, steps=5, cache=None, force=False):
     """Choose the ionic kernel instance and the CG blocks per SM for a prepared
     ``Monodomain`` (after ``prepare`` or ``_setup``) and set them in its tcb_mono.
@@ -237,17 +259,20 @@ def tune_single(sim, steps=5, cache=None, force=False):
     d = sim._sim
     m = d["struct"]
     model = sim.ionic_model
-    key = single_key(sim.device, int(m.n_nodes), int(sim.system.nnz), model.name)
-    hit = None if force else cache.get(key)
     shapes = _lib.ionic_variants(model.model_id)
     lib = _lib.load()
-    # where a stretch of steps is one persistent launch (tcb_mono.work), the fused step is no candidate
-    m.fused_step = 0
+    # whether a stretch of steps is one persistent launch (tcb_mono.work)
+    as_default = _lib.tcb_mono()
+    C.memmove(C.byref(as_default), C.byref(m), C.sizeof(m))
+    as_default.fused_step = 0
     slices = sim.system.host_slices
-    stretches = slices is not None and int(lib.tcb_mono_work_bytes_host(C.byref(m), _lib.ptr(slices), C.byref(C.c_int32()))) > 0
+    stretches = slices is not None and int(lib.tcb_mono_work_bytes_host(C.byref(as_default), _lib.ptr(slices),
+                                                                        C.byref(C.c_int32()))) > 0
+    key = single_key(sim.device, int(m.n_nodes), int(sim.system.nnz), model.name) + ("/stretches" if stretches else "")
+    hit = None if force else cache.get(key)
     if hit is not None and 0 <= int(hit.get("ionic_variant", 0)) <= len(shapes):
         m.ionic_variant, m.cg_per_sm = int(hit["ionic_variant"]), int(hit.get("cg_per_sm", 0))
-        m.fused_step = 0 if stretches else int(hit.get("fused_step", 0))
+        m.fused_step = int(hit.get("fused_step", 0))
         return dict(hit, cached=True)
     first = d["next_step"]
     if sim.nt + 1 - first < steps + 1:
@@ -255,6 +280,24 @@ def tune_single(sim, steps=5, cache=None, force=False):
                 "fused_step": int(m.fused_step), "measured": False}
     stream = torch.cuda.current_stream(sim.device)
     scratch = ScratchSim(sim)
+    if stretches:
+        from torchcor_b200.simulator.monodomain import _work_buffer
+        scratch.struct.fused_step, scratch.struct.cg_per_sm = 0, 0
+        scratch.buf["work"] = _work_buffer(scratch.struct, sim.system)
+        t_policy = {}
+        for k, shape in enumerate(shapes, 1):
+            if shape[2] not in t_policy:
+                scratch.struct.ionic_variant = k
+                t_policy[shape[2]] = time_stretch(scratch, first, steps, stream)
+        del scratch
+        ms = {k: t_policy[shape[2]] for k, shape in enumerate(shapes, 1)}   # an instance stands for its policy
+        best = min(ms, key=ms.get)
+        m.ionic_variant, m.cg_per_sm, m.fused_step = best, 0, 0
+        choice = {"ionic_variant": best, "cg_per_sm": 0, "fused_step": 0, "ionic_shape": list(shapes[best - 1]),
+                  "ionic_ms": {str(k): v for k, v in ms.items()},
+                  "step_ms": {f"stretch_fast{p}": v for p, v in t_policy.items()}}
+        cache.put(key, choice)
+        return dict(choice, measured=True)
     t_ion = {}
     for k in range(1, len(shapes) + 1):
         scratch.struct.ionic_variant, scratch.struct.cg_per_sm = k, 0
@@ -263,7 +306,7 @@ def tune_single(sim, steps=5, cache=None, force=False):
     # the step as two launches (ionic + CG) or as one (fused), for each CG blocks per SM
     t_step = {}
     for c in (2, 1):
-        for fused in (0,) if stretches else (0, 1):
+        for fused in (0, 1):
             st = scratch.struct
             st.ionic_variant, st.cg_per_sm, st.fused_step = best_ion, c, fused
             if lib.tcb_mono_cg_kernel(C.byref(st)) != (2 if fused else 1):   # not resident / not fusable
