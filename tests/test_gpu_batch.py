@@ -230,3 +230,55 @@ def test_batch_with_mixed_code_paths(lib, cuda, tmp_path):
     uniform.add(build(cases[0], dirs[0], cuda), 1e-5, 1e-5, 100)
     uniform.step(1)
     assert uniform._plan.cg_flags == 7
+
+
+def test_largest_batch_keeps_two_blocks_on_an_sm(lib, cuda):
+    """A plan for 1,024 simulations (one simulation's descriptor 1,024 times, never run): the default
+    CG variant has the blocks of two per SM, as a small batch of as many rows has."""
+    import ctypes as CT
+    from tests.test_gpu_steps import _sim
+    from torchcor_b200 import _lib
+    sim = _sim("cube", 8, "ms", cuda)
+    sim.prepare(1e-5, 1e-5, 100, snapshot_interval=sim.T)
+    sms = torch.cuda.get_device_properties(cuda).multi_processor_count
+    for n in (1024, 825, 500):
+        arr = (_lib.tcb_mono * n)(*[sim._sim["struct"]] * n)
+        ws = torch.empty(int(lib.tcb_batch_workspace_bytes(n)), dtype=torch.uint8, device=cuda)
+        plan = _lib.tcb_batch_plan()
+        _lib.check(lib.tcb_batch_prepare(arr, n, ws.data_ptr(), ws.numel(), CT.byref(plan)))
+        assert plan.total_slices >= 64 * sms          # enough rows for every block
+        assert (plan.cg_variant, plan.cg_blocks) == (2, 2 * sms), n
+        assert plan.cg_stage_ok
+
+
+@pytest.mark.parametrize("variant", [2, 1, 3])
+def test_more_simulations_than_a_block_stages(lib, cuda, variant):
+    """70 simulations, 64 of which a block holds at once: views are staged by every sweep, and the
+    limits of the last six, far from the others', are read from their descriptors.  Against
+    each simulation alone, launched step by step: bounds as in the tests of stretches of steps
+    (sums in another order), iteration counts equal."""
+    from tests.test_gpu_steps import _run, _sim
+    from torchcor_b200.simulator import MonodomainBatch
+    steps = 30
+    kinds = [("cube", 5, "ms"), ("cube", 7, "ttp"), ("ico", 2, "ms")]
+    limits = lambda k: (1e-6, 100) if k < 64 else ((1e-2, 100) if k % 2 else (1e-7, 1))
+    alone = {}
+    for k in range(70):
+        what = (kinds[k % 3], limits(k))
+        if what not in alone:
+            s = _sim(*what[0], cuda, steps=steps)
+            alone[what] = _run(s, what[1][0], what[1][1], True, 2, [steps])
+    batch = MonodomainBatch(cuda, max_sims=70)
+    for k in range(70):
+        s = _sim(*kinds[k % 3], cuda, steps=steps)
+        tol, most = limits(k)
+        batch.add(s, tol, tol, most, snapshot_interval=s.T)
+    batch.set_cg(variant)
+    batch.step(steps)
+    batch.check()
+    for k, s in enumerate(batch.sims):
+        ref = alone[kinds[k % 3], limits(k)]
+        d = s._sim
+        assert torch.equal(d["step_iters"], ref["iters"]), k
+        err = (d["x"][:, : s.n_nodes] - ref["x"]).abs().max().item() / ref["x"].abs().max().item()
+        assert err <= steps * 2.0 ** -23, (k, err)

@@ -312,12 +312,13 @@ struct ApStreams {
 
 struct BatchShared {
     double *rz, *zz, *bn, *al, *be;   // [n] per simulation
-    double *at, *rt;             // [n] tolerances
+    double *at, *rt;             // tolerances of the first kBatchMaxPerBlock simulations
     double* wp;                  // [warps][kBatchMaxPerBlock][3] warp partials of the staged simulations
     int64_t* pre;                // [n+1] prefix of the active simulations' slice counts
     int64_t* bb;                 // [nb+1] first virtual slice of each block
     CgView* cg;                  // [kBatchMaxPerBlock] staged views
-    int *it, *act, *step, *ns, *most;   // [n]; act: 0 done, 1 iterating, 2 in its last pass; most: max_iter
+    int *it, *act, *step, *ns;   // [n]; act: 0 done, 1 iterating, 2 in its last pass
+    int* most;                   // max_iter of the first kBatchMaxPerBlock simulations
     int *w0, *w1;                // [n] first and last block holding each active simulation's slices
 };
 
@@ -329,8 +330,8 @@ __device__ __forceinline__ BatchShared carve(double* smd, int n, int nb) {
     s.al = s.bn + n;
     s.be = s.al + n;
     s.at = s.be + n;
-    s.rt = s.at + n;
-    s.wp = s.rt + n;
+    s.rt = s.at + kBatchMaxPerBlock;
+    s.wp = s.rt + kBatchMaxPerBlock;
     s.pre = reinterpret_cast<int64_t*>(s.wp + kCgWarps * kBatchMaxPerBlock * 3);
     s.bb = s.pre + n + 1;
     s.cg = reinterpret_cast<CgView*>(s.bb + nb + 1);
@@ -339,7 +340,7 @@ __device__ __forceinline__ BatchShared carve(double* smd, int n, int nb) {
     s.step = s.act + n;
     s.ns = s.step + n;
     s.most = s.ns + n;
-    s.w0 = s.most + n;
+    s.w0 = s.most + kBatchMaxPerBlock;
     s.w1 = s.w0 + n;
     return s;
 }
@@ -745,12 +746,17 @@ __device__ __forceinline__ void totals(BatchShared& S, int n, const double* part
     __syncthreads();
 }
 
-// bytes of the shared carve-out before the staging area (128-byte aligned)
+// Bytes of the shared carve-out before the staging area (128-byte aligned): 72 a simulation beside
+// 41 KB, so that two blocks of the largest batch (1,024 simulations, 112 KB) fit on an SM.
 __host__ __device__ inline size_t carve_bytes(int n) {
-    const size_t b = (size_t)n * (7 * sizeof(double) + 7 * sizeof(int)) +
+    const size_t b = (size_t)n * (5 * sizeof(double) + 6 * sizeof(int)) +
+                     (size_t)kBatchMaxPerBlock * (2 * sizeof(double) + sizeof(int)) +
                      sizeof(double) * kCgWarps * kBatchMaxPerBlock * 3 + sizeof(int64_t) * (n + 1) +
                      sizeof(int64_t) * (kBatchMaxBlocks + 1) + sizeof(CgView) * kBatchMaxPerBlock;
     return (b + 127) / 128 * 128;
+}
+__device__ __forceinline__ int max_iter(const BatchWS* W, const BatchShared& S, int i) {
+    return i < kBatchMaxPerBlock ? S.most[i] : W->dev[i].max_iter;
 }
 constexpr size_t kStageBarBytes = 128 * ((kCgWarps * kStages * 8 + 127) / 128);
 
@@ -794,9 +800,11 @@ __global__ void __launch_bounds__(kCgThreads, PER_SM) batch_cg_kernel(const Batc
         const MonoDev& d = W->dev[i];
         const int64_t st = d.counter[0];
         S.step[i] = (st >= 1 && st <= d.nt) ? (int)st : 0;   // 0 = not stepping
-        S.at[i] = d.a_tol;
-        S.rt[i] = d.r_tol;
-        S.most[i] = d.max_iter;
+        if (i < kBatchMaxPerBlock) {
+            S.at[i] = d.a_tol;
+            S.rt[i] = d.r_tol;
+            S.most[i] = d.max_iter;
+        }
         S.ns[i] = W->slices[i];
         S.act[i] = 0;
         S.it[i] = 0;
@@ -835,7 +843,7 @@ __global__ void __launch_bounds__(kCgThreads, PER_SM) batch_cg_kernel(const Batc
         S.rz[i] = t[1];
         S.zz[i] = t[2];
         S.be[i] = 0.0;
-        S.act[i] = S.most[i] > 0;
+        S.act[i] = max_iter(W, S, i) > 0;
     });
 
     for (int pass = 0;; ++pass) {
@@ -879,7 +887,9 @@ __global__ void __launch_bounds__(kCgThreads, PER_SM) batch_cg_kernel(const Batc
             const double zz1 = S.zz[i] - alpha * (2.0 * t[1] - alpha * t[2]);
             const double zn = sqrt(zz1 < 0.0 ? 0.0 : zz1);
             S.al[i] = alpha;
-            if (zn < S.at[i] || zn < S.rt[i] * S.bn[i]) S.act[i] = 2;
+            const bool held = i < kBatchMaxPerBlock;
+            const double at = held ? S.at[i] : W->dev[i].a_tol, rt = held ? S.rt[i] : W->dev[i].r_tol;
+            if (zn < at || zn < rt * S.bn[i]) S.act[i] = 2;
         });
 
         // ---- x += alpha p, r -= alpha Ap, z = D r; r.z, z.z
@@ -913,7 +923,7 @@ __global__ void __launch_bounds__(kCgThreads, PER_SM) batch_cg_kernel(const Batc
             S.rz[i] = t[0];
             S.zz[i] = t[1];
             S.it[i] += 1;
-            if (S.it[i] >= S.most[i]) S.act[i] = 0;
+            if (S.it[i] >= max_iter(W, S, i)) S.act[i] = 0;
         });
     }
     // block 0 records the iterations and advances the step counters (every
