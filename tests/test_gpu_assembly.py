@@ -165,3 +165,34 @@ def test_gather_of_the_last_contributions_below_2_31(lib, cuda, k):
     assert np.array_equal(out.cpu().numpy(), want)
     del slot_src
     torch.cuda.empty_cache()
+
+
+def test_element_matrices_divide_by_the_determinant(lib, cuda):
+    """Tetrahedra on the axes with edges 1, 2, m: the gradient along the first is (2 m) / (2 m) = 1 and
+    K[1][1] = volume * sigma is half way between two float32 values, so that it rounds to the even one
+    only if the quotient is rounded once.  The determinants are those for which the product with
+    the reciprocal is below 1."""
+    from torchcor_b200._lib import check, ptr, stream_ptr
+    dets, sigma = [], []
+    for det in range(12, 60000, 12):                      # volume det / 6, m = det / 2
+        if float(det) * (1.0 / det) >= 1.0:
+            continue
+        for j in range(1, 256):
+            s = 1.0 + j * 2.0 ** -23
+            v = det / 6 * s                               # exact: 13 and 24 bits
+            below = v * (1 - 2.0 ** -53)
+            if np.float32(v) > np.float32(below):
+                dets.append(det)
+                sigma.append(s)
+                break
+    E = len(dets)
+    assert E >= 20
+    nodes = np.zeros((E, 4, 3), dtype=np.float32)
+    nodes[:, 1, 0], nodes[:, 2, 1], nodes[:, 3, 2] = 1, 2, np.array(dets) / 2
+    elems = np.arange(4 * E, dtype=np.int32).reshape(E, 4)
+    fib = np.tile(np.array([1, 0, 0], dtype=np.float32), (E, 1))
+    d = [torch.from_numpy(a).to(cuda) for a in (nodes.reshape(-1, 3), elems, np.array(sigma, dtype=np.float32), fib)]
+    ke, mw = torch.empty((E, 16), device=cuda), torch.empty(E, device=cuda)
+    check(lib.tcb_assemble_local(4, ptr(d[0]), ptr(d[1]), E, ptr(d[2]), ptr(d[2]), ptr(d[3]), ptr(ke), ptr(mw), stream_ptr()))
+    want = (np.array(dets) / 6 * np.array(sigma)).astype(np.float32)
+    assert np.array_equal(ke[:, 5].cpu().numpy(), want)

@@ -50,18 +50,18 @@ __global__ void tet_local_kernel(const float* __restrict__ nodes, const int32_t*
     double C01 = J[1][2] * J[2][0] - J[1][0] * J[2][2];
     double C02 = J[1][0] * J[2][1] - J[1][1] * J[2][0];
     double det = J[0][0] * C00 + J[0][1] * C01 + J[0][2] * C02;
-    // inverse = adj / det
-    const double rdet = 1.0 / det;
+    // inverse = adj / det (nine divisions: the products with one reciprocal, rounded once more each, were
+    // 25 us faster at 3.1 million elements and moved 2 of 31 million values of K by an ulp)
     double inv[3][3];
-    inv[0][0] = C00 * rdet;
-    inv[1][0] = C01 * rdet;
-    inv[2][0] = C02 * rdet;
-    inv[0][1] = (J[0][2] * J[2][1] - J[0][1] * J[2][2]) * rdet;
-    inv[1][1] = (J[0][0] * J[2][2] - J[0][2] * J[2][0]) * rdet;
-    inv[2][1] = (J[0][1] * J[2][0] - J[0][0] * J[2][1]) * rdet;
-    inv[0][2] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) * rdet;
-    inv[1][2] = (J[0][2] * J[1][0] - J[0][0] * J[1][2]) * rdet;
-    inv[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * rdet;
+    inv[0][0] = C00 / det;
+    inv[1][0] = C01 / det;
+    inv[2][0] = C02 / det;
+    inv[0][1] = (J[0][2] * J[2][1] - J[0][1] * J[2][2]) / det;
+    inv[1][1] = (J[0][0] * J[2][2] - J[0][2] * J[2][0]) / det;
+    inv[2][1] = (J[0][1] * J[2][0] - J[0][0] * J[2][1]) / det;
+    inv[0][2] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) / det;
+    inv[1][2] = (J[0][2] * J[1][0] - J[0][0] * J[1][2]) / det;
+    inv[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) / det;
     // G = dN @ inv(J): row 0 = -(sum of rows), row a = inv row a-1
     double G[4][3];
     for (int c = 0; c < 3; ++c) {
