@@ -250,3 +250,32 @@ def test_first_calls_from_several_threads(lib, cuda):
     root = Path(__file__).resolve().parent.parent
     r = subprocess.run([sys.executable, "-c", FIRST_CALLS], cwd=root, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "same" in r.stdout, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("mesh,size,model,tol", [("cube", 20, "ms", 1e-8), ("cube", 12, "ttp", 1e-8), ("ico", 4, "crn", 1e-8),
+                                                 ("cube", 20, "ttp", 1e-5), ("ico", 5, "ms", 1e-6)])
+def test_every_stopping_test_ends_the_same_iterations(lib, cuda, monkeypatch, mesh, size, model, tol):
+    """The streaming kernel sums |z'|^2 itself; the resident, the batched and the persistent kernels
+    take it from the sums of the pass before (over z and w = D A p rounded to float32 in the
+    first two).  Where a pass leaves 1e-3 of |z| that is right to about 1e-4 of it: the kernels stop
+    at the same iteration in every step, tight tolerances and many passes a step included."""
+    from torchcor_b200.simulator import MonodomainBatch
+    steps = 60
+    sim = _sim(mesh, size, model, cuda, steps=steps)
+    iters = {"stretch": _run(sim, tol, 100, False, 0, [steps])["iters"],
+             "resident": _run(sim, tol, 100, False, 2, [steps])["iters"],
+             "fused": _run(sim, tol, 100, False, 1, [steps])["iters"]}
+    for variant in (1, 2, 3):
+        sim._sim = None
+        batch = MonodomainBatch(cuda, max_sims=1)
+        batch.add(sim, tol, tol, 100, linear_guess=False, snapshot_interval=sim.T)
+        batch.set_cg(variant)
+        batch.step(steps)
+        batch.check()
+        iters[f"batch{variant}"] = sim._sim["step_iters"].clone()
+    monkeypatch.setenv("TCB_CG_KERNEL", "streaming")
+    want = _run(sim, tol, 100, False, 2, [steps])["iters"]
+    if tol < 1e-7:
+        assert want.max().item() >= 4          # several passes a step
+    for name, got in iters.items():
+        assert torch.equal(got, want), (name, (got - want).nonzero().tolist())
