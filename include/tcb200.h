@@ -82,7 +82,8 @@ int tcb_sell_layout_device(const int32_t* rowptr, int64_t n_rows, int64_t* slice
  * parse exactly are counted in *bad (device int64, caller-zeroed).
  * Pattern: tcb_pattern_device with work = 2*(N+1) int64, keys = k*k*E uint64,
  * iwork = 2*N+1 int32 returns nnz; tcb_pattern_device_emit writes the same arrays
- * as tcb_pattern_build (device pointers).  slot_src may be the first k*k*E int32 of
+ * as tcb_pattern_build (device pointers; a node in no element, which that call refuses, gets an empty
+ * row and -1 for its diagonal slot).  slot_src may be the first k*k*E int32 of
  * keys, where the first call leaves it: nothing is copied then. */
 int64_t tcb_text_scratch(int64_t n_bytes);
 int tcb_text_newlines(const char* text, int64_t n_bytes, int64_t* scratch, int64_t* pos, int64_t cap, int64_t* count,
@@ -112,7 +113,7 @@ int tcb_assemble_gather(int32_t k, const int32_t* slot_ptr, const int32_t* slot_
                         const float* ke, const float* mw, float* k_val, float* m_val, void* stream);
 /* Monodomain.assemble system values (monodomain.py:93-106, preconditioner.py:9-27):
  * k_val /= chi (in place); a_val = m*cm + (k*dt)*theta; k_rhs = ((1-theta)*dt)*k;
- * d_inv[i] = 1/a(i,i) (0 for i >= n_nodes up to n_pad).  *a_split (device int32, caller sets 1)
+ * d_inv[i] = 1/a(i,i) (0 for i >= n_nodes up to n_pad, and where diag[i] < 0).  *a_split (device int32, caller sets 1)
  * is cleared if any a_val differs from fp32(fp32(m*cm) + k_rhs); it stays 1 for theta = 0.5, and the
  * solver then rebuilds A from M and k_rhs instead of streaming it. */
 int tcb_assemble_system(int64_t nnz, int64_t n_nodes, int64_t n_pad, const int32_t* diag, float* k_val,
@@ -125,7 +126,7 @@ int tcb_assemble_system(int64_t nnz, int64_t n_nodes, int64_t n_pad, const int32
 int tcb_sell_delta(int64_t n_rows, const int64_t* slice_ptr, int64_t n_slices, const int32_t* sell_col,
                    int16_t* delta, int32_t* max_abs, void* stream);
 /* Repack up to 4 CSR value arrays (and the columns) into sliced ELL; padding
- * entries get column = own row and value 0. */
+ * entries get column = own row and value 0, in the rows past n_rows of the last slice column 0. */
 int tcb_sell_pack(int64_t n_rows, const int32_t* rowptr, const int32_t* col, const int64_t* slice_ptr,
                   int64_t n_slices, int32_t n_vals, const float* const* vals /* host array of device ptrs */,
                   int32_t* sell_col, float* const* sell_vals, void* stream);
@@ -181,7 +182,8 @@ int tcb_model_differentiate(int32_t model, const double* params, const float* ta
 typedef struct tcb_mono {
     int64_t n_nodes, n_pad, n_slices, nt;
     int32_t model, n_states;
-    /* matrix (sliced ELL, TCB_SLICE rows per slice) */
+    /* matrix (sliced ELL, TCB_SLICE rows per slice; every entry of a slice, those of rows past n_nodes
+     * too, has a column of an existing row, as tcb_sell_pack and tcb_sell_delta write them) */
     const int64_t* slice_ptr;
     const int32_t* col;
     const int16_t* col_delta; /* optional: col - row as int16 (all |col-row| < 32768), or NULL */

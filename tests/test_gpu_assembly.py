@@ -196,3 +196,28 @@ def test_element_matrices_divide_by_the_determinant(lib, cuda):
     check(lib.tcb_assemble_local(4, ptr(d[0]), ptr(d[1]), E, ptr(d[2]), ptr(d[2]), ptr(d[3]), ptr(ke), ptr(mw), stream_ptr()))
     want = (np.array(dets) / 6 * np.array(sigma)).astype(np.float32)
     assert np.array_equal(ke[:, 5].cpu().numpy(), want)
+
+
+def test_nodes_in_no_element_on_the_device(lib, cuda):
+    """The device pattern takes nodes that no element has: empty rows, -1 for the diagonal slot, 0 for
+    the preconditioner; the other nodes' values are those of the mesh without them."""
+    from torchcor_b200 import meshgen
+    from torchcor_b200.core.assemble import assemble_system, build_pattern_device
+    nodes, elems = meshgen.cube(5, 0.25)
+    n, gaps = len(nodes), [0, 40, 41, 216]
+    keep = np.setdiff1d(np.arange(n + len(gaps)), gaps)
+    wide = np.zeros((n + len(gaps), 3), dtype=np.float32)
+    wide[keep] = nodes
+    spread = keep[elems].astype(np.int32)
+    pat = build_pattern_device(torch.from_numpy(spread).to(cuda), len(wide))
+    assert (pat.host("diag")[gaps] == -1).all() and (np.diff(pat.host("rowptr"))[gaps] == 0).all()
+    assert (pat.host("col")[pat.host("diag")[keep]] == keep).all()
+    fib = torch.tensor([[1.0, 0, 0]], device=cuda).repeat(len(elems), 1).contiguous()
+    s = torch.full((len(elems),), 0.3, device=cuda)
+    def system(x, el):
+        return assemble_system(torch.from_numpy(np.ascontiguousarray(x, dtype=np.float32)).to(cuda),
+                               torch.from_numpy(np.ascontiguousarray(el, dtype=np.int32)).to(cuda), s, s, fib, 0.01)
+    a, b = system(wide, spread), system(nodes, elems)
+    assert (a.d_inv[gaps] == 0).all()
+    assert torch.equal(a.d_inv[torch.from_numpy(keep).to(cuda)], b.d_inv[:n])
+    assert torch.equal(a.a_val, b.a_val) and torch.equal(a.k_val, b.k_val)

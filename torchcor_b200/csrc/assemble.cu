@@ -238,7 +238,8 @@ __global__ void jacobi_kernel(int64_t n, int64_t n_pad, const int32_t* __restric
                               const float* __restrict__ aval, float* __restrict__ dinv) {
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_pad) return;
-    dinv[i] = i < n ? __fdiv_rn(1.0f, aval[diag[i]]) : 0.0f;   // preconditioner.py:27
+    const int32_t s = i < n ? diag[i] : -1;
+    dinv[i] = s >= 0 ? __fdiv_rn(1.0f, aval[s]) : 0.0f;   // preconditioner.py:27; 0 for a node in no element
 }
 
 struct SellVals {

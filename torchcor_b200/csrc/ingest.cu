@@ -668,6 +668,7 @@ __global__ void __launch_bounds__(256) pattern_emit_kernel(const int64_t* __rest
     const int64_t b = row_off[row], w = rowptr64[row];
     const int u = (int)(rowptr64[row + 1] - w);
     if (lane == 0) rowptr[row] = (int32_t)w;
+    if (u == 0 && lane == 0) diag[row] = -1;   // a node in no element
     bool flagged = false;
     for (int i = lane; i < u; i += 16) {
         const uint32_t v = list[b + i];
