@@ -71,6 +71,9 @@ int tcb_sell_layout(const int32_t* rowptr, int64_t n_rows, int64_t* slice_ptr, i
 int64_t tcb_sell_layout_scratch(int64_t n_rows);
 int tcb_sell_layout_device(const int32_t* rowptr, int64_t n_rows, int64_t* slice_ptr, int64_t* scratch,
                            int64_t* n_entries, void* stream);
+/* The same with all n_slices + 1 offsets on the host too, the last of them the entries. */
+int tcb_sell_layout_both(const int32_t* rowptr, int64_t n_rows, int64_t* slice_ptr, int64_t* scratch,
+                         int64_t* host_slice_ptr, void* stream);
 
 /* ---------------------------------------------------------------- device ingest
  * Mesh ingest on the device (replaces MeshReader's np.loadtxt, mesh.py:26-63, and

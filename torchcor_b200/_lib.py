@@ -83,6 +83,7 @@ SIGNATURES = [
     ("tcb_sell_layout", C.c_int, [_vp, _i64, _vp, _pi64]),
     ("tcb_sell_layout_scratch", _i64, [_i64]),
     ("tcb_sell_layout_device", C.c_int, [_vp, _i64, _vp, _vp, _pi64, _vp]),
+    ("tcb_sell_layout_both", C.c_int, [_vp, _i64, _vp, _vp, _vp, _vp]),
     ("tcb_assemble_local", C.c_int, [_i32, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp]),
     ("tcb_assemble_gather", C.c_int, [_i32, _vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp]),
     ("tcb_assemble_system", C.c_int, [_i64, _i64, _i64, _vp, _vp, _vp, _f64, _f64, _f64, _f64, _vp, _vp, _vp, _vp,

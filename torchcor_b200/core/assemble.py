@@ -1,7 +1,7 @@
 """P1 assembly on the device (the role of ``torchcor/core/assemble.py``).
 
-``assemble_system`` builds, for one mesh, the CSR pattern and scatter map (host
-C++), the element matrices (one thread per element), the deterministic
+``assemble_system`` builds, for one mesh, the CSR pattern and scatter map (on the
+device for elements there, else and for rows beyond its limits in host C++), the element matrices (one thread per element), the deterministic
 slot-ordered sums into CSR values, the monodomain system values and the
 sliced-ELL copy the solver streams.  ``Matrices3D`` / ``Matrices3DSurface``
 keep the reference's class names and return (K, M) as sparse CSR tensors.
@@ -156,7 +156,7 @@ HOST_SLICES = 1 << 14
 def _sliced_ell(pat, rowptr, col, values, dev, flag=None):
     """Sliced-ELL copy of CSR values on the device: (n_slices, slice_ptr, columns, int16
     column offsets or None, [values...], flag as a bool).  ``flag``: an int32 device scalar read in
-    the same copy as the width of the columns."""
+    the same synchronisation as the width of the columns."""
     return _sliced_ell_host(pat, rowptr, col, values, dev, flag)[:-1]
 
 
@@ -166,13 +166,16 @@ def _sliced_ell_host(pat, rowptr, col, values, dev, flag=None):
     s = stream_ptr()
     n = pat.n_nodes
     n_slices = (n + _lib.TCB_SLICE - 1) // _lib.TCB_SLICE
-    # the two flags behind the offsets: one copy to the host for all of them
-    ends = torch.empty(n_slices + 2, device=dev, dtype=torch.int64)
-    slice_ptr, flags = ends[:n_slices + 1], ends[n_slices + 1:].view(torch.int32)
+    slice_ptr = torch.empty(n_slices + 1, device=dev, dtype=torch.int64)
     scratch = torch.empty(int(lib.tcb_sell_layout_scratch(n)), device=dev, dtype=torch.int64)
-    n_entries = C.c_int64()
-    check(lib.tcb_sell_layout_device(ptr(rowptr), n, ptr(slice_ptr), ptr(scratch), C.byref(n_entries), s))
-    ne = n_entries.value
+    host = np.empty(n_slices + 1, dtype=np.int64) if n_slices <= HOST_SLICES else None
+    if host is not None:
+        check(lib.tcb_sell_layout_both(ptr(rowptr), n, ptr(slice_ptr), ptr(scratch), ptr(host), s))
+        ne = int(host[-1])
+    else:
+        n_entries = C.c_int64()
+        check(lib.tcb_sell_layout_device(ptr(rowptr), n, ptr(slice_ptr), ptr(scratch), C.byref(n_entries), s))
+        ne = n_entries.value
     sell_col = torch.empty(ne, device=dev, dtype=torch.int32)
     sell = [torch.empty(ne, device=dev, dtype=torch.float32) for _ in values]
     vin = (C.c_void_p * len(values))(*[ptr(t) for t in values])
@@ -180,15 +183,12 @@ def _sliced_ell_host(pat, rowptr, col, values, dev, flag=None):
     check(lib.tcb_sell_pack(n, ptr(rowptr), ptr(col), ptr(slice_ptr), n_slices, len(values), vin, ptr(sell_col), vout, s))
     # int16 column offsets when the mesh ordering keeps every |col - row| < 32768
     dcol = torch.empty(ne, device=dev, dtype=torch.int16)
-    flags.zero_()
+    flags = torch.zeros(2, device=dev, dtype=torch.int32)
     check(lib.tcb_sell_delta(n, ptr(slice_ptr), n_slices, ptr(sell_col), ptr(dcol), ptr(flags), s))
     if flag is not None:
         flags[1:] = flag
-    small = n_slices <= HOST_SLICES
-    host = (ends if small else ends[n_slices + 1:]).cpu().numpy()
-    width, flag = host[-1:].view(np.int32).tolist()
-    return (n_slices, slice_ptr, sell_col, dcol if width < 32768 else None, sell, bool(flag),
-            host[:-1] if small else None)
+    width, flag = flags.tolist()
+    return n_slices, slice_ptr, sell_col, dcol if width < 32768 else None, sell, bool(flag), host
 
 
 def assemble_system(nodes, elems_np, sl, st, fibres, dt, chi=140, cm=0.01, theta=0.5, pattern=None) -> System:

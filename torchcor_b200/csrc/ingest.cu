@@ -830,17 +830,29 @@ extern "C" int64_t tcb_sell_layout_scratch(int64_t n_rows) {
     return scan_tiles(ns) + 1;
 }
 
-extern "C" int tcb_sell_layout_device(const int32_t* rowptr, int64_t n_rows, int64_t* slice_ptr, int64_t* scratch,
-                                      int64_t* n_entries, void* stream) {
-    if (!rowptr || !slice_ptr || !scratch || !n_entries || n_rows <= 0)
-        return fail(TCB_EINVAL, "tcb_sell_layout_device: bad arguments");
-    cudaStream_t s = as_stream(stream);
+// `host` gets the last `n_host` of the offsets (synchronises the stream)
+static int sell_layout(const int32_t* rowptr, int64_t n_rows, int64_t* slice_ptr, int64_t* scratch, int64_t* host, int64_t n_host,
+                       cudaStream_t s) {
     const int64_t ns = ceil_div(n_rows, TCB_SLICE);
     slice_width_kernel<<<blocks(ns, 8), 256, 0, s>>>(rowptr, n_rows, ns, slice_ptr);
     TCB_CHECK_LAUNCH("slice width kernel");
     const int st = scan(slice_ptr, slice_ptr, ns, TCB_SLICE, slice_ptr + ns, scratch, s);
     if (st) return st;
-    TCB_CHECK_CUDA(cudaMemcpyAsync(n_entries, slice_ptr + ns, sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+    TCB_CHECK_CUDA(cudaMemcpyAsync(host, slice_ptr + ns + 1 - n_host, n_host * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     TCB_CHECK_CUDA(cudaStreamSynchronize(s));
     return TCB_OK;
+}
+
+extern "C" int tcb_sell_layout_device(const int32_t* rowptr, int64_t n_rows, int64_t* slice_ptr, int64_t* scratch,
+                                      int64_t* n_entries, void* stream) {
+    if (!rowptr || !slice_ptr || !scratch || !n_entries || n_rows <= 0)
+        return fail(TCB_EINVAL, "tcb_sell_layout_device: bad arguments");
+    return sell_layout(rowptr, n_rows, slice_ptr, scratch, n_entries, 1, as_stream(stream));
+}
+
+extern "C" int tcb_sell_layout_both(const int32_t* rowptr, int64_t n_rows, int64_t* slice_ptr, int64_t* scratch,
+                                    int64_t* host_slice_ptr, void* stream) {
+    if (!rowptr || !slice_ptr || !scratch || !host_slice_ptr || n_rows <= 0)
+        return fail(TCB_EINVAL, "tcb_sell_layout_both: bad arguments");
+    return sell_layout(rowptr, n_rows, slice_ptr, scratch, host_slice_ptr, ceil_div(n_rows, TCB_SLICE) + 1, as_stream(stream));
 }
