@@ -295,9 +295,10 @@ def test_misaligned_tables_rejected_before_any_launch(lib):
 
 
 def test_misaligned_barrier_words_rejected_before_any_launch(lib):
-    """The CG kernels' grid barrier keeps its count and generation in one 64-bit
-    word: barrier words that are not 8-byte aligned are refused on the host, before
-    any device access (fake addresses are enough)."""
+    """The CG kernels' grid barrier counts arrivals and keeps their number between
+    launches in two 32-bit words of the caller's: barrier words that are not 8-byte
+    aligned are refused on the host, before any device access (fake addresses are
+    enough)."""
     import ctypes
     from torchcor_b200 import _lib
     m = _lib.tcb_mono()

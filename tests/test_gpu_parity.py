@@ -165,10 +165,11 @@ def test_monodomain_matches_reference(lib, cuda, name, tmp_path, launch=None):
     assert abs(total - ref_total) <= max(3, ref_total // 50), (total, ref_total)
 
 
-@pytest.mark.parametrize("fused", [0, 1])
+@pytest.mark.parametrize("fused", [0, 1, 2])
 @pytest.mark.parametrize("name", TISSUE)
 def test_monodomain_step_launches(lib, cuda, name, tmp_path, fused):
-    """The step as two launches and as one fused launch, both against the reference."""
+    """Stretches of steps as one launch (0; these meshes suit it), the step as one fused launch (1) and as
+    two launches (2), each against the reference."""
     test_monodomain_matches_reference(lib, cuda, name, tmp_path, launch=dict(fused_step=fused))
 
 

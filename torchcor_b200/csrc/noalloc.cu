@@ -29,10 +29,10 @@ namespace tcb {
 int validate_mono(const tcb_mono* m);
 namespace {
 
-// Both CG kernels place their second partial buffer at scratch + 2 * cgk::kMaxBlocks
-// whatever the block count, so the array is sized from that constant.
+// The streaming CG kernel places its second partial buffer at scratch + 2 * cgk::kMaxBlocks whatever the
+// block count (the resident one uses less), so the array is sized from that constant.
 constexpr int kNoAllocMaxBlocks = cgk::kMaxBlocks;
-constexpr int kPartials = 4 * kNoAllocMaxBlocks;   // doubles: two parity buffers x 2 values x blocks
+constexpr int kPartials = 4 * kNoAllocMaxBlocks;   // doubles: two buffers x 2 values x blocks
 static_assert(kPartials == 4 * cgk::kMaxBlocks, "static scratch must hold what tcb_mono_scratch_doubles() asks for");
 constexpr int kBarrierWords = 4;
 
