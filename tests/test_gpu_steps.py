@@ -279,3 +279,31 @@ def test_every_stopping_test_ends_the_same_iterations(lib, cuda, monkeypatch, me
         assert want.max().item() >= 4          # several passes a step
     for name, got in iters.items():
         assert torch.equal(got, want), (name, (got - want).nonzero().tolist())
+
+
+def test_exchange_buffer_made_beside_outlives_steps_on_the_current_stream(lib, cuda):
+    """First steps on a stream of the caller's, more behind other work on the current one, then the
+    buffer is dropped: its memory is not handed out on the first stream while the steps are pending."""
+    sim = _sim("cube", 20, "ttp", cuda)
+    ref = _run(sim, 1e-6, 100, True, 0, [20])
+    sim.prepare(1e-6, 1e-6, 100, snapshot_interval=sim.T)
+    torch.cuda.synchronize(cuda)
+    side = torch.cuda.Stream(cuda)
+    sim.run_steps(10, stream=side)
+    side.synchronize()
+    big = torch.empty((2, 1 << 30), device=cuda, dtype=torch.uint8)
+    for _ in range(100):
+        big[1].copy_(big[0])
+    sim.run_steps(10)
+    done = torch.cuda.Event()
+    done.record()
+    d = sim._sim
+    work = d.pop("work")
+    at, nbytes = work.data_ptr(), work.numel()
+    del work
+    with torch.cuda.stream(side):
+        others = [torch.full((nbytes,), 255, device=cuda, dtype=torch.uint8) for _ in range(4)]
+    assert not done.query()
+    assert at not in [t.data_ptr() for t in others]
+    torch.cuda.synchronize(cuda)
+    assert torch.equal(d["x"][:, : sim.n_nodes], ref["x"])

@@ -226,6 +226,7 @@ class Monodomain:
             scratch=torch.zeros(int(_lib.load().tcb_mono_scratch_doubles()), device=dev, dtype=torch.float64),
             barrier=torch.zeros(4, device=dev, dtype=torch.int32),
             params=im.param_array(), per_frame=per_frame, next_step=1, work=None, work_asked=False,
+            work_beside=False,
         )
         m = _lib.tcb_mono()
         m.n_nodes, m.n_pad, m.n_slices, m.nt = n, n_pad, s.n_slices, nt
@@ -279,6 +280,14 @@ class Monodomain:
                 if not torch.cuda.is_current_stream_capturing():
                     sim["work"] = _work_buffer(sim["struct"], self.system)
                     sim["work_asked"] = True
+            sim["work_beside"] = stream is not None and sim["work"] is not None
+        elif sim["work_beside"]:
+            self._work_used_on(stream)
+
+    def _work_used_on(self, stream=None):
+        """An exchange buffer made on a stream of the caller's belongs to that stream's memory: what
+        other streams do with it keeps it from being handed out again there."""
+        self._sim["work"].record_stream(stream if stream is not None else torch.cuda.current_stream(self.device))
 
     def run_steps(self, n_steps, stream=None):
         """Advance the prepared simulation by ``n_steps`` steps on ``stream`` (default: the current
@@ -318,8 +327,6 @@ class Monodomain:
         lib = _lib.load()
         # the first launch on a device configures kernel attributes: keep it outside capture
         graph = torch.cuda.CUDAGraph()
-        # the buffers' set-up and earlier steps, on whatever stream they were queued
-        torch.cuda.synchronize(self.device)
         # recorded on a stream of its own without the garbage collection and release of
         # cached memory that torch.cuda.graph() begins with (2 to 60 ms): nothing is
         # allocated while the launches are recorded, and the collector, which could free
@@ -328,6 +335,8 @@ class Monodomain:
         side = torch.cuda.Stream(self.device)
         struct, stream = C.byref(sim["struct"]), side.cuda_stream
         with _recording, torch.cuda.stream(side):
+            # the buffers' set-up and earlier steps, on whatever stream they were queued
+            torch.cuda.synchronize(self.device)
             collecting = gc.isenabled()
             gc.disable()
             try:
@@ -345,6 +354,8 @@ class Monodomain:
         def replay():
             if sim["next_step"] + n_steps > self.nt + 1:
                 raise RuntimeError("not enough steps left for a full replay")
+            if sim["work_beside"]:
+                self._work_used_on()
             graph.replay()
             sim["next_step"] += n_steps
         replay.graph = graph
