@@ -146,7 +146,10 @@ def test_first_steps_on_a_stream_of_the_callers(lib, cuda):
         big[1].copy_(big[0])
     busy = torch.cuda.Event()
     busy.record()
-    assert sim.run_steps(20, stream=side) == 20
+    assert sim.run_steps(12, stream=side) == 12
+    class Handle:                 # any object with a stream's address, as stream_ptr takes
+        cuda_stream = side.cuda_stream
+    assert sim.run_steps(8, stream=Handle()) == 8
     side.synchronize()
     assert not busy.query()       # the steps did not wait for the copies
     assert sim._sim["work"] is not None

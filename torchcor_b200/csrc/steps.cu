@@ -109,11 +109,12 @@ __device__ __forceinline__ Alpha split(double alpha) {
 // {r, p, A p, 1/diag}.  Every row that needs p' of a neighbour forms it, so the
 // conversions to float64 that r' would take (8.5 cycles of a scheduler each, three for
 // r' alone) weigh more than the sum: r' is taken from the exact product and sum in
-// float32 pairs instead (Dekker 1971, Knuth's two-sum), right to about 2^-46 of |r| + |alpha A p|
-// before its one rounding.  z' is one rounding of an exact product in either form.  Against the same
-// kernel with r' formed in float64, the errors of 24 extracellular recoveries (cubes of 2,197 to 195,112
-// nodes) and 13 runs against 64 bits are equal (ratios 1.000, spread 0.001), and the pairs are faster: recovery of 68,921 nodes 12.8 -> 11.8 ms, CRN shell 40,962 18.1 -> 16.9, TTP cube
-// 50,653 19.8 -> 19.2.
+// float32 pairs instead (Dekker 1971, Knuth's two-sum), right to about 2^-46 of
+// |r| + |alpha A p| before its one rounding.  z' is one rounding of an exact product in
+// either form.  Against the same kernel with r' formed in float64, the errors of 24
+// extracellular recoveries (cubes of 2,197 to 195,112 nodes) and 13 runs against 64 bits
+// are equal (ratios 1.000, spread 0.001), and the pairs are faster: recovery of 68,921
+// nodes 12.8 -> 11.8 ms, CRN shell 40,962 18.1 -> 16.9, TTP cube 50,653 19.8 -> 19.2.
 __device__ __forceinline__ void advance(const float4& f, const Alpha& alpha, float beta, float& r, float& z, float& p) {
     const float h = __fmul_rn(alpha.hi, f.z);
     const float l = __fmaf_rn(alpha.lo, f.z, __fmaf_rn(alpha.hi, f.z, -h));

@@ -273,9 +273,9 @@ class Monodomain:
         self._sync_node_params()
         sim = self._sim
         # (not asked under a pinned launch shape, which may be taken back later)
+        if stream is not None and not isinstance(stream, torch.cuda.Stream):
+            stream = torch.cuda.ExternalStream(stream.cuda_stream, device=self.device)
         if not sim["work_asked"] and not sim["struct"].fused_step:
-            if stream is not None and not isinstance(stream, torch.cuda.Stream):
-                stream = torch.cuda.ExternalStream(stream.cuda_stream, device=self.device)
             with torch.cuda.stream(stream):
                 if not torch.cuda.is_current_stream_capturing():
                     sim["work"] = _work_buffer(sim["struct"], self.system)
